@@ -1,6 +1,6 @@
 """Build libmwfgpu.so (the C-ABI library) in-tree with nvcc for sm_103a.
 
-The three translation units compile in parallel; the result lands in mwf_gb300/lib/.
+The translation units compile in parallel; the result lands in mwf_gb300/lib/.
 """
 import os
 import subprocess
@@ -12,7 +12,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(LIBDIR, "libmwfgpu.so")
-SOURCES = ["mwf_host.cu", "kernels_f64.cu", "kernels_f32.cu", "kernels_zb.cu", "kernels_xb.cu", "kernels_persist.cu"]
+SOURCES = ["mwf_host.cu", "kernels_f64.cu", "kernels_f32.cu", "kernels_zb.cu", "kernels_xb.cu", "kernels_persist.cu", "kernels_fx.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off"]
 

@@ -16,7 +16,16 @@ Structure of the generated code (per physical point; p holds the KK y-coefficien
 so the z pass can form the term field by field.  p and nl are indexable accessors (register
 arrays or shared-memory views); each nl entry is read once and written once per call.
 
-Usage: python gen_nl.py > nl_gen.cuh   (the output is committed; nvcc does not run this).
+emit_fx writes the same coupling for the fixed-point FP64 z pass (mwf_fxpass.cuh): twice the
+projection, as sums of signed products, one function per kind of component and direction, so that
+the sums of one direction are the only accumulators alive:
+    nl_fx_p_<K0>(S, ld, A)   u or w component, x direction (S = u, ld(J) = d/dx f_J) or z (S = w)
+    nl_fx_v_<K0>(S, ld, A)   v component, x or z direction
+    nl_fx_yp_<K0>(V, F, A)   v d/dy of the u or w fields F, in units of b
+    nl_fx_yv_<K0>(V, A)      v d/dy of the v fields, in units of b
+
+Usage: python gen_nl.py > nl_gen.cuh; python gen_nl.py fx > nl_fx_gen.cuh   (the outputs are
+committed; nvcc does not run this).
 """
 from fractions import Fraction
 import sys
@@ -170,7 +179,50 @@ def emit(K0, out):
     out.append("}")
 
 
+def emit_fx(K0, out):
+    Gp, Gv, Hp, Hv = tensors(K0)
+    head = "template <typename S_, typename LD> __device__ __forceinline__ void"
+    for kind, G, lo in (("p", Gp, 0), ("v", Gv, 1)):
+        out.append(f"{head} nl_fx_{kind}_{K0}(const S_& S, LD&& ld, FxAcc (&A)[{K0}]) {{")
+        for j in range(lo, K0):
+            terms = [(k, i, c) for (k, i, jj), c in sorted(G.items()) if jj == j and c != 0]
+            out.append(f"  {{ const FxLimbs d = ld({j});")
+            if any(abs(c) == 1 for _, _, c in terms):
+                out.append("    const FxLimbs e = fx_twice(d);")
+            for k, i, c in terms:
+                if abs(c) not in (1, Fraction(1, 2)):
+                    raise ValueError(f"unexpected x/z coupling coefficient {c}")
+                out.append(f"    {'fx_mac' if c > 0 else 'fx_msb'}(A[{k}], S[{i}], {'e' if abs(c) == 1 else 'd'});")
+            out.append("  }")
+        out.append("}")
+    for kind, H, lo, args in (("yp", Hp, 0, "const S_& V, const F_& F"), ("yv", Hv, 1, "const S_& V")):
+        t = "typename S_, typename F_" if kind == "yp" else "typename S_"
+        out.append(f"template <{t}> __device__ __forceinline__ void nl_fx_{kind}_{K0}({args}, FxAcc (&A)[{K0}]) {{")
+        for j in range(1, K0):
+            terms = [(k, i, c) for (k, i, jj), c in sorted(H.items()) if jj == j and c != 0]
+            if not terms:
+                continue
+            out.append(f"  {{ const FxLimbs d = fx_times({'F' if kind == 'yp' else 'V'}[{j}], {j});")
+            if any(abs(c) == j for _, _, c in terms):
+                out.append("    const FxLimbs e = fx_twice(d);")
+            for k, i, c in terms:
+                if abs(c) not in (j, Fraction(j, 2)):
+                    raise ValueError(f"unexpected y coupling coefficient {c}")
+                out.append(f"    {'fx_mac' if c > 0 else 'fx_msb'}(A[{k}], V[{i}], {'e' if abs(c) == j else 'd'});")
+            out.append("  }")
+        out.append("}")
+
+
 def main():
+    if sys.argv[1:] == ["fx"]:
+        out = ["// Generated by gen_nl.py fx -- do not edit.  The Galerkin coupling as fixed-point products.",
+               "#pragma once",
+               "namespace mwf {"]
+        for K0 in (4, 6):
+            emit_fx(K0, out)
+        out.append("}  // namespace mwf")
+        sys.stdout.write("\n".join(out) + "\n")
+        return
     out = ["// Generated by gen_nl.py -- do not edit.  Galerkin coupling of Model Waleffe Flow.",
            "#pragma once",
            "#define MWF_BETA 1.5707963267948966",

@@ -69,6 +69,20 @@ struct FftPlanDev {
   FastDiv fns[MWF_MAX_STAGES];  // division by ns
 };
 
+// Plan of the in-place fixed-point transforms (mwf_fx.cuh) for one line length N = 2^a 3^b: stage s
+// has butterflies of radix[s] elements stride[s] apart, stride[s] = N / (radix[0] ... radix[s]), and
+// its twiddles at tw_off[s] of the run's table, (radix - 1) stride of them.
+struct FxPlan {
+  int N;
+  int nst;
+  int radix[MWF_MAX_STAGES];
+  int stride[MWF_MAX_STAGES];
+  int tw_off[MWF_MAX_STAGES];
+  FastDiv fnb[MWF_MAX_STAGES];  // division by N / radix
+  FastDiv fst[MWF_MAX_STAGES];  // division by stride
+};
+constexpr int kFxMaxCols = 8;   // columns of an item of the fixed-point x passes
+
 // Shared-memory index of element i of an FFT buffer: one pad element after every 128
 // bytes, so the radix-R strided accesses of the Stockham stages spread over all banks.
 template <typename T>
@@ -119,6 +133,17 @@ struct RunDesc {
   unsigned long long test_wait_ns;
   double diag_ct;               // threshold of the physical-space diagnostic
   FftPlanDev planX, planQ;
+  // FP64 runs in fixed point (mwf_fxpass.cuh): columns per x-forward / x-inverse item (powers of
+  // two), column blocks of the x forward, x lines per z item; twiddles e^{-2 pi i t/N} as fixed-point
+  // pairs (t < X, t < Z) and by stage for MM and NN; gamma n as mantissa and exponent; position ->
+  // element of the digit-reversed x lines; the scales of what the passes store
+  int fx;
+  int fx_nb, fx_xi_nb, fx_nblk, fx_lines;
+  const int4 *fx_twX, *fx_twZ, *fx_twM, *fx_twQ, *fx_gn;
+  const unsigned short* fx_rev;
+  int *fx_colE, *fx_blkE, *fx_rowE, *fx_minE;
+  float* fx_rowP;
+  FxPlan fx_planM, fx_planQ;
 };
 
 // One CTA's share of a pass.

@@ -1,0 +1,779 @@
+// The three passes of the FP64 timestep in 64-bit fixed point (mwf_fx.cuh; sm_103a).
+//
+//   x forward  item (run, first column n0, field f in 0 .. 2KK-1): the field's spectral values are
+//              formed in FP64 (var_mpt2spec + vel_addlam + var_spec_grad, variables.f90:390-434,
+//              600-612), scaled to integers column by column and transformed in x as three
+//              interleaved subsets x = s + 3q of length MM (tra_spec2phys, transform.fftw5.f90:69-78)
+//   z          item (run, first x line x0, z-subset s): all NPAIR + KK backward transforms of the
+//              lines z = s + 3q, the Galerkin coupling (udotgradu, modes.M4.f90:14-28 /
+//              modes.M6.f90:14-20) as integer products, NPAIR forward transforms and the split
+//              (transform.fftw5.f90:80-85, 126-135)
+//   x inverse  item (run, first column n0, wall-normal mode k): the three partials summed, forward
+//              x transforms, var_spec2mpt (variables.f90:440-480) and the update of vel_TS
+//              (velocity.f90:21-41) in FP64
+//
+// What is stored between the passes (RunDesc, fx_*):
+//   T     longlong2[2KK][X][NN], column (f, n) scaled by 2^colE[f][n]
+//   rowP  float[2KK][X][nblk] and blkE int[2KK][nblk]: for row (f, x) and column block b, the sum of
+//         |re| + |im| over the block is rowP 2^(32 - blkE), the last entry being column n = 0, which
+//         block 0 leaves out; the z pass scales its lines by the sums
+//   NLT   longlong2[3][KK][X][NN], row (s, f, x) scaled by 2^rowE[s][f][x]; minE[f] = the smallest
+//         of field f, the scale at which the x inverse adds the partials
+// Values are unnormalised; the 1/(3MM 3NN) of the forward transform is applied in the update.
+#pragma once
+#include "mwf_kernels.cuh"
+#include "mwf_fx.cuh"
+#include "nl_fx_gen.cuh"
+
+namespace mwf {
+
+// The e with 2^(e-1) <= v < 2^e, for a normal v > 0.
+__device__ __forceinline__ int fx_bits_above(float v) { return (int)((__float_as_uint(v) >> 23) & 255) - 126; }
+// 2^k for k <= 0, zero below the float range.
+__device__ __forceinline__ float fx_pow2(int k) { return k < -126 ? 0.f : __int_as_float((k + 127) << 23); }
+// Number of bits of values whose largest high word is hi (at least 32).
+__device__ __forceinline__ int fx_bitlen(int hi) { return 64 - __clz(hi); }
+
+__device__ __forceinline__ float fx_warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// A sum of moduli S 2^E; S = 0: nothing but zeros.
+struct FxNorm { float S; int E; };
+__device__ __forceinline__ FxNorm fx_norm_add(FxNorm a, FxNorm b) {
+  if (a.S == 0.f) return b;
+  if (b.S == 0.f) return a;
+  FxNorm r;
+  r.E = max(a.E, b.E);
+  r.S = a.S * fx_pow2(max(a.E - r.E, -127)) + b.S * fx_pow2(max(b.E - r.E, -127));
+  return r;
+}
+
+// ---------------------------------------------------------------------------------------
+// x forward
+// ---------------------------------------------------------------------------------------
+
+// Sum over the M slots of a row of |re| + |im| times |m|^p0 (S0) and |m|^p1 (S1), each as a float times
+// 2^E; nan: a NaN or an infinity in the row.  One warp; the high words are enough (truncated by
+// less than 2^-20, which the caller covers).
+__device__ __forceinline__ void fx_row_moments(const double2* __restrict__ row, int M, int MM, int p0, int p1,
+                                               float& S0, float& S1, int& E, int& nan) {
+  const int lane = threadIdx.x & 31;
+  int top = 0;
+  for (int ms = lane; ms < M; ms += 32) {
+    const double2 v = row[ms];
+    top = max(top, max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff));
+  }
+  top = __reduce_max_sync(0xffffffffu, top) >> 20;
+  nan = top >= 0x7ff;
+  float a = 0.f, b = 0.f;
+  for (int ms = lane; ms < M; ms += 32) {
+    const double2 v = row[ms];
+    auto part = [&](double x) {
+      const int h = (__double2hiint(x) & 0x7fffffff) - (top - 127) * (1 << 20);   // exponent relative to the largest
+      return h < (1 << 20) ? 0.f : __int_as_float(h << 3);
+    };
+    const float t = part(v.x) + part(v.y);
+    const float m = (float)(ms < MM ? ms : M - ms);
+    a += t * (p0 == 0 ? 1.f : p0 == 1 ? m : p0 == 2 ? m * m : m * m * m);
+    b += t * (p1 == 0 ? 1.f : p1 == 1 ? m : m * m);
+  }
+  S0 = top ? fx_warp_sum(a) : 0.f;                   // (zeros and subnormals count as zeros)
+  S1 = top ? fx_warp_sum(b) : 0.f;
+  E = top - 1023;
+}
+
+template <int NT>
+__global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDesc* __restrict__ runs, const WorkItem* __restrict__ items) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  longlong2* buf = reinterpret_cast<longlong2*>(smem_raw);       // line (l, s) at (3 l + s) MM
+  __shared__ int colE[kFxMaxCols];
+  const WorkItem wi = items[blockIdx.x];
+  const RunDesc& R = runs[wi.run];
+  if (!R.active) return;
+  const int X = R.X, MM = R.MM, NN = R.NN, KK = R.KK, M = R.M, K = R.K, K0 = R.K0;
+  const int n0 = wi.a, f = wi.b, nbw = R.fx_nb;
+  const int nb = min(nbw, NN - n0);
+  const bool deriv = f >= KK;
+  const int fs = deriv ? f - KK : f;
+  const int k = field_k(fs, K0);
+  const int comp = fs < K0 ? 0 : (fs < 2 * K0 - 1 ? 1 : 2);
+  const double2* __restrict__ c = reinterpret_cast<const double2*>(R.c);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int4* tw = reinterpret_cast<int4*>(buf + ((3 * nbw * MM + 7) & ~7));
+  for (int i = threadIdx.x; i < MM; i += NT) tw[i] = R.fx_twM[i];
+  if (n0 == 0 && !deriv && threadIdx.x == 0) R.fx_minE[f] = 1 << 29;      // the z pass takes minima into it
+
+  // Column scales from bounds on the columns' L1 norms: u = i(-n1 psi + k1 m1 phi), w = i(m1 psi +
+  // k1 n1 phi), v = (m1^2 + n1^2) phi and the same times m1 (m1 = alpha m, n1 = gamma n)
+  for (int l = warp; l < nb; l += NT / 32) {
+    const int n = n0 + l;
+    const double a1 = fabs(R.alpha), g1 = fabs(R.gamma * n), k1 = fabs(kbeta<double>(k));
+    const int d = deriv ? 1 : 0;
+    double L = 0.0;
+    int nan = 0;
+    const double2* col = c + (size_t)n * K * M;
+    if (comp != 1) {                                  // psi: u needs m^d, w m^(d+1)
+      float s0, s1;
+      int E, bad;
+      fx_row_moments(col + (size_t)k * M, M, MM, comp == 0 ? d : d + 1, 0, s0, s1, E, bad);
+      nan |= bad;
+      L += scalbn((comp == 0 ? g1 : a1) * (double)s0, E);
+      if (n == 0 && !deriv) {                         // the mean flow u_k = psi_k, and the base flow
+        const double2 v = col[(size_t)k * M];
+        L += fabs(v.x) + fabs(v.y) + (k == 1 ? 1.0 : 0.0);
+      }
+    }
+    if (k >= 1) {                                     // phi: u m^(d+1), w m^d, v m^(d+2) and m^d
+      float s0, s1;
+      int E, bad;
+      fx_row_moments(col + (size_t)(k + K0 - 1) * M, M, MM, comp == 0 ? d + 1 : comp == 2 ? d : d + 2, d, s0, s1, E, bad);
+      nan |= bad;
+      if (comp == 0) L += scalbn(k1 * a1 * (double)s0, E);
+      else if (comp == 2) L += scalbn(k1 * g1 * (double)s0, E);
+      else L += scalbn(a1 * a1 * (double)s0, E) + scalbn(g1 * g1 * (double)s1, E);
+      if (comp == 2 && n == 0 && !deriv) {            // the mean flow w_k = phi_k
+        const double2 v = col[(size_t)(k + K0 - 1) * M];
+        L += fabs(v.x) + fabs(v.y);
+      }
+    }
+    if (deriv) L *= a1;
+    L *= 1.0001;
+    const int ex = (int)(fx_bits(L) >> 52) & 0x7ff;
+    const int e = nan || ex == 0x7ff ? kFxNan : (L == 0.0 ? kFxZero : 61 - (ex - 1022));
+    if (lane == 0) {
+      colE[l] = e;
+      R.fx_colE[(size_t)f * NN + n] = e;
+    }
+  }
+  __syncthreads();
+
+  // fill: a = value at m = j, b = value at m = j - MM; subset s of the column has the length-MM
+  // spectrum e^{2 pi i js/X} (a + e^{-2 pi i s/3} b)
+  const int4* __restrict__ xm = R.fx_twX;             // e^{-2 pi i t/X}
+  const FastDiv fMM = make_fastdiv(MM);
+  const double kb1 = kbeta<double>(k);
+  for (int e = threadIdx.x; e < nb * MM; e += NT) {
+    const int l = fMM.div(e);
+    const int j = e - l * MM;
+    const int ce = colE[l];
+    const double n1 = R.gamma * (n0 + l);
+    auto value = [&](int m) {
+      const double m1 = R.alpha * m;
+      double2 v = mpt_to_field_w<double>(R, c, fs, m, n0 + l, true, m1, n1, kb1);
+      if (deriv) v = make_double2(-v.y * m1, v.x * m1);
+      longlong2 q;
+      q.x = fx_from_double(v.x, ce);
+      q.y = fx_from_double(v.y, ce);
+      return q;
+    };
+    const longlong2 a = value(j);
+    const int base = 3 * l * MM + j;
+    if (j == 0) {
+      buf[fx_at(base)] = a;
+      buf[fx_at(base + MM)] = a;
+      buf[fx_at(base + 2 * MM)] = a;
+      continue;
+    }
+    const longlong2 b = value(j - MM);
+    buf[fx_at(base)] = cadd(a, b);
+    constexpr FxConst s3 = fx_const(kFxSqrt34);
+    const i64 rx = fx_mulc(b.x, s3), ry = fx_mulc(b.y, s3);
+    longlong2 h, p, q;
+    h.x = a.x - (b.x >> 1);
+    h.y = a.y - (b.y >> 1);
+    p.x = h.x + ry; p.y = h.y - rx;                   // a + e^{-2 pi i/3} b
+    q.x = h.x - ry; q.y = h.y + rx;                   // a + e^{-4 pi i/3} b
+    buf[fx_at(base + MM)] = fx_cmul<true>(p, xm[j]);
+    buf[fx_at(base + 2 * MM)] = fx_cmul<true>(q, xm[2 * j]);
+  }
+  __syncthreads();
+
+  {
+    const int lines = 3 * nb;
+    const int G = max(1, min(lines, 256 / MM));
+    for (int t = warp * G; t < lines; t += (NT / 32) * G)
+      fx_fft<true>(buf, t * MM, min(G, lines - t), R.fx_planM, tw, nullptr);
+  }
+  __syncthreads();
+
+  // store: consecutive lanes take consecutive columns (nbw of them, a power of two), then
+  // positions; the block's part of the row norms is summed over those lanes
+  // (column n = 0 apart: it holds the base and mean flows, which the z derivatives do not have)
+  const int nblk = R.fx_nblk, blk = n0 / nbw, lo = n0 == 0 ? 1 : 0;
+  int eb = kFxZero;
+  for (int l = lo; l < nb; ++l) eb = min(eb, colE[l]);
+  if (threadIdx.x == 0) {
+    R.fx_blkE[(size_t)f * nblk + blk] = eb;
+    if (lo) R.fx_blkE[(size_t)f * nblk + nblk - 1] = colE[0];
+  }
+  const int lw = 31 - __clz(nbw);
+  const int l = threadIdx.x & (nbw - 1);
+  const bool live = l < nb, apart = l < lo;
+  const int ce = live ? colE[l] : kFxZero;
+  const int er = apart ? ce : eb;
+  const float wgt = (ce >= kFxZero || er <= kFxNan) ? 0.f : fx_pow2(max(er - ce, -127));
+  longlong2* __restrict__ T = reinterpret_cast<longlong2*>(R.T) + (size_t)f * X * NN;
+  float* __restrict__ P = R.fx_rowP + (size_t)f * X * nblk;
+  for (int e0 = 0; e0 < (X << lw); e0 += NT) {
+    const int sp = (e0 + threadIdx.x) >> lw;          // s MM + position
+    const bool on = sp < X;
+    const int s = on ? fMM.div(sp) : 0;
+    const int p = on ? sp - s * MM : 0;
+    const int x = s + 3 * R.fx_rev[p];
+    float part = 0.f;
+    if (on && live) {
+      const longlong2 v = buf[fx_at((3 * l + s) * MM + p)];
+      T[(size_t)x * NN + n0 + l] = v;
+      part = ((float)fx_abs_hi(v.x) + (float)fx_abs_hi(v.y) + 2.f) * wgt;
+    }
+    if (on && apart) P[(size_t)x * nblk + nblk - 1] = part;
+    if (apart) part = 0.f;
+    for (int o = 1; o < nbw; o <<= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    if (on && l == 0) P[(size_t)x * nblk + blk] = part;
+  }
+}
+
+// ---------------------------------------------------------------------------------------
+// z pass
+// ---------------------------------------------------------------------------------------
+
+// Sums of moduli of row (f, x), and of the moduli times the z wavenumber index (an upper bound: the
+// block's largest), over the W lanes (a power of two) of a warp's segment; lane = place in it.
+__device__ __forceinline__ void fx_row_norm(const RunDesc& R, int f, int x, int W, int lane, float& S, float& Z, int& E, int& bad) {
+  const int nblk = R.fx_nblk;
+  const float* __restrict__ P = R.fx_rowP + ((size_t)f * R.X + x) * nblk;
+  const int* __restrict__ EB = R.fx_blkE + (size_t)f * nblk;
+  int ref = -(1 << 29);
+  bad = 0;
+  float s = 0.f, z = 0.f;
+  for (int b0 = 0; b0 < nblk; b0 += 4 * W) {          // four blocks of a lane in flight
+    float p[4];
+    int e[4], top = -(1 << 29);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int b = b0 + i * W + lane;
+      p[i] = b < nblk ? P[b] : 0.f;
+      e[i] = b < nblk ? EB[b] : kFxZero;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      bad |= e[i] <= kFxNan;
+      if (p[i] > 0.f) top = max(top, -e[i]);
+    }
+    for (int o = 1; o < W; o <<= 1) {
+      top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+      bad |= __shfl_xor_sync(0xffffffffu, bad, o);
+    }
+    if (top > ref) {                                  // the same for the whole segment
+      const float k = fx_pow2(max(ref - top, -127));
+      s *= k;
+      z *= k;
+      ref = top;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (p[i] > 0.f) {
+        const float v = p[i] * fx_pow2(max(-e[i] - ref, -127));
+        s += v;
+        const int b = b0 + i * W + lane;
+        if (b < nblk - 1) z += v * (float)((b + 1) * R.fx_nb - 1);    // the last entry is n = 0
+      }
+  }
+  for (int o = 1; o < W; o <<= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    z += __shfl_xor_sync(0xffffffffu, z, o);
+  }
+  S = s;
+  Z = z;
+  E = ref + 32;
+}
+
+// Groups of values with one scale in the coupling: the velocity components, and their x and z
+// derivatives.
+enum { kFxU = 0, kFxV = 1, kFxW = 2, kFxDx = 3, kFxDz = 6, kFxGroups = 9 };
+
+template <int K0> __host__ __device__ constexpr int fx_comp(int f) { return f < K0 ? 0 : (f < 2 * K0 - 1 ? 1 : 2); }
+template <int K0> __host__ __device__ constexpr int fx_first(int comp) { return comp == 0 ? 0 : (comp == 1 ? K0 : 2 * K0 - 1); }
+template <int K0> __host__ __device__ constexpr int fx_count(int comp) { return comp == 1 ? K0 - 1 : K0; }
+
+template <int K0, int NT>
+__global__ void __launch_bounds__(NT, 512 / NT) z_fx_kernel(const RunDesc* __restrict__ runs, const WorkItem* __restrict__ items) {
+  constexpr int KK = 3 * K0 - 1, NPAIR = (KK + 1) / 2, NTR = NPAIR + KK;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const WorkItem wi = items[blockIdx.x];
+  const RunDesc& R = runs[wi.run];
+  if (!R.active) return;
+  const int X = R.X, Q = R.NN, x0 = wi.a, s = wi.b;
+  const int L = min(R.fx_lines, X - x0);
+  // line (t, l) at t TS + l Q: TS is a multiple of 64, so the place of an element within the
+  // lines of one t is the same for every t
+  const int TS = (L * Q + 63) & ~63;
+  longlong2* buf = reinterpret_cast<longlong2*>(smem_raw);
+  int4* tw = reinterpret_cast<int4*>(buf + (size_t)NTR * TS);    // [Q] stage twiddles
+  int* eL = reinterpret_cast<int*>(tw + Q);                      // [NTR L] line exponents
+  int* mx = eL + NTR * L;                                        // [2 NTR L] largest high words (re, im), then shifts
+  int* ge = mx + 2 * NTR * L;                                    // [kFxGroups L] group exponents
+  int* eo = ge + kFxGroups * L;                                  // [3 L] exponents of the products
+  int* sh = eo + 3 * L;                                          // [NPAIR L] forward line shifts
+  int* bad = sh + NPAIR * L;                                     // [L] NaN lines
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int NW = NT / 32;
+  const longlong2* __restrict__ T = reinterpret_cast<const longlong2*>(R.T);
+  const size_t fstride = (size_t)X * Q;
+
+  for (int i = threadIdx.x; i < Q; i += NT) tw[i] = R.fx_twQ[i];
+  for (int i = threadIdx.x; i < 2 * NTR * L; i += NT) mx[i] = 0;
+  for (int i = threadIdx.x; i < L; i += NT) bad[i] = 0;
+  __syncthreads();
+
+  // ---- line scales: the rows' norms, a warp segment each (in the lines' space, not yet in use) ----
+  {
+    float* nS = reinterpret_cast<float*>(smem_raw);              // [2KK L]
+    float* nZ = nS + 2 * KK * L;
+    int* nE = reinterpret_cast<int*>(nZ + 2 * KK * L);
+    int W = 1;
+    while (W < 32 && 2 * W < R.fx_nblk) W <<= 1;
+    const int sub = lane / W, seg = 32 / W;
+    for (int i0 = warp * seg; i0 < 2 * KK * L; i0 += NW * seg) {
+      const int i = min(i0 + sub, 2 * KK * L - 1);
+      const int f = i / L, l = i - f * L;
+      float a, z;
+      int e, nan;
+      fx_row_norm(R, f, x0 + l, W, lane & (W - 1), a, z, e, nan);
+      if ((lane & (W - 1)) == 0) {
+        nS[i] = a;
+        nZ[i] = z * fabsf(R.gamma_f);
+        nE[i] = e;
+        if (nan) bad[l] = 1;
+      }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < NTR * L; i += NT) {
+      const int t = i / L, l = i - t * L;
+      const int a = (t < NPAIR ? 2 * t : KK + t - NPAIR) * L + l;
+      const int b = (t < NPAIR ? 2 * t + 1 : t - NPAIR) * L + l;
+      const bool two = t >= NPAIR || 2 * t + 1 < KK;
+      const FxNorm v = fx_norm_add(FxNorm{nS[a], nE[a]}, FxNorm{two ? (t < NPAIR ? nS[b] : nZ[b]) : 0.f, two ? nE[b] : 0});
+      // the Hermitian extension doubles every coefficient: the line's norm is below 2 S 2^E
+      eL[i] = v.S > 0.f ? 61 - (v.E + 1 + fx_bits_above(v.S * 1.001f)) : kFxZero;
+    }
+  }
+  __syncthreads();
+
+  // ---- fill and backward transforms: a warp per line (or G short ones) ----
+  // With w = e^{2 pi i ns/Z}, eps = e^{-2 pi i s/3}: H[n] = w (U + eps V) and
+  // H[Q-n] = w' (U' + eps V'), w' = e^{2 pi i (Q-n)s/Z}, where U = a + i b at n, V = conj a + i conj b
+  // at Q-n, and U', V' the same with n and Q-n exchanged.  Slot n < (Q+1)/2 of a line is the pair
+  // (n, Q-n); slot 0 is n = 0 with, for even Q, n = Q/2 (its own partner).
+  const int4* __restrict__ om = R.fx_twZ;             // e^{-2 pi i t/Z}
+  const int* __restrict__ colE = R.fx_colE;
+  const int4* __restrict__ gn = R.fx_gn;              // gamma n as (h, l, exponent)
+  constexpr FxConst s3 = fx_const(kFxSqrt34);
+  auto times_eps = [&](longlong2 a) {                 // eps a for this subset (s = 1, 2)
+    const i64 rx = fx_mulc(a.x, s3), ry = fx_mulc(a.y, s3);
+    longlong2 r;
+    r.x = s == 1 ? -(a.x >> 1) + ry : -(a.x >> 1) - ry;
+    r.y = s == 1 ? -(a.y >> 1) - rx : -(a.y >> 1) + rx;
+    return r;
+  };
+  const int G = max(1, min(L, 256 / Q));
+  const int groups = (L + G - 1) / G;
+  const int slots = (Q + 1) / 2;
+  const bool even = (Q & 1) == 0;
+  const FastDiv fSl = make_fastdiv(slots);
+  struct In { longlong2 Pa, Ra, Pb, Rb; int ea, ra, eb, rb; };
+  for (int i = warp; i < NTR * groups; i += NW) {
+    const int t = i / groups, l0 = (i - t * groups) * G, nl = min(G, L - l0);
+    const bool der = t >= NPAIR;
+    const int fa = der ? KK + t - NPAIR : 2 * t;
+    const bool two = der || 2 * t + 1 < KK;
+    const int fb = der ? t - NPAIR : (two ? 2 * t + 1 : fa);
+    const int* __restrict__ ea = colE + (size_t)fa * Q;
+    const int* __restrict__ eb = colE + (size_t)fb * Q;
+    const longlong2* __restrict__ pa = T + (size_t)fa * fstride + (size_t)(x0 + l0) * Q;
+    const longlong2* __restrict__ pb = T + (size_t)fb * fstride + (size_t)(x0 + l0) * Q;
+    const int total = nl * slots;
+    auto load = [&](int idx) {
+      In v;
+      const int l = fSl.div(idx), sl = idx - l * slots;
+      const int n = sl ? sl : (even ? Q / 2 : 0), nq = sl ? Q - sl : 0;
+      v.Pa = pa[l * Q + n];
+      v.Ra = pa[l * Q + nq];
+      v.Pb = pb[l * Q + n];
+      v.Rb = pb[l * Q + nq];
+      v.ea = ea[n]; v.ra = ea[nq]; v.eb = eb[n]; v.rb = eb[nq];
+      return v;
+    };
+    In nx;
+    if (lane < total) nx = load(lane);
+    for (int idx = lane; idx < total; idx += 32) {
+      const In v = nx;
+      if (idx + 32 < total) nx = load(idx + 32);      // the next slot's rows while this one is formed
+      const int l = fSl.div(idx), sl = idx - l * slots;
+      const int n = sl ? sl : (even ? Q / 2 : 0), nq = sl ? Q - sl : n;
+      const int e = eL[t * L + l0 + l], base = t * TS + (l0 + l) * Q;
+      const longlong2 Pa = fx_shift2(v.Pa, e - v.ea);
+      longlong2 Ra = fx_shift2(v.Ra, e - v.ra), Pb, Rb;
+      if (der) {
+        // b = i gamma n f: a + i b = a - gamma n f
+        const int4 gp = gn[n], gq = gn[sl ? nq : 0];
+        const int sp = e - v.eb + gp.z, sq = e - v.rb + gq.z;
+        Pb.x = fx_shift(fx_mulc(v.Pb.x, FxConst{gp.x, gp.y}), sp);
+        Pb.y = fx_shift(fx_mulc(v.Pb.y, FxConst{gp.x, gp.y}), sp);
+        Rb.x = fx_shift(fx_mulc(v.Rb.x, FxConst{gq.x, gq.y}), sq);
+        Rb.y = fx_shift(fx_mulc(v.Rb.y, FxConst{gq.x, gq.y}), sq);
+      } else {
+        Pb = fx_shift2(v.Pb, e - v.eb);
+        Rb = fx_shift2(v.Rb, e - v.rb);
+        if (!two) Pb.x = Pb.y = Rb.x = Rb.y = 0;
+      }
+      if (sl == 0) {                                  // H = Re X_0; the z derivative has none
+        longlong2 h;
+        h.x = Ra.x;
+        h.y = der ? 0 : Rb.x;
+        buf[fx_at(base)] = h;
+        Ra = Pa;
+        Rb = Pb;
+      }
+      longlong2 U, V, U2, V2;
+      if (der) {
+        U.x = Pa.x - Pb.x;  U.y = Pa.y - Pb.y;
+        V.x = Ra.x + Rb.x;  V.y = -Ra.y - Rb.y;
+        U2.x = Ra.x - Rb.x; U2.y = Ra.y - Rb.y;
+        V2.x = Pa.x + Pb.x; V2.y = -Pa.y - Pb.y;
+      } else {
+        U.x = Pa.x - Pb.y;  U.y = Pa.y + Pb.x;
+        V.x = Ra.x + Rb.y;  V.y = Rb.x - Ra.y;
+        U2.x = Ra.x - Rb.y; U2.y = Ra.y + Rb.x;
+        V2.x = Pa.x + Pb.y; V2.y = Pb.x - Pa.y;
+      }
+      longlong2 Hn, Hq;
+      if (s == 0) {
+        Hn = cadd(U, V);
+        Hq = cadd(U2, V2);
+      } else {
+        Hn = fx_cmul<true>(cadd(U, times_eps(V)), om[n * s]);
+        Hq = fx_cmul<true>(cadd(U2, times_eps(V2)), om[nq * s]);
+      }
+      if (sl || even) buf[fx_at(base + n)] = Hn;
+      if (sl) buf[fx_at(base + nq)] = Hq;
+    }
+    __syncwarp();
+    fx_fft<true>(buf, t * TS + l0 * Q, nl, R.fx_planQ, tw, mx + 2 * (t * L + l0));
+  }
+  __syncthreads();
+
+  // ---- one exponent per group: the largest value of a velocity group fills 56 bits, of a
+  //      derivative group 57; mx becomes the shift of each part of a line to its group ----
+  for (int i = threadIdx.x; i < kFxGroups * L; i += NT) {
+    const int g = i / L, l = i - g * L, comp = g % 3;
+    const int f0 = fx_first<K0>(comp), f1 = f0 + fx_count<K0>(comp);
+    const bool vel = g < kFxDx;
+    auto place = [&](int f) { return 2 * ((vel ? f / 2 : NPAIR + f) * L + l) + (vel ? (f & 1) : (g >= kFxDz)); };
+    int top = -(1 << 29);
+    for (int f = f0; f < f1; ++f) top = max(top, fx_bitlen(mx[place(f)]) - eL[place(f) >> 1]);
+    const int e = (vel ? 56 : 57) - top;
+    ge[i] = e;
+    for (int f = f0; f < f1; ++f) mx[place(f)] = e - eL[place(f) >> 1];
+  }
+  __syncthreads();
+
+  // ---- coupling: the projections of one component at a time, one direction after the other, so
+  //      that the code of a direction is held once (straight-line code for all nine overran the
+  //      instruction cache) ----
+  const FastDiv fQ = make_fastdiv(Q);
+  for (int e = threadIdx.x; e < L * Q; e += NT) {
+    const int l = L == 1 ? 0 : fQ.div(e);
+    unsigned char* const at = smem_raw + (size_t)fx_at(e) * 16;
+    const size_t ts = (size_t)TS * 16;
+    // velocities: scaled to their group and split, in place
+#pragma unroll
+    for (int f = 0; f < KK; ++f) {
+      i64* const q = reinterpret_cast<i64*>(at + (f / 2) * ts) + (f & 1);
+      const FxLimbs v = fx_limbs(fx_scale(*q, mx[2 * ((f / 2) * L + l) + (f & 1)]));
+      *reinterpret_cast<int2*>(q) = make_int2(v.h, v.l);
+    }
+    auto vel = [&](int f) {
+      const int2 v = *(reinterpret_cast<const int2*>(at + (f >> 1) * ts) + (f & 1));
+      return FxLimbs{v.x, v.y};
+    };
+    constexpr FxConst b2 = fx_const(kFxQuarterPi);
+    const int gu = ge[kFxU * L + l], gv = ge[kFxV * L + l], gw = ge[kFxW * L + l];
+#pragma unroll 1
+    for (int comp = 0; comp < 3; ++comp) {
+      const int gx = gu + ge[(kFxDx + comp) * L + l] - 56;
+      const int gz = gw + ge[(kFxDz + comp) * L + l] - 56;
+      const int gy = gv + (comp == 0 ? gu : comp == 1 ? gv : gw) - 57;
+      const int go = min(gx, min(gy, gz)) - 2;
+      if (e == l * Q) eo[comp * L + l] = go;
+      const int f0 = comp == 0 ? 0 : comp == 1 ? K0 - 1 : 2 * K0 - 1;    // field of mode 0 (v has none)
+      i64 sum[K0];
+      FxAcc A[K0];
+#pragma unroll
+      for (int k = 0; k < K0; ++k) sum[k] = 0;
+#pragma unroll 1
+      for (int dir = 0; dir < 3; ++dir) {             // x, z, y
+#pragma unroll
+        for (int k = 0; k < K0; ++k) A[k] = FxAcc{0, 0};
+        if (dir < 2) {
+          FxLimbs S[K0];
+          const int s0 = dir ? 2 * K0 - 1 : 0;
+#pragma unroll
+          for (int k = 0; k < K0; ++k) S[k] = vel(s0 + k);
+          auto ld = [&](int j) {
+            const i64 q = *(reinterpret_cast<const i64*>(at + (NPAIR + f0 + j) * ts) + dir);
+            return fx_limbs(fx_scale(q, mx[2 * ((NPAIR + f0 + j) * L + l) + dir]));
+          };
+          if constexpr (K0 == 4) { if (comp == 1) nl_fx_v_4(S, ld, A); else nl_fx_p_4(S, ld, A); }
+          else { if (comp == 1) nl_fx_v_6(S, ld, A); else nl_fx_p_6(S, ld, A); }
+          const int r = (dir ? gz : gx) - go;
+#pragma unroll
+          for (int k = 0; k < K0; ++k) sum[k] += fx_down(fx_sum(A[k]), r);
+        } else {
+          // in units of b = pi/2: 2 nl = sum v (j f_j) b
+          FxLimbs V[K0], F[K0];
+          V[0] = F[0] = FxLimbs{0, 0};
+#pragma unroll
+          for (int k = 1; k < K0; ++k) V[k] = vel(K0 - 1 + k);
+          if (comp != 1) {
+#pragma unroll
+            for (int k = 1; k < K0; ++k) F[k] = vel(f0 + k);
+            if constexpr (K0 == 4) nl_fx_yp_4(V, F, A); else nl_fx_yp_6(V, F, A);
+          } else {
+            if constexpr (K0 == 4) nl_fx_yv_4(V, A); else nl_fx_yv_6(V, A);
+          }
+#pragma unroll
+          for (int k = 0; k < K0; ++k) sum[k] += fx_down(fx_mulc(fx_sum(A[k]), b2), gy - go);
+        }
+      }
+      // field f goes to line NPAIR + f/2, where only derivatives of this or an earlier component were
+#pragma unroll
+      for (int k = 0; k < K0; ++k) {
+        if (comp == 1 && k == 0) continue;
+        const int f = f0 + k;
+        *(reinterpret_cast<i64*>(at + (NPAIR + (f >> 1)) * ts) + (f & 1)) = sum[k];
+      }
+    }
+    if (KK & 1) *(reinterpret_cast<i64*>(at + (NPAIR + KK / 2) * ts) + 1) = 0;
+  }
+  __syncthreads();
+
+  // ---- forward transforms, split and store ----
+  longlong2* __restrict__ NLT = reinterpret_cast<longlong2*>(R.NLT) + (size_t)s * KK * fstride;
+  int WQ = 1;
+  while (WQ < 32 && WQ < Q) WQ <<= 1;
+  for (int i = warp; i < NPAIR * groups; i += NW) {
+    const int t = i / groups, l0 = (i - t * groups) * G, nl = min(G, L - l0);
+    const int first = (NPAIR + t) * TS + l0 * Q;
+    // scale each line so that its norm just fits (from the high words, rounded up)
+    for (int l = lane / WQ; l - lane / WQ < nl; l += 32 / WQ) {
+      float a = 0.f;
+      if (l < nl)
+        for (int n = lane & (WQ - 1); n < Q; n += WQ) {
+          const longlong2 v = buf[fx_at(first + l * Q + n)];
+          a += (float)fx_abs_hi(v.x) + (float)fx_abs_hi(v.y) + 2.f;
+        }
+      for (int o = 1; o < WQ; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (l < nl && (lane & (WQ - 1)) == 0) sh[t * L + l0 + l] = 61 - 32 - fx_bits_above(a * 1.001f);
+    }
+    __syncwarp();
+    fx_fft<false>(buf, first, nl, R.fx_planQ, tw, sh + t * L + l0);
+    const int ka = 2 * t;
+    const bool two = ka + 1 < KK;
+    longlong2* __restrict__ oa = NLT + (size_t)ka * fstride + (size_t)(x0 + l0) * Q;
+    longlong2* __restrict__ ob = oa + fstride;
+    // A = G[n] + conj G[Q-n] and B = (G[n] - conj G[Q-n]) / i are twice the spectra at n; at Q-n
+    // they are conj(A), conj(B), and e^{-2 pi i (Q-n)s/Z} = eps conj(e^{-2 pi i ns/Z})
+    for (int idx = lane; idx < nl * slots; idx += 32) {
+      const int l = fSl.div(idx), sl = idx - l * slots;
+      const int base = first + l * Q, o = l * Q;
+      const int n = sl ? sl : (even ? Q / 2 : 0), nq = sl ? Q - sl : n;
+      const longlong2 g = buf[fx_at(base + n)], m = buf[fx_at(base + nq)];
+      longlong2 A, B;
+      A.x = g.x + m.x; A.y = g.y - m.y;
+      B.x = g.y + m.y; B.y = m.x - g.x;
+      if (s != 0) {
+        const int4 w = om[n * s];
+        A = fx_cmul<false>(A, w);
+        B = fx_cmul<false>(B, w);
+      }
+      if (sl || even) {
+        oa[o + n] = A;
+        if (two) ob[o + n] = B;
+      }
+      if (sl) {
+        A.y = -A.y;
+        B.y = -B.y;
+        if (s != 0) { A = times_eps(A); B = times_eps(B); }
+        oa[o + nq] = A;
+        if (two) ob[o + nq] = B;
+      } else {
+        const longlong2 z = buf[fx_at(base)];
+        A.x = 2 * z.x; A.y = 0;
+        B.x = 2 * z.y; B.y = 0;
+        oa[o] = A;
+        if (two) ob[o] = B;
+      }
+    }
+    for (int j = lane; j < nl * 2; j += 32) {
+      const int l = l0 + (j >> 1), f = ka + (j & 1);
+      if (f >= KK) continue;
+      // the coupling is 2 nl, the split another factor of two
+      int e = eo[fx_comp<K0>(f) * L + l] + sh[t * L + l] + 2;
+      if (bad[l]) e = kFxNan;
+      R.fx_rowE[((size_t)s * KK + f) * X + x0 + l] = e;
+      atomicMin(&R.fx_minE[f], e);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------
+// x inverse and update
+// ---------------------------------------------------------------------------------------
+template <int NT>
+__global__ void __launch_bounds__(NT, 512 / NT) x_inverse_fx_kernel(const RunDesc* __restrict__ runs, const WorkItem* __restrict__ items) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  longlong2* buf = reinterpret_cast<longlong2*>(smem_raw);       // line (comp, l, s) at ((comp nb + l) 3 + s) MM
+  __shared__ u64 norm[9 * kFxMaxCols];
+  __shared__ int sh[9 * kFxMaxCols];
+  const WorkItem wi = items[blockIdx.x];
+  const RunDesc& R = runs[wi.run];
+  if (!R.active) return;
+  const int X = R.X, MM = R.MM, NN = R.NN, M = R.M, K0 = R.K0, K = R.K, KK = R.KK;
+  const int n0 = wi.a, k = wi.b, nbw = R.fx_xi_nb;
+  const int nb = min(nbw, NN - n0);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int NW = NT / 32;
+  const longlong2* __restrict__ NLT = reinterpret_cast<const longlong2*>(R.NLT);
+  const size_t fstride = (size_t)X * NN;
+  const int fu = k, fv = K0 + k - 1, fw = 2 * K0 - 1 + k;
+  const FastDiv fMM = make_fastdiv(MM);
+  int4* tw = reinterpret_cast<int4*>(buf + ((9 * nbw * MM + 7) & ~7));
+  for (int i = threadIdx.x; i < MM; i += NT) tw[i] = R.fx_twM[i];
+  const int lw = 31 - __clz(nbw);
+  const int l_ = threadIdx.x & (nbw - 1);
+  int ref[3];                                         // scale of each field's sum of partials
+#pragma unroll
+  for (int comp = 0; comp < 3; ++comp)
+    ref[comp] = (comp == 1 && k == 0) ? kFxZero : R.fx_minE[comp == 0 ? fu : comp == 1 ? fv : fw] - 2;
+
+  // load: consecutive lanes take consecutive columns, then positions
+  if (l_ < nb) {
+    for (int comp = 0; comp < 3; ++comp) {
+      const int f = comp == 0 ? fu : comp == 1 ? fv : fw;
+      const bool none = comp == 1 && k == 0;
+      for (int sp = threadIdx.x >> lw; sp < X; sp += NT >> lw) {
+        const int s = fMM.div(sp), p = sp - s * MM;
+        longlong2 v;
+        v.x = v.y = 0;
+        if (!none) {
+          const int x = s + 3 * R.fx_rev[p];
+          const size_t o = (size_t)f * fstride + (size_t)x * NN + n0 + l_;
+          const size_t ss = (size_t)KK * fstride;
+          const int* __restrict__ E = R.fx_rowE + (size_t)f * X + x;
+#pragma unroll
+          for (int z = 0; z < 3; ++z) {
+            const longlong2 q = NLT[o + z * ss];
+            const int r = E[(size_t)z * KK * X] - ref[comp];     // at least 2
+            v.x += fx_down(q.x, r);
+            v.y += fx_down(q.y, r);
+          }
+        }
+        buf[fx_at(((comp * nb + l_) * 3 + s) * MM + p)] = v;
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = warp; i < 9 * nb; i += NW) {
+    u64 a = 0;
+    for (int p = lane; p < MM; p += 32) {
+      const longlong2 v = buf[fx_at(i * MM + p)];
+      a += ((u64)(v.x ^ (v.x >> 63)) >> 13) + ((u64)(v.y ^ (v.y >> 63)) >> 13) + 2;
+    }
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (lane == 0) norm[i] = a;
+  }
+  __syncthreads();
+  // the three subsets of a line share a scale: their combined norm is below 2^61
+  for (int i = threadIdx.x; i < 9 * nb; i += NT) {
+    const int b = i / 3 * 3;
+    sh[i] = 61 - 13 - (64 - __clzll((i64)(norm[b] + norm[b + 1] + norm[b + 2])));
+  }
+  __syncthreads();
+  {
+    const int lines = 9 * nb;
+    const int G = max(1, min(lines, 256 / MM));
+    for (int t = warp * G; t < lines; t += NW * G)
+      fx_fft<false>(buf, t * MM, min(G, lines - t), R.fx_planM, tw, sh + t);
+  }
+  __syncthreads();
+
+  const int4* __restrict__ xm = R.fx_twX;
+  double2* __restrict__ c = reinterpret_cast<double2*>(R.c);
+  double2* __restrict__ onl = reinterpret_cast<double2*>(R.onl);
+  const double* __restrict__ ilhs = R.inv_lhs;
+  const double* __restrict__ rhs = R.rhs;
+  const bool first = *R.nst != 0;
+  const double hdt = R.dt / 2.0, alpha = R.alpha, gamma = R.gamma, scale = R.scale;
+  const double kb1 = kbeta<double>(k);
+  const FastDiv fM = make_fastdiv(M);
+  for (int o = threadIdx.x; o < nb * M; o += NT) {
+    const int l = fM.div(o);
+    const int ms = o - l * M;
+    const int n = n0 + l;
+    const int m = signed_m(ms, MM, M);
+    const size_t i0 = ((size_t)n * K + k) * M + ms;
+    const size_t i1 = i0 + (size_t)(K0 - 1) * M;
+    const int j = m >= 0 ? m : m + MM;
+    const int4 w1 = xm[m >= 0 ? m : m + X], w2 = xm[m >= 0 ? 2 * m : 2 * m + X];
+    double2 sp[3];
+#pragma unroll
+    for (int comp = 0; comp < 3; ++comp) {
+      const int base = (comp * nb + l) * 3 * MM + j;
+      const longlong2 F0 = buf[fx_at(base)], F1 = buf[fx_at(base + MM)], F2 = buf[fx_at(base + 2 * MM)];
+      const longlong2 v = cadd(cadd(F0, fx_cmul<false>(F1, w1)), fx_cmul<false>(F2, w2));
+      const int e = ref[comp] + sh[(comp * nb + l) * 3];
+      sp[comp].x = fx_to_double(v.x, e) * scale;
+      sp[comp].y = fx_to_double(v.y, e) * scale;
+      if (ref[comp] < kFxNan / 2) sp[comp].x = sp[comp].y = nan("");
+    }
+    const double2 su = sp[0], sv = sp[1], sw = sp[2];
+    const double m1 = alpha * m, n1 = gamma * n;
+    const double H = (-alpha * m * alpha * m) + (-gamma * n * gamma * n);
+    // var_spec2mpt (variables.f90:455-464)
+    double2 nphi, npsi;
+    nphi.x = -(su.y * m1 * kb1 + sw.y * n1 * kb1) + sv.x * H;
+    nphi.y = (su.x * m1 * kb1 + sw.x * n1 * kb1) + sv.y * H;
+    npsi.x = sw.y * m1 - su.y * n1;
+    npsi.y = -(sw.x * m1 - su.x * n1);
+    if (ms == 0 && n == 0) {   // mean modes (variables.f90:467-479)
+      if (k == 0) npsi = make_double2(0.0, 0.0);
+      else {
+        npsi = make_double2(-su.x, -su.y);
+        nphi = make_double2(-sw.x, -sw.y);
+      }
+    }
+    // AB2 / implicit update (velocity.f90:24-40); onl <- nl
+#pragma unroll
+    for (int which = 0; which < 2; ++which) {
+      if (which == 1 && k == 0) continue;
+      const size_t idx = which == 0 ? i0 : i1;
+      const double2 nlv = which == 0 ? npsi : nphi;
+      const double2 cold = c[idx];
+      const double2 ov = first ? nlv : onl[idx];
+      const double rr = rhs[idx], il = ilhs[idx];
+      double cx_ = rr * cold.x + hdt * (3.0 * nlv.x - ov.x);
+      double cy_ = rr * cold.y + hdt * (3.0 * nlv.y - ov.y);
+      cx_ *= il;
+      cy_ *= il;
+      if (k == 0 && which == 0 && ms == 0 && n == 0) cx_ = 0.0;
+      c[idx] = make_double2(cx_, cy_);
+      onl[idx] = nlv;
+    }
+  }
+}
+
+}  // namespace mwf

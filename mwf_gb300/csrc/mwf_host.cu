@@ -114,6 +114,62 @@ void twiddles_into(int N, int t0, int cnt, T* out) {
   }
 }
 
+// A twiddle (re, im) times 2^62 as two 32-bit limbs per part (FxConst: high, signed low), the low
+// limbs kept off -2^31 so that they can be negated.
+int4 fx_twiddle(const long double* v) {
+  int out[4];
+  for (int i = 0; i < 2; ++i) {
+    long long w = llroundl(v[i] * 4611686018427387904.0L);
+    if ((unsigned)w == 0x80000000u) ++w;
+    const int l = (int)(unsigned)w;
+    out[2 * i] = (int)((w - l) >> 32);
+    out[2 * i + 1] = l;
+  }
+  return make_int4(out[0], out[1], out[2], out[3]);
+}
+
+// Radix plan of the in-place fixed-point transforms, its stage twiddles (from w, the table of
+// e^{-2 pi i t/(3N)}) and the element that each position of a digit-reversed line holds.
+bool make_fx_plan(int N, const std::vector<int4>& w, FxPlan& pl, std::vector<int4>& tw, std::vector<unsigned short>& rev) {
+  if (!is_23_smooth(N) || N < 2) return false;
+  std::vector<int> rad;
+  int rest = N;
+  auto take = [&](int r) { rad.push_back(r); rest /= r; };
+  while (rest % 8 == 0 && rest != 16) take(8);          // 16 = 4 x 4, not 8 x 2
+  while (rest % 4 == 0) take(4);
+  while (rest % 2 == 0) take(2);
+  while (rest % 9 == 0) take(9);
+  while (rest % 3 == 0) take(3);
+  if ((int)rad.size() > MWF_MAX_STAGES) return false;
+  memset(&pl, 0, sizeof pl);
+  pl.N = N;
+  pl.nst = (int)rad.size();
+  tw.clear();
+  int span = N;
+  for (int s = 0; s < pl.nst; ++s) {
+    const int st = span / rad[s];
+    pl.radix[s] = rad[s];
+    pl.stride[s] = st;
+    pl.tw_off[s] = (int)tw.size();
+    pl.fnb[s] = make_fastdiv(N / rad[s]);
+    pl.fst[s] = make_fastdiv(st);
+    if (st > 1)
+      for (int r = 1; r < rad[s]; ++r)
+        for (int j = 0; j < st; ++j) tw.push_back(w[(size_t)3 * (j * r * (N / span) % N)]);
+    span = st;
+  }
+  rev.assign(N, 0);
+  for (int p = 0; p < N; ++p) {
+    int q = 0, span_q = 1;
+    for (int s = 0; s < pl.nst; ++s) {
+      q += (p / pl.stride[s]) % pl.radix[s] * span_q;
+      span_q *= pl.radix[s];
+    }
+    rev[p] = (unsigned short)q;
+  }
+  return span == 1;
+}
+
 template <typename T>
 std::vector<T> twiddles(int N) {
   std::vector<T> out(2 * (size_t)N);
@@ -179,6 +235,31 @@ struct RunHost {
   int xbf_nb = 0, xbi_nb = 0;   // columns per item of the subset-split FP32 x passes (0: not used)
   bool persist = false;         // all three passes batched: the run steps in the persistent kernel
   int active = 1;    // host copy of RunDesc::active
+  // FP64 in fixed point (mwf_fxpass.cuh): columns and block sizes of the x passes, lines and block
+  // size of the z pass
+  bool fx = false;
+  int fx_nb = 0, fx_xi_nb = 0, fx_lines = 0, fx_nblk = 0;
+  int fx_xf_nt = 0, fx_z_nt = 0, fx_xi_nt = 0;
+  size_t off_fx = 0;
+  struct FxOff { size_t twX, twZ, twM, twQ, gn, rev, colE, blkE, rowE, minE, rowP, end; };
+  FxOff fx_off() const {
+    FxOff o;
+    size_t a = off_fx;
+    auto put = [&](size_t bytes) { const size_t at = a; a = (a + bytes + 255) / 256 * 256; return at; };
+    o.twX = put(16 * (size_t)X);
+    o.twZ = put(16 * (size_t)Z);
+    o.twM = put(16 * (size_t)d.MM);           // a length N has fewer than N stage twiddles
+    o.twQ = put(16 * (size_t)d.NN);
+    o.gn = put(16 * (size_t)d.NN);
+    o.rev = put(2 * (size_t)d.MM);
+    o.colE = put(4 * (size_t)2 * KK * d.NN);
+    o.blkE = put(4 * (size_t)2 * KK * fx_nblk);
+    o.rowE = put(4 * (size_t)3 * KK * X);
+    o.minE = put(4 * (size_t)KK);
+    o.rowP = put(4 * (size_t)2 * KK * X * fx_nblk);
+    o.end = a;
+    return o;
+  }
 };
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -278,6 +359,33 @@ bool plan_run(RunHost& r, const char*& why) {
   if (!radix_ok(d.x_radix, xcap) || !radix_ok(d.z_radix, zcap)) { why = "x_radix/z_radix must be 8, 12 or 16 within the pass caps"; return false; }
   r.x_radix = d.x_radix ? d.x_radix : xcap;
   r.z_radix = d.z_radix ? d.z_radix : zcap;
+  // FP64 runs without tuning knobs step in 64-bit fixed point (mwf_fxpass.cuh) where one line of
+  // the z pass, all transforms of a z-subset, fits a CTA; the knobs belong to the FP64-arithmetic
+  // kernels, which the longest z lines (M4 beyond NN = 768) keep
+  r.fx = d.precision == MWF_FP64 && !d.xf_cols && !d.xi_cols && !d.z_lines && !d.x_radix && !d.z_radix &&
+         fx_z_smem(d.K0, d.NN, 1) <= zb_smem_budget(1);
+  if (r.fx) {
+    const size_t half = zb_smem_budget(2) - 1024, whole = zb_smem_budget(1) - 1024;   // the x passes' static arrays
+    const int slots = 2 * 152;                // CTAs of 256 threads that the chip holds
+    auto items = [&](int nb, int per) { return (d.NN + nb - 1) / nb * per; };
+    // widest column blocks (whole sectors of T) that still give every slot an item
+    r.fx_nb = kFxMaxCols;
+    while (r.fx_nb > 1 && (fx_xf_smem(d.MM, r.fx_nb) > half || (r.fx_nb > 2 && items(r.fx_nb, 2 * r.KK) < slots))) r.fx_nb /= 2;
+    r.fx_xf_nt = fx_xf_smem(d.MM, r.fx_nb) <= half ? 256 : 512;
+    r.fx_nblk = (d.NN + r.fx_nb - 1) / r.fx_nb + 1;    // and column n = 0 by itself
+    r.fx_xi_nb = kFxMaxCols;
+    while (r.fx_xi_nb > 1 && (fx_xi_smem(d.MM, r.fx_xi_nb) > (r.fx_xi_nb == 2 ? whole : half) ||
+                              (r.fx_xi_nb > 2 && items(r.fx_xi_nb, d.K0) < slots))) r.fx_xi_nb /= 2;
+    r.fx_xi_nt = fx_xi_smem(d.MM, r.fx_xi_nb) <= half ? 256 : 512;
+    // enough lines that a warp's butterflies fill its lanes, twice as many where that leaves two
+    // waves of items
+    r.fx_z_nt = fx_z_smem(d.K0, d.NN, 1) <= zb_smem_budget(2) ? 256 : 512;
+    const size_t zbud = zb_smem_budget(r.fx_z_nt == 256 ? 2 : 1);
+    const int g = std::max(1, 256 / d.NN);
+    int L = std::min(r.X / (2 * g) * 3 >= 2 * slots ? 2 * g : g, r.X);
+    while (L > 1 && fx_z_smem(d.K0, d.NN, L) > zbud) --L;
+    r.fx_lines = L;
+  }
   r.n_diag_xf = ((d.NN + r.xf_nb - 1) / r.xf_nb) * r.KK;
   r.n_diag_z = ((r.X + r.z_lx - 1) / r.z_lx) * 3;
   return true;
@@ -297,6 +405,10 @@ size_t run_bytes(RunHost& r, size_t base) {
   r.off_twQ = o; o = align_up(o + (size_t)r.d.NN * cb, 256);
   r.off_twZ = o; o = align_up(o + (size_t)r.Z * cb, 256);
   r.off_nst = o; o = align_up(o + sizeof(int), 256);
+  if (r.fx) {
+    r.off_fx = o;
+    o = r.fx_off().end;
+  }
   return o;
 }
 
@@ -309,10 +421,16 @@ struct Launch {
   int zbQ = 0;     // z pass: 0 = z_nonlinear_kernel, else the batched FP32 z pass for NN = zbQ
   int xbMM = 0;    // x passes: 0 = x_forward_kernel / x_inverse_kernel, else the subset-split
                    // FP32 kernels for MM = xbMM
+  bool fx = false;              // FP64 passes in fixed point
   bool persist_group = false;   // its runs can step in the persistent kernel instead (step mode)
 };
 
 cudaError_t launch_pass(const Launch& L, const RunDesc* runs, const WorkItem* items, int* err, cudaStream_t st) {
+  if (L.fx) {
+    if (L.kind == 0) return launch_x_forward_fx(L.nt, runs, items, L.nitems, L.smem, st);
+    if (L.kind == 1) return launch_z_fx(L.K0, L.nt, runs, items, L.nitems, L.smem, st);
+    return launch_x_inverse_fx(L.nt, runs, items, L.nitems, L.smem, st);
+  }
   if (L.kind == 0 && L.xbMM) return launch_x_forward_batched(L.xbMM, runs, items, L.nitems, L.smem, err, st);
   if (L.kind == 2 && L.xbMM) return launch_x_inverse_batched(L.xbMM, runs, items, L.nitems, L.smem, err, st);
   if (L.kind == 0)
@@ -472,6 +590,13 @@ int mwf_describe_run(const mwf_run_desc* d, mwf_run_plan* out) {
     p.xi_smem = (long long)xbi_smem(d->MM, r.xbi_nb);
     p.xf_items = ((d->NN + r.xbf_nb - 1) / r.xbf_nb) * d->K0;
     p.xi_items = ((d->NN + r.xbi_nb - 1) / r.xbi_nb) * d->K0;
+  } else if (r.fx) {
+    p.xf_cols = r.fx_nb;
+    p.xi_cols = r.fx_xi_nb;
+    p.xf_smem = (long long)fx_xf_smem(d->MM, r.fx_nb);
+    p.xi_smem = (long long)fx_xi_smem(d->MM, r.fx_xi_nb);
+    p.xf_items = (r.fx_nblk - 1) * 2 * r.KK;
+    p.xi_items = ((d->NN + r.fx_xi_nb - 1) / r.fx_xi_nb) * d->K0;
   } else {
     p.xf_cols = r.xf_nb;
     p.xi_cols = r.xi_nb;
@@ -485,6 +610,10 @@ int mwf_describe_run(const mwf_run_desc* d, mwf_run_plan* out) {
     p.z_ctas_per_sm = zb_blocks_per_sm(d->K0, d->NN);
     p.z_smem = (long long)zb_smem(d->K0, d->NN, r.zb_lx);
     p.z_items = (r.X + r.zb_lx - 1) / r.zb_lx;
+  } else if (r.fx) {
+    p.z_lines = r.fx_lines;
+    p.z_smem = (long long)fx_z_smem(d->K0, d->NN, r.fx_lines);
+    p.z_items = ((r.X + r.fx_lines - 1) / r.fx_lines) * 3;
   } else {
     p.z_lines = r.z_lx;
     p.z_smem = (long long)zpass_smem(prec, d->K0, r.z_ppt, r.z_nt);
@@ -558,7 +687,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
       Launch L{0, prec, 0, 0, nt, 0, items.size(), 0};
       for (int i = 0; i < n_runs; ++i) {
         const RunHost& r = h->runs[i];
-        if (r.persist != pset || r.d.precision != prec || r.x_nt != nt || r.xbf_nb) continue;
+        if (r.persist != pset || r.d.precision != prec || r.x_nt != nt || r.xbf_nb || r.fx) continue;
         for (int n0 = 0; n0 < r.d.NN; n0 += r.xf_nb)
           for (int f = 0; f < 2 * r.KK; ++f) items.push_back(WorkItem{i, n0, f, 0});
         L.smem = std::max(L.smem, xpass_smem(prec, (size_t)r.xf_nb * r.X));
@@ -585,7 +714,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
         Launch L{1, prec, K0, ppt, nt, 0, items.size(), 0};
         for (int i = 0; i < n_runs; ++i) {
           const RunHost& r = h->runs[i];
-          if (r.persist != pset || r.d.precision != prec || r.d.K0 != K0 || r.z_ppt != ppt || r.z_nt != nt || r.zb_lx) continue;
+          if (r.persist != pset || r.d.precision != prec || r.d.K0 != K0 || r.z_ppt != ppt || r.z_nt != nt || r.zb_lx || r.fx) continue;
           // FP32: one item per line block running the three z-subsets, summed (RunDesc::z_sum),
           // so the x-inverse pass reads one partial instead of three
           for (int x0 = 0; x0 < r.X; x0 += r.z_lx) {
@@ -615,7 +744,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
       Launch L{2, prec, 0, 0, nt, 0, items.size(), 0};
       for (int i = 0; i < n_runs; ++i) {
         const RunHost& r = h->runs[i];
-        if (r.persist != pset || r.d.precision != prec || r.x_nt != nt || r.xbi_nb) continue;
+        if (r.persist != pset || r.d.precision != prec || r.x_nt != nt || r.xbi_nb || r.fx) continue;
         for (int n0 = 0; n0 < r.d.NN; n0 += r.xi_nb)
           for (int k = 0; k < r.d.K0; ++k) items.push_back(WorkItem{i, n0, k, 0});
         L.smem = std::max(L.smem, xpass_smem(prec, (size_t)3 * r.xi_nb * r.X));
@@ -627,6 +756,33 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
   };
   build_groups(false);
   build_groups(true);
+  // FP64 runs in fixed point: one launch per pass and block size (and model, for the z pass)
+  for (int kind = 0; kind < 3; ++kind)
+    for (int K0 : {4, 6})
+      for (int nt : {256, 512}) {
+        if (kind != 1 && K0 == 6) continue;
+        Launch L{kind, 0, K0, 0, nt, 0, items.size(), 0};
+        L.fx = true;
+        for (int i = 0; i < n_runs; ++i) {
+          const RunHost& r = h->runs[i];
+          if (!r.fx) continue;
+          if (kind == 0 && r.fx_xf_nt == nt) {
+            for (int n0 = 0; n0 < r.d.NN; n0 += r.fx_nb)
+              for (int f = 0; f < 2 * r.KK; ++f) items.push_back(WorkItem{i, n0, f, 0});
+            L.smem = std::max(L.smem, fx_xf_smem(r.d.MM, r.fx_nb));
+          } else if (kind == 1 && r.fx_z_nt == nt && r.d.K0 == K0) {
+            for (int x0 = 0; x0 < r.X; x0 += r.fx_lines)
+              for (int sub = 0; sub < 3; ++sub) items.push_back(WorkItem{i, x0, sub, 0});
+            L.smem = std::max(L.smem, fx_z_smem(K0, r.d.NN, r.fx_lines));
+          } else if (kind == 2 && r.fx_xi_nt == nt) {
+            for (int n0 = 0; n0 < r.d.NN; n0 += r.fx_xi_nb)
+              for (int k = 0; k < r.d.K0; ++k) items.push_back(WorkItem{i, n0, k, 0});
+            L.smem = std::max(L.smem, fx_xi_smem(r.d.MM, r.fx_xi_nb));
+          }
+        }
+        L.nitems = (int)(items.size() - L.item_off);
+        if (L.nitems) h->launches.push_back(L);
+      }
   // the persistent step's items: a three-stage pipeline over groups of runs whose x-transformed
   // fields total at most kGroupBytes (the x forward of group p beside the z pass of group p-1 and
   // the x inverse of group p-2, each stage's lists merged in proportion), so every item's
@@ -805,9 +961,57 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
         ck(cudaMemcpy(h->arena + off, t.data(), t.size() * 4, cudaMemcpyHostToDevice), "twiddle upload");
       }
     };
-    up(r.off_twX, r.X);
+    if (!r.fx) up(r.off_twX, r.X);
     up(r.off_twQ, r.d.NN);
-    up(r.off_twZ, r.Z);
+    if (!r.fx) up(r.off_twZ, r.Z);
+    if (r.fx) {
+      const RunHost::FxOff fo = r.fx_off();
+      std::vector<int4> wX, wZ, tM, tQ, gn(r.d.NN);
+      std::vector<unsigned short> rev, unused;
+      // the double and the fixed-point tables of X and Z from one evaluation
+      auto table = [&](int N, size_t off_d, size_t off_fx, std::vector<int4>& w) {
+        const std::vector<long double> v = twiddles<long double>(N);
+        const std::vector<double> t(v.begin(), v.end());
+        w.resize(N);
+        for (int j = 0; j < N; ++j) w[j] = fx_twiddle(&v[2 * (size_t)j]);
+        ck(cudaMemcpy(h->arena + off_d, t.data(), t.size() * 8, cudaMemcpyHostToDevice), "twiddle upload");
+        ck(cudaMemcpy(h->arena + off_fx, w.data(), w.size() * sizeof(int4), cudaMemcpyHostToDevice), "twiddle upload");
+      };
+      table(r.X, r.off_twX, fo.twX, wX);
+      table(r.Z, r.off_twZ, fo.twZ, wZ);
+      if (!make_fx_plan(r.d.MM, wX, D.fx_planM, tM, rev) || !make_fx_plan(r.d.NN, wZ, D.fx_planQ, tQ, unused) ||
+          tM.size() > (size_t)r.d.MM || tQ.size() > (size_t)r.d.NN) {
+        rc = fail(MWF_ERR_SIZE, "run %d: no fixed-point FFT plan", i);
+        break;
+      }
+      // gamma n (the FP64 product) = mantissa in [1/2, 1) times 2^exponent
+      for (int n = 0; n < r.d.NN; ++n) {
+        int ex = 0;
+        const long long w = (long long)std::ldexp(std::frexp(r.d.gamma * n, &ex), 62);
+        const int l = (int)(unsigned)w;
+        gn[n] = make_int4((int)((w - l) >> 32), l, ex, 0);
+      }
+      auto put = [&](size_t off, const void* p, size_t bytes) {
+        if (bytes) ck(cudaMemcpy(h->arena + off, p, bytes, cudaMemcpyHostToDevice), "fixed-point table upload");
+      };
+      put(fo.twM, tM.data(), tM.size() * sizeof(int4));
+      put(fo.twQ, tQ.data(), tQ.size() * sizeof(int4));
+      put(fo.gn, gn.data(), gn.size() * sizeof(int4));
+      put(fo.rev, rev.data(), rev.size() * sizeof(unsigned short));
+      D.fx = 1;
+      D.fx_nb = r.fx_nb; D.fx_xi_nb = r.fx_xi_nb; D.fx_nblk = r.fx_nblk; D.fx_lines = r.fx_lines;
+      D.fx_twX = reinterpret_cast<const int4*>(h->arena + fo.twX);
+      D.fx_twZ = reinterpret_cast<const int4*>(h->arena + fo.twZ);
+      D.fx_twM = reinterpret_cast<const int4*>(h->arena + fo.twM);
+      D.fx_twQ = reinterpret_cast<const int4*>(h->arena + fo.twQ);
+      D.fx_gn = reinterpret_cast<const int4*>(h->arena + fo.gn);
+      D.fx_rev = reinterpret_cast<const unsigned short*>(h->arena + fo.rev);
+      D.fx_colE = reinterpret_cast<int*>(h->arena + fo.colE);
+      D.fx_blkE = reinterpret_cast<int*>(h->arena + fo.blkE);
+      D.fx_rowE = reinterpret_cast<int*>(h->arena + fo.rowE);
+      D.fx_minE = reinterpret_cast<int*>(h->arena + fo.minE);
+      D.fx_rowP = reinterpret_cast<float*>(h->arena + fo.rowP);
+    }
     const int one = 1;
     ck(cudaMemcpy(h->arena + r.off_nst, &one, sizeof(int), cudaMemcpyHostToDevice), "nst init");
   }

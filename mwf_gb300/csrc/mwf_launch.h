@@ -96,6 +96,20 @@ int persistent_grid(size_t smem);
 cudaError_t launch_persistent_step(const RunDesc* runs, const void* items, int n_items, int* counters, size_t smem,
                                    int grid, int* err, cudaStream_t st);
 
+// FP64 passes in fixed point (mwf_fxpass.cuh).  CTAs of 256 threads, two per SM, where an item fits
+// half an SM's shared memory, else 512 threads.
+// (lines, then the stage twiddles of the line length, then the z pass's scales)
+constexpr size_t fx_z_stride(int Q, int L) { return ((size_t)L * Q + 63) & ~(size_t)63; }
+constexpr size_t fx_z_smem(int K0, int Q, int L) {
+  const size_t kk = 3 * K0 - 1, np = (kk + 1) / 2, nt = np + kk;
+  return 16 * (nt * fx_z_stride(Q, L) + Q) + 4 * (size_t)L * (3 * nt + 9 + 3 + np + 1);
+}
+constexpr size_t fx_xf_smem(int MM, int nb) { return 16 * ((((size_t)3 * nb * MM + 7) & ~(size_t)7) + MM); }
+constexpr size_t fx_xi_smem(int MM, int nb) { return 16 * ((((size_t)9 * nb * MM + 7) & ~(size_t)7) + MM); }
+cudaError_t launch_x_forward_fx(int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st);
+cudaError_t launch_z_fx(int K0, int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st);
+cudaError_t launch_x_inverse_fx(int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st);
+
 // Physical-field z transform (one line of length Z <= kPhysVpt * kPhysThreads per CTA).
 constexpr int kPhysThreads = 256;
 constexpr int kPhysVpt = 12;
