@@ -69,7 +69,7 @@ struct FftPlanDev {
   FastDiv fns[MWF_MAX_STAGES];  // division by ns
 };
 
-// Plan of the in-place fixed-point transforms (mwf_fx.cuh) for one line length N = 2^a 3^b: stage s
+// Plan of the in-place transforms (mwf_fx.cuh, mwf_zwarp.cuh) for one line length N = 2^a 3^b: stage s
 // has butterflies of radix[s] elements stride[s] apart, stride[s] = N / (radix[0] ... radix[s]), and
 // its twiddles at tw_off[s] of the run's table, (radix - 1) stride of them.
 struct FxPlan {
@@ -80,6 +80,13 @@ struct FxPlan {
   int tw_off[MWF_MAX_STAGES];
   FastDiv fnb[MWF_MAX_STAGES];  // division by N / radix
   FastDiv fst[MWF_MAX_STAGES];  // division by stride
+  // mwf_zwarp.cuh: one pad element after every group of the last stage where its radix is even, so
+  // that element i lies at i + i / pad, LS elements a line; in those places stage s steps by
+  // step[s] within a butterfly and by bstep[s] from block to block
+  FastDiv fpad;
+  int LS;
+  int step[MWF_MAX_STAGES];
+  int bstep[MWF_MAX_STAGES];
 };
 constexpr int kFxMaxCols = 8;   // columns of an item of the fixed-point x passes
 
@@ -133,13 +140,26 @@ struct RunDesc {
   unsigned long long test_wait_ns;
   double diag_ct;               // threshold of the physical-space diagnostic
   FftPlanDev planX, planQ;
+  // FP32 runs whose z lines a warp transforms in place (mwf_zwarp.cuh): x lines per item (0: not
+  // used), plan and stage twiddles of NN
+  int zw_lines;
+  FxPlan zw_plan;
+  const float2* zw_tw;
+  // the same for the x passes (mwf_xwarp.cuh): columns per x-forward / x-inverse item (powers of two,
+  // 0: not used), field and derivative at once (2) or in turn (1), plan, twiddles and element order of MM
+  int xw_fnb, xw_inb, xw_nd;
+  FxPlan xw_plan;
+  const float2* xw_tw;
+  const unsigned short* xw_rev;
   // FP64 runs in fixed point (mwf_fxpass.cuh): columns per x-forward / x-inverse item (powers of
   // two), column blocks of the x forward, x lines per z item; twiddles e^{-2 pi i t/N} as fixed-point
-  // pairs (t < X, t < Z) and by stage for MM and NN; gamma n as mantissa and exponent; position ->
+  // pairs (t < X, t < Z) and by stage for MM and NN; gamma n and
+  // powers of alpha m as mantissa and exponent, alpha m and its square times `scale`; position ->
   // element of the digit-reversed x lines; the scales of what the passes store
   int fx;
   int fx_nb, fx_xi_nb, fx_nblk, fx_lines;
-  const int4 *fx_twX, *fx_twZ, *fx_twM, *fx_twQ, *fx_gn;
+  const int4 *fx_twX, *fx_twZ, *fx_twM, *fx_twQ, *fx_gn, *fx_mp;
+  const double2* fx_ms;
   const unsigned short* fx_rev;
   int *fx_colE, *fx_blkE, *fx_rowE, *fx_minE;
   float* fx_rowP;

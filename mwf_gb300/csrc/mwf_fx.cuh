@@ -156,6 +156,29 @@ __host__ __device__ __forceinline__ double fx_to_double(i64 q, int e) {
   return fx_value(b | (q < 0 ? 0x8000000000000000ull : 0ull));
 }
 
+// A factor w = (h 2^32 + l) 2^(e - 62) with the mantissa in [1/2, 1) (zero: h = l = 0).
+struct FxFactor { int h, l, e; };
+__host__ __device__ __forceinline__ FxFactor fx_factor(double w) {
+  const u64 b = fx_bits(w);
+  const int ex = (int)(b >> 52) & 0x7ff;
+  i64 m = (i64)(((b & 0xfffffffffffffull) | 0x10000000000000ull) << 9);
+  if ((i64)b < 0) m = -m;
+  if (ex == 0) m = 0;
+  const FxConst c = fx_split(m);
+  return FxFactor{c.h, c.l, ex - 1022};
+}
+// round(x m n 2^e) for factors m, n; |.| <= 2^61.  Two integer products on the mantissa in the place
+// of FP64 multiplications.
+__host__ __device__ __forceinline__ i64 fx_term(double x, FxFactor m, FxFactor n, int e) {
+  const u64 b = fx_bits(x);
+  const int ex = (int)(b >> 52) & 0x7ff;
+  i64 v = (i64)(((b & 0xfffffffffffffull) | 0x10000000000000ull) << 9);
+  v = fx_mulc(fx_mulc(v, FxConst{m.h, m.l}), FxConst{n.h, n.l});
+  v = fx_shift(v, ex - 1084 + m.e + n.e + e);
+  if (ex == 0) v = 0;
+  return (i64)b < 0 ? -v : v;
+}
+
 // Element index -> place: the low three bits (16-byte columns of a 128-byte row) are mixed with
 // the row, so strided butterflies spread over the banks without padding.
 __device__ __forceinline__ int fx_at(int i) { return i ^ ((i >> 3) & 7); }

@@ -1,9 +1,9 @@
 // The three passes of the FP64 timestep in 64-bit fixed point (mwf_fx.cuh; sm_103a).
 //
-//   x forward  item (run, first column n0, field f in 0 .. 2KK-1): the field's spectral values are
-//              formed in FP64 (var_mpt2spec + vel_addlam + var_spec_grad, variables.f90:390-434,
-//              600-612), scaled to integers column by column and transformed in x as three
-//              interleaved subsets x = s + 3q of length MM (tra_spec2phys, transform.fftw5.f90:69-78)
+//   x forward  item (run, first column n0, field f in 0 .. 2KK-1): the field's spectral values
+//              (var_mpt2spec + vel_addlam + var_spec_grad, variables.f90:390-434, 600-612) as
+//              integers with one scale per column, transformed in x as three interleaved subsets
+//              x = s + 3q of length MM (tra_spec2phys, transform.fftw5.f90:69-78)
 //   z          item (run, first x line x0, z-subset s): all NPAIR + KK backward transforms of the
 //              lines z = s + 3q, the Galerkin coupling (udotgradu, modes.M4.f90:14-28 /
 //              modes.M6.f90:14-20) as integer products, NPAIR forward transforms and the split
@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDes
   extern __shared__ __align__(128) unsigned char smem_raw[];
   longlong2* buf = reinterpret_cast<longlong2*>(smem_raw);       // line (l, s) at (3 l + s) MM
   __shared__ int colE[kFxMaxCols];
+  __shared__ FxFactor colN[2][kFxMaxCols];
   const WorkItem wi = items[blockIdx.x];
   const RunDesc& R = runs[wi.run];
   if (!R.active) return;
@@ -146,30 +147,61 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDes
     if (lane == 0) {
       colE[l] = e;
       R.fx_colE[(size_t)f * NN + n] = e;
+      const double n1 = R.gamma * n, kb = kbeta<double>(k), sg = deriv ? -1.0 : 1.0;
+      colN[0][l] = fx_factor(comp == 0 ? -sg * n1 : comp == 2 ? sg : 1.0);
+      colN[1][l] = fx_factor(comp == 0 ? sg * kb : comp == 2 ? sg * (kb * n1) : n1 * n1);
     }
   }
   __syncthreads();
 
   // fill: a = value at m = j, b = value at m = j - MM; subset s of the column has the length-MM
-  // spectrum e^{2 pi i js/X} (a + e^{-2 pi i s/3} b)
+  // spectrum e^{2 pi i js/X} (a + e^{-2 pi i s/3} b).  A value is i^rot (A m1^pa na + B m1^pb nb) of two
+  // MPT coefficients A, B, m1 = alpha m, with na, nb of the column alone:
+  //   u = i (-n1 psi + k1 m1 phi),  w = i (m1 psi + k1 n1 phi),  v = (m1^2 + n1^2) phi,
+  // and i m1 times that for the derivatives.  The products are integer ones on the mantissas: with
+  // FP64 multiplications the fill was bound by the FP64 pipe and took 57 % of the pass.
   const int4* __restrict__ xm = R.fx_twX;             // e^{-2 pi i t/X}
   const FastDiv fMM = make_fastdiv(MM);
-  const double kb1 = kbeta<double>(k);
+  const int d = deriv ? 1 : 0;
+  const int pa = d + (comp == 0 ? 0 : comp == 1 ? 2 : 1), pb = d + (comp == 0 ? 1 : 0);
+  const bool rot = (comp != 1) != deriv;
+  const size_t rowa = (size_t)(comp == 1 ? k + K0 - 1 : k) * M, rowb = (size_t)(k + K0 - 1) * M;
+  const bool hasb = k >= 1;
+  const int4* __restrict__ mp = R.fx_mp;              // (alpha m)^p, p = 0 .. 3, as (h, l, exponent)
+#pragma unroll 1
   for (int e = threadIdx.x; e < nb * MM; e += NT) {
     const int l = fMM.div(e);
     const int j = e - l * MM;
     const int ce = colE[l];
-    const double n1 = R.gamma * (n0 + l);
-    auto value = [&](int m) {
-      const double m1 = R.alpha * m;
-      double2 v = mpt_to_field_w<double>(R, c, fs, m, n0 + l, true, m1, n1, kb1);
-      if (deriv) v = make_double2(-v.y * m1, v.x * m1);
+    const FxFactor na = colN[0][l], nbf = colN[1][l];
+    const double2* __restrict__ col = c + (size_t)(n0 + l) * K * M;
+    const int jn = j == 0 ? 0 : MM - j;               // -m of the negative wavenumber
+    const int msn = j == 0 ? 0 : M - jn;
+    const double2 zero = make_double2(0.0, 0.0);
+    const double2 A = col[rowa + j], An = col[rowa + msn];
+    const double2 B = hasb ? col[rowb + j] : zero, Bn = hasb ? col[rowb + msn] : zero;
+    auto form = [&](double2 a, double2 b, int m, bool neg) {
+      const int4 ta = mp[pa * MM + m], tb = mp[pb * MM + m];
+      const FxFactor fa{ta.x, ta.y, ta.z}, fb{tb.x, tb.y, tb.z};
+      i64 xa = fx_term(a.x, fa, na, ce), ya = fx_term(a.y, fa, na, ce);
+      i64 xb = fx_term(b.x, fb, nbf, ce), yb = fx_term(b.y, fb, nbf, ce);
+      if (neg && (pa & 1)) { xa = -xa; ya = -ya; }
+      if (neg && (pb & 1)) { xb = -xb; yb = -yb; }
       longlong2 q;
-      q.x = fx_from_double(v.x, ce);
-      q.y = fx_from_double(v.y, ce);
+      q.x = rot ? -(ya + yb) : xa + xb;
+      q.y = rot ? xa + xb : ya + yb;
       return q;
     };
-    const longlong2 a = value(j);
+    longlong2 a = form(A, B, j, false);
+    if (j == 0 && n0 + l == 0) {                      // mean flows: u_k = psi_k, w_k = phi_k (k >= 1), and the base flow
+      double2 v = zero;
+      if (!deriv && comp != 1 && k >= 1) {
+        v = comp == 0 ? A : B;
+        if (k == 1) v.x += comp == 0 ? R.cth : R.sth;
+      }
+      a.x = fx_from_double(v.x, ce);
+      a.y = fx_from_double(v.y, ce);
+    }
     const int base = 3 * l * MM + j;
     if (j == 0) {
       buf[fx_at(base)] = a;
@@ -177,7 +209,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDes
       buf[fx_at(base + 2 * MM)] = a;
       continue;
     }
-    const longlong2 b = value(j - MM);
+    const longlong2 b = form(An, Bn, jn, true);
     buf[fx_at(base)] = cadd(a, b);
     constexpr FxConst s3 = fx_const(kFxSqrt34);
     const i64 rx = fx_mulc(b.x, s3), ry = fx_mulc(b.y, s3);
@@ -639,6 +671,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_inverse_fx_kernel(const RunDes
   longlong2* buf = reinterpret_cast<longlong2*>(smem_raw);       // line (comp, l, s) at ((comp nb + l) 3 + s) MM
   __shared__ u64 norm[9 * kFxMaxCols];
   __shared__ int sh[9 * kFxMaxCols];
+  __shared__ double colw[3][kFxMaxCols];              // gamma n, (-1)^k k b gamma n and (gamma n)^2, times the scale
   const WorkItem wi = items[blockIdx.x];
   const RunDesc& R = runs[wi.run];
   if (!R.active) return;
@@ -653,6 +686,12 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_inverse_fx_kernel(const RunDes
   const FastDiv fMM = make_fastdiv(MM);
   int4* tw = reinterpret_cast<int4*>(buf + ((9 * nbw * MM + 7) & ~7));
   for (int i = threadIdx.x; i < MM; i += NT) tw[i] = R.fx_twM[i];
+  if (threadIdx.x < nb) {
+    const double n1 = R.gamma * (n0 + threadIdx.x), n1s = n1 * R.scale;
+    colw[0][threadIdx.x] = n1s;
+    colw[1][threadIdx.x] = kbeta<double>(k) * n1s;
+    colw[2][threadIdx.x] = n1 * n1s;
+  }
   const int lw = 31 - __clz(nbw);
   const int l_ = threadIdx.x & (nbw - 1);
   int ref[3];                                         // scale of each field's sum of partials
@@ -714,64 +753,70 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_inverse_fx_kernel(const RunDes
   const int4* __restrict__ xm = R.fx_twX;
   double2* __restrict__ c = reinterpret_cast<double2*>(R.c);
   double2* __restrict__ onl = reinterpret_cast<double2*>(R.onl);
+  // The wavenumbers carry the 1/(3MM 3NN) of the transforms and come from tables: forming them in place
+  // (conversions, products, the scale) made 44 FP64 operations per mode, which bound the pass.
   const double* __restrict__ ilhs = R.inv_lhs;
   const double* __restrict__ rhs = R.rhs;
+  const double hdt = R.dt / 2.0;
+  const double2* __restrict__ mtab = R.fx_ms;         // (alpha m, (alpha m)^2) times the scale
   const bool first = *R.nst != 0;
-  const double hdt = R.dt / 2.0, alpha = R.alpha, gamma = R.gamma, scale = R.scale;
   const double kb1 = kbeta<double>(k);
   const FastDiv fM = make_fastdiv(M);
+#pragma unroll 1
   for (int o = threadIdx.x; o < nb * M; o += NT) {
     const int l = fM.div(o);
     const int ms = o - l * M;
     const int n = n0 + l;
+    const double n1 = colw[0][l], kn = colw[1][l], n2 = colw[2][l];
+    const int eu = ref[0] + sh[l * 3], ev = ref[1] + sh[(nb + l) * 3], ew = ref[2] + sh[(2 * nb + l) * 3];
     const int m = signed_m(ms, MM, M);
     const size_t i0 = ((size_t)n * K + k) * M + ms;
     const size_t i1 = i0 + (size_t)(K0 - 1) * M;
+    const double2 zero = make_double2(0.0, 0.0);
+    // operands of both slots first, so that their loads overlap the rest
+    const double2 c0 = c[i0], o0 = onl[i0];
+    const double r0 = rhs[i0], v0 = ilhs[i0];
+    const double2 c1 = k > 0 ? c[i1] : zero, o1 = k > 0 ? onl[i1] : zero;
+    const double r1 = k > 0 ? rhs[i1] : 0.0, v1 = k > 0 ? ilhs[i1] : 0.0;
+    const double2 mt = mtab[m < 0 ? -m : m];
     const int j = m >= 0 ? m : m + MM;
     const int4 w1 = xm[m >= 0 ? m : m + X], w2 = xm[m >= 0 ? 2 * m : 2 * m + X];
-    double2 sp[3];
-#pragma unroll
-    for (int comp = 0; comp < 3; ++comp) {
-      const int base = (comp * nb + l) * 3 * MM + j;
+    auto comp = [&](int i, int e, bool bad) {
+      const int base = (i * nb + l) * 3 * MM + j;
       const longlong2 F0 = buf[fx_at(base)], F1 = buf[fx_at(base + MM)], F2 = buf[fx_at(base + 2 * MM)];
       const longlong2 v = cadd(cadd(F0, fx_cmul<false>(F1, w1)), fx_cmul<false>(F2, w2));
-      const int e = ref[comp] + sh[(comp * nb + l) * 3];
-      sp[comp].x = fx_to_double(v.x, e) * scale;
-      sp[comp].y = fx_to_double(v.y, e) * scale;
-      if (ref[comp] < kFxNan / 2) sp[comp].x = sp[comp].y = nan("");
-    }
-    const double2 su = sp[0], sv = sp[1], sw = sp[2];
-    const double m1 = alpha * m, n1 = gamma * n;
-    const double H = (-alpha * m * alpha * m) + (-gamma * n * gamma * n);
+      return bad ? make_double2(nan(""), nan("")) : make_double2(fx_to_double(v.x, e), fx_to_double(v.y, e));
+    };
+    const double2 su = comp(0, eu, ref[0] < kFxNan / 2), sw = comp(2, ew, ref[2] < kFxNan / 2);
+    const double2 sv = k > 0 ? comp(1, ev, ref[1] < kFxNan / 2) : zero;
+    const double m1 = m < 0 ? -mt.x : mt.x, km = kb1 * m1, H = mt.y + n2;
     // var_spec2mpt (variables.f90:455-464)
     double2 nphi, npsi;
-    nphi.x = -(su.y * m1 * kb1 + sw.y * n1 * kb1) + sv.x * H;
-    nphi.y = (su.x * m1 * kb1 + sw.x * n1 * kb1) + sv.y * H;
-    npsi.x = sw.y * m1 - su.y * n1;
-    npsi.y = -(sw.x * m1 - su.x * n1);
+    nphi.x = -fma(su.y, km, fma(sw.y, kn, sv.x * H));
+    nphi.y = fma(su.x, km, fma(sw.x, kn, -(sv.y * H)));
+    npsi.x = fma(sw.y, m1, -(su.y * n1));
+    npsi.y = fma(-sw.x, m1, su.x * n1);
     if (ms == 0 && n == 0) {   // mean modes (variables.f90:467-479)
-      if (k == 0) npsi = make_double2(0.0, 0.0);
+      if (k == 0) npsi = zero;
       else {
-        npsi = make_double2(-su.x, -su.y);
-        nphi = make_double2(-sw.x, -sw.y);
+        npsi = make_double2(-su.x * R.scale, -su.y * R.scale);
+        nphi = make_double2(-sw.x * R.scale, -sw.y * R.scale);
       }
     }
     // AB2 / implicit update (velocity.f90:24-40); onl <- nl
-#pragma unroll
-    for (int which = 0; which < 2; ++which) {
-      if (which == 1 && k == 0) continue;
-      const size_t idx = which == 0 ? i0 : i1;
-      const double2 nlv = which == 0 ? npsi : nphi;
-      const double2 cold = c[idx];
-      const double2 ov = first ? nlv : onl[idx];
-      const double rr = rhs[idx], il = ilhs[idx];
-      double cx_ = rr * cold.x + hdt * (3.0 * nlv.x - ov.x);
-      double cy_ = rr * cold.y + hdt * (3.0 * nlv.y - ov.y);
-      cx_ *= il;
-      cy_ *= il;
-      if (k == 0 && which == 0 && ms == 0 && n == 0) cx_ = 0.0;
-      c[idx] = make_double2(cx_, cy_);
-      onl[idx] = nlv;
+    auto update = [&](double rr, double il, double cv, double nv, double ov) { return fma(rr, cv, hdt * fma(3.0, nv, -ov)) * il; };
+    {
+      const double2 ov = first ? npsi : o0;
+      double x = update(r0, v0, c0.x, npsi.x, ov.x);
+      const double y = update(r0, v0, c0.y, npsi.y, ov.y);
+      if (k == 0 && ms == 0 && n == 0) x = 0.0;
+      c[i0] = make_double2(x, y);
+      onl[i0] = npsi;
+    }
+    if (k > 0) {
+      const double2 ov = first ? nphi : o1;
+      c[i1] = make_double2(update(r1, v1, c1.x, nphi.x, ov.x), update(r1, v1, c1.y, nphi.y, ov.y));
+      onl[i1] = nphi;
     }
   }
 }

@@ -128,18 +128,69 @@ int4 fx_twiddle(const long double* v) {
   return make_int4(out[0], out[1], out[2], out[3]);
 }
 
-// Radix plan of the in-place fixed-point transforms, its stage twiddles (from w, the table of
-// e^{-2 pi i t/(3N)}) and the element that each position of a digit-reversed line holds.
-bool make_fx_plan(int N, const std::vector<int4>& w, FxPlan& pl, std::vector<int4>& tw, std::vector<unsigned short>& rev) {
-  if (!is_23_smooth(N) || N < 2) return false;
+// Radices of the in-place transforms of length N.  Fixed point: 8s (of 16 two 4s), then 9s and 3s; a
+// butterfly of 12 or 16 would not leave 128 registers a thread.  FP32: the fewest stages of radices up
+// to 16, the balanced choice among them.
+std::vector<int> inplace_radices(int N, bool fx) {
   std::vector<int> rad;
-  int rest = N;
-  auto take = [&](int r) { rad.push_back(r); rest /= r; };
-  while (rest % 8 == 0 && rest != 16) take(8);          // 16 = 4 x 4, not 8 x 2
-  while (rest % 4 == 0) take(4);
-  while (rest % 2 == 0) take(2);
-  while (rest % 9 == 0) take(9);
-  while (rest % 3 == 0) take(3);
+  if (fx) {
+    int rest = N;
+    auto take = [&](int r) { rad.push_back(r); rest /= r; };
+    while (rest % 8 == 0 && rest != 16) take(8);
+    while (rest % 4 == 0) take(4);
+    while (rest % 2 == 0) take(2);
+    while (rest % 9 == 0) take(9);
+    while (rest % 3 == 0) take(3);
+    return rad;
+  }
+  static const int all[] = {16, 12, 9, 8, 6, 4, 3, 2};
+  std::vector<int> cur, best;
+  int best_sum = 0;
+  // depth-first over non-increasing radices: fewest stages, then the least padding (the last radix,
+  // below), then the smallest sum
+  auto padding = [](const std::vector<int>& r) {
+    for (int v : r)
+      if (v % 2) return 0;
+    return 48 / r[0];
+  };
+  auto go = [&](auto&& self, int rest, int from) -> void {
+    if (rest == 1) {
+      int sum = 0;
+      for (int r : cur) sum += r;
+      const int a = padding(cur), b = best.empty() ? 0 : padding(best);
+      if (best.empty() || cur.size() < best.size() || (cur.size() == best.size() && (a < b || (a == b && sum < best_sum)))) {
+        best = cur;
+        best_sum = sum;
+      }
+      return;
+    }
+    if (!best.empty() && cur.size() + 1 > best.size()) return;
+    for (int k = from; k < 8; ++k)
+      if (rest % all[k] == 0) {
+        cur.push_back(all[k]);
+        self(self, rest / all[k], k);
+        cur.pop_back();
+      }
+  };
+  go(go, N, 0);
+  // last: an odd radix, which needs no padding (mwf_zwarp.cuh), else the largest
+  size_t last = 0;
+  for (size_t k = 0; k < best.size(); ++k)
+    if (best[k] % 2) { last = k; break; }
+  std::swap(best[last], best.back());
+  return best;
+}
+int inplace_line(int N) {                    // padded line length
+  const int last = inplace_radices(N, false).back();
+  return last % 2 ? N : N + N / last;
+}
+
+// Plan of the in-place transforms of length N, its stage twiddles (from w, the table of
+// e^{-2 pi i t/(3N)}) and the element that each position of a digit-reversed line holds.
+template <typename W>
+bool make_fx_plan(int N, const std::vector<W>& w, bool fx, FxPlan& pl, std::vector<W>& tw, std::vector<unsigned short>& rev) {
+  if (!is_23_smooth(N) || N < 2) return false;
+  const std::vector<int> rad = inplace_radices(N, fx);
   if ((int)rad.size() > MWF_MAX_STAGES) return false;
   memset(&pl, 0, sizeof pl);
   pl.N = N;
@@ -157,6 +208,14 @@ bool make_fx_plan(int N, const std::vector<int4>& w, FxPlan& pl, std::vector<int
       for (int r = 1; r < rad[s]; ++r)
         for (int j = 0; j < st; ++j) tw.push_back(w[(size_t)3 * (j * r * (N / span) % N)]);
     span = st;
+  }
+  const int pad = rad.back() % 2 ? 0 : rad.back();
+  pl.fpad = pad ? make_fastdiv(pad) : FastDiv{0, 2};      // without padding: quotient 0
+  auto place = [&](int i) { return pad ? i + i / pad : i; };
+  pl.LS = place(N);
+  for (int s = 0; s < pl.nst; ++s) {
+    pl.step[s] = pl.stride[s] == 1 ? 1 : place(pl.stride[s]);
+    pl.bstep[s] = place(pl.stride[s] * rad[s]);
   }
   rev.assign(N, 0);
   for (int p = 0; p < N; ++p) {
@@ -235,13 +294,21 @@ struct RunHost {
   int xbf_nb = 0, xbi_nb = 0;   // columns per item of the subset-split FP32 x passes (0: not used)
   bool persist = false;         // all three passes batched: the run steps in the persistent kernel
   int active = 1;    // host copy of RunDesc::active
+  // FP32 z pass with a warp per line (mwf_zwarp.cuh): lines per item (0: not used), subsets at once,
+  // block size
+  int zw_lines = 0, zw_ns = 0, zw_nt = 0;
+  size_t off_zw = 0;
+  // FP32 x passes with a warp per line (mwf_xwarp.cuh): columns per item (0: not used), field and
+  // derivative at once or in turn, block sizes
+  int xw_fnb = 0, xw_inb = 0, xw_nd = 0, xw_fnt = 0, xw_int = 0;
+  size_t off_xw = 0;
   // FP64 in fixed point (mwf_fxpass.cuh): columns and block sizes of the x passes, lines and block
   // size of the z pass
   bool fx = false;
   int fx_nb = 0, fx_xi_nb = 0, fx_lines = 0, fx_nblk = 0;
   int fx_xf_nt = 0, fx_z_nt = 0, fx_xi_nt = 0;
   size_t off_fx = 0;
-  struct FxOff { size_t twX, twZ, twM, twQ, gn, rev, colE, blkE, rowE, minE, rowP, end; };
+  struct FxOff { size_t twX, twZ, twM, twQ, gn, mp, ms, rev, colE, blkE, rowE, minE, rowP, end; };
   FxOff fx_off() const {
     FxOff o;
     size_t a = off_fx;
@@ -251,6 +318,8 @@ struct RunHost {
     o.twM = put(16 * (size_t)d.MM);           // a length N has fewer than N stage twiddles
     o.twQ = put(16 * (size_t)d.NN);
     o.gn = put(16 * (size_t)d.NN);
+    o.mp = put(16 * (size_t)4 * d.MM);
+    o.ms = put(16 * (size_t)d.MM);
     o.rev = put(2 * (size_t)d.MM);
     o.colE = put(4 * (size_t)2 * KK * d.NN);
     o.blkE = put(4 * (size_t)2 * KK * fx_nblk);
@@ -359,6 +428,39 @@ bool plan_run(RunHost& r, const char*& why) {
   if (!radix_ok(d.x_radix, xcap) || !radix_ok(d.z_radix, zcap)) { why = "x_radix/z_radix must be 8, 12 or 16 within the pass caps"; return false; }
   r.x_radix = d.x_radix ? d.x_radix : xcap;
   r.z_radix = d.z_radix ? d.z_radix : zcap;
+  // FP32 runs that neither the batched z pass takes nor a knob directs to z_nonlinear_kernel: a warp
+  // per line
+  r.zw_lines = 0;
+  if (d.precision == MWF_FP32 && !r.zb_lx && !d.z_radix && !d.z_lines) {
+    const int LS = inplace_line(d.NN);
+    auto need = [&](int L) { return zw_smem(d.K0, d.NN, LS, r.zw_ns, L); };
+    r.zw_ns = 3;
+    if (need(1) > zb_smem_budget(1)) r.zw_ns = 1;
+    if (need(1) <= zb_smem_budget(1)) {
+      r.zw_nt = need(1) <= zb_smem_budget(2) ? 256 : 512;
+      const size_t zbud = zb_smem_budget(r.zw_nt == 256 ? 2 : 1);
+      const int g = std::max(1, 128 / d.NN);    // lines of a warp's task
+      int L = 1;
+      while (L < r.X && L * d.NN < 512 && need(L + 1) <= zbud) ++L;
+      r.zw_lines = L > g ? L / g * g : L;
+    }
+  }
+  r.xw_fnb = r.xw_inb = 0;
+  if (d.precision == MWF_FP32 && !xb && !d.x_radix && !d.xf_cols && !d.xi_cols) {
+    const int LS = inplace_line(d.MM);
+    const size_t half = zb_smem_budget(2), whole = zb_smem_budget(1);
+    // eight columns at most; narrower where field and derivative do not fit half an SM together,
+    // and then, from four columns (a sector of T) down, one after the other
+    r.xw_nd = 2;
+    r.xw_fnb = 8;
+    while (r.xw_fnb > 4 && (xw_fsmem(d.MM, LS, 2, r.xw_fnb) > half || r.xw_fnb / 2 >= d.NN)) r.xw_fnb /= 2;
+    if (xw_fsmem(d.MM, LS, 2, r.xw_fnb) > half) r.xw_nd = 1;
+    while (r.xw_fnb > 1 && xw_fsmem(d.MM, LS, r.xw_nd, r.xw_fnb) > half) r.xw_fnb /= 2;
+    r.xw_fnt = xw_fsmem(d.MM, LS, r.xw_nd, r.xw_fnb) <= half ? 256 : 512;
+    r.xw_inb = 8;
+    while (r.xw_inb > 1 && (xw_ismem(d.MM, LS, r.xw_inb) > (r.xw_inb <= 4 ? whole : half) || r.xw_inb / 2 >= d.NN)) r.xw_inb /= 2;
+    r.xw_int = xw_ismem(d.MM, LS, r.xw_inb) <= half ? 256 : 512;
+  }
   // FP64 runs without tuning knobs step in 64-bit fixed point (mwf_fxpass.cuh) where one line of
   // the z pass, all transforms of a z-subset, fits a CTA; the knobs belong to the FP64-arithmetic
   // kernels, which the longest z lines (M4 beyond NN = 768) keep
@@ -405,6 +507,15 @@ size_t run_bytes(RunHost& r, size_t base) {
   r.off_twQ = o; o = align_up(o + (size_t)r.d.NN * cb, 256);
   r.off_twZ = o; o = align_up(o + (size_t)r.Z * cb, 256);
   r.off_nst = o; o = align_up(o + sizeof(int), 256);
+  if (r.zw_lines) {
+    r.off_zw = o;
+    o = align_up(o + sizeof(float2) * (size_t)r.d.NN, 256);
+  }
+  if (r.xw_fnb) {
+    r.off_xw = o;
+    o = align_up(o + sizeof(float2) * (size_t)r.d.MM, 256);
+    o = align_up(o + sizeof(unsigned short) * (size_t)r.d.MM, 256);
+  }
   if (r.fx) {
     r.off_fx = o;
     o = r.fx_off().end;
@@ -422,6 +533,8 @@ struct Launch {
   int xbMM = 0;    // x passes: 0 = x_forward_kernel / x_inverse_kernel, else the subset-split
                    // FP32 kernels for MM = xbMM
   bool fx = false;              // FP64 passes in fixed point
+  int zw_ns = 0;                // FP32 z pass with a warp per line: subsets at once
+  bool xw = false;              // FP32 x passes with a warp per line
   bool persist_group = false;   // its runs can step in the persistent kernel instead (step mode)
 };
 
@@ -431,6 +544,10 @@ cudaError_t launch_pass(const Launch& L, const RunDesc* runs, const WorkItem* it
     if (L.kind == 1) return launch_z_fx(L.K0, L.nt, runs, items, L.nitems, L.smem, st);
     return launch_x_inverse_fx(L.nt, runs, items, L.nitems, L.smem, st);
   }
+  if (L.xw)
+    return L.kind == 0 ? launch_x_forward_warp(L.nt, runs, items, L.nitems, L.smem, st)
+                       : launch_x_inverse_warp(L.nt, runs, items, L.nitems, L.smem, st);
+  if (L.zw_ns) return launch_z_warp(L.K0, L.zw_ns, L.nt, runs, items, L.nitems, L.smem, st);
   if (L.kind == 0 && L.xbMM) return launch_x_forward_batched(L.xbMM, runs, items, L.nitems, L.smem, err, st);
   if (L.kind == 2 && L.xbMM) return launch_x_inverse_batched(L.xbMM, runs, items, L.nitems, L.smem, err, st);
   if (L.kind == 0)
@@ -590,6 +707,14 @@ int mwf_describe_run(const mwf_run_desc* d, mwf_run_plan* out) {
     p.xi_smem = (long long)xbi_smem(d->MM, r.xbi_nb);
     p.xf_items = ((d->NN + r.xbf_nb - 1) / r.xbf_nb) * d->K0;
     p.xi_items = ((d->NN + r.xbi_nb - 1) / r.xbi_nb) * d->K0;
+  } else if (r.xw_fnb) {
+    const int LS = inplace_line(d->MM);
+    p.xf_cols = r.xw_fnb;
+    p.xi_cols = r.xw_inb;
+    p.xf_smem = (long long)xw_fsmem(d->MM, LS, r.xw_nd, r.xw_fnb);
+    p.xi_smem = (long long)xw_ismem(d->MM, LS, r.xw_inb);
+    p.xf_items = ((d->NN + r.xw_fnb - 1) / r.xw_fnb) * d->K0;
+    p.xi_items = ((d->NN + r.xw_inb - 1) / r.xw_inb) * d->K0;
   } else if (r.fx) {
     p.xf_cols = r.fx_nb;
     p.xi_cols = r.fx_xi_nb;
@@ -610,6 +735,10 @@ int mwf_describe_run(const mwf_run_desc* d, mwf_run_plan* out) {
     p.z_ctas_per_sm = zb_blocks_per_sm(d->K0, d->NN);
     p.z_smem = (long long)zb_smem(d->K0, d->NN, r.zb_lx);
     p.z_items = (r.X + r.zb_lx - 1) / r.zb_lx;
+  } else if (r.zw_lines) {
+    p.z_lines = r.zw_lines;
+    p.z_smem = (long long)zw_smem(d->K0, d->NN, inplace_line(d->NN), r.zw_ns, r.zw_lines);
+    p.z_items = (r.X + r.zw_lines - 1) / r.zw_lines;
   } else if (r.fx) {
     p.z_lines = r.fx_lines;
     p.z_smem = (long long)fx_z_smem(d->K0, d->NN, r.fx_lines);
@@ -687,7 +816,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
       Launch L{0, prec, 0, 0, nt, 0, items.size(), 0};
       for (int i = 0; i < n_runs; ++i) {
         const RunHost& r = h->runs[i];
-        if (r.persist != pset || r.d.precision != prec || r.x_nt != nt || r.xbf_nb || r.fx) continue;
+        if (r.persist != pset || r.d.precision != prec || r.x_nt != nt || r.xbf_nb || r.xw_fnb || r.fx) continue;
         for (int n0 = 0; n0 < r.d.NN; n0 += r.xf_nb)
           for (int f = 0; f < 2 * r.KK; ++f) items.push_back(WorkItem{i, n0, f, 0});
         L.smem = std::max(L.smem, xpass_smem(prec, (size_t)r.xf_nb * r.X));
@@ -714,7 +843,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
         Launch L{1, prec, K0, ppt, nt, 0, items.size(), 0};
         for (int i = 0; i < n_runs; ++i) {
           const RunHost& r = h->runs[i];
-          if (r.persist != pset || r.d.precision != prec || r.d.K0 != K0 || r.z_ppt != ppt || r.z_nt != nt || r.zb_lx || r.fx) continue;
+          if (r.persist != pset || r.d.precision != prec || r.d.K0 != K0 || r.z_ppt != ppt || r.z_nt != nt || r.zb_lx || r.zw_lines || r.fx) continue;
           // FP32: one item per line block running the three z-subsets, summed (RunDesc::z_sum),
           // so the x-inverse pass reads one partial instead of three
           for (int x0 = 0; x0 < r.X; x0 += r.z_lx) {
@@ -744,7 +873,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
       Launch L{2, prec, 0, 0, nt, 0, items.size(), 0};
       for (int i = 0; i < n_runs; ++i) {
         const RunHost& r = h->runs[i];
-        if (r.persist != pset || r.d.precision != prec || r.x_nt != nt || r.xbi_nb || r.fx) continue;
+        if (r.persist != pset || r.d.precision != prec || r.x_nt != nt || r.xbi_nb || r.xw_inb || r.fx) continue;
         for (int n0 = 0; n0 < r.d.NN; n0 += r.xi_nb)
           for (int k = 0; k < r.d.K0; ++k) items.push_back(WorkItem{i, n0, k, 0});
         L.smem = std::max(L.smem, xpass_smem(prec, (size_t)3 * r.xi_nb * r.X));
@@ -756,6 +885,37 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
   };
   build_groups(false);
   build_groups(true);
+  // FP32 x passes with a warp per line: one launch per pass and block size
+  for (int kind : {0, 2})
+    for (int nt : {256, 512}) {
+      Launch L{kind, 1, 0, 0, nt, 0, items.size(), 0};
+      L.xw = true;
+      for (int i = 0; i < n_runs; ++i) {
+        const RunHost& r = h->runs[i];
+        if (!r.xw_fnb || (kind == 0 ? r.xw_fnt : r.xw_int) != nt) continue;
+        const int nb = kind == 0 ? r.xw_fnb : r.xw_inb, LS = inplace_line(r.d.MM);
+        for (int n0 = 0; n0 < r.d.NN; n0 += nb)
+          for (int k = 0; k < r.d.K0; ++k) items.push_back(WorkItem{i, n0, k, 0});
+        L.smem = std::max(L.smem, kind == 0 ? xw_fsmem(r.d.MM, LS, r.xw_nd, nb) : xw_ismem(r.d.MM, LS, nb));
+      }
+      L.nitems = (int)(items.size() - L.item_off);
+      if (L.nitems) h->launches.push_back(L);
+    }
+  // FP32 z pass with a warp per line: one launch per model, subsets at once and block size
+  for (int K0 : {4, 6})
+    for (int ns : {3, 1})
+      for (int nt : {256, 512}) {
+        Launch L{1, 1, K0, 0, nt, 0, items.size(), 0};
+        L.zw_ns = ns;
+        for (int i = 0; i < n_runs; ++i) {
+          const RunHost& r = h->runs[i];
+          if (!r.zw_lines || r.d.K0 != K0 || r.zw_ns != ns || r.zw_nt != nt) continue;
+          for (int x0 = 0; x0 < r.X; x0 += r.zw_lines) items.push_back(WorkItem{i, x0, 0, 0});
+          L.smem = std::max(L.smem, zw_smem(K0, r.d.NN, inplace_line(r.d.NN), ns, r.zw_lines));
+        }
+        L.nitems = (int)(items.size() - L.item_off);
+        if (L.nitems) h->launches.push_back(L);
+      }
   // FP64 runs in fixed point: one launch per pass and block size (and model, for the z pass)
   for (int kind = 0; kind < 3; ++kind)
     for (int K0 : {4, 6})
@@ -964,10 +1124,36 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
     if (!r.fx) up(r.off_twX, r.X);
     up(r.off_twQ, r.d.NN);
     if (!r.fx) up(r.off_twZ, r.Z);
+    // in-place FP32 transforms of length N, their stage twiddles at off
+    auto inplace = [&](int N, FxPlan& pl, size_t off, std::vector<unsigned short>& rev) {
+      const std::vector<float> v = twiddles<float>(3 * N);
+      std::vector<float2> w(3 * (size_t)N), t;
+      for (size_t j = 0; j < w.size(); ++j) w[j] = make_float2(v[2 * j], v[2 * j + 1]);
+      if (!make_fx_plan(N, w, false, pl, t, rev) || t.size() > (size_t)N) {
+        rc = fail(MWF_ERR_SIZE, "run %d: no in-place FFT plan", i);
+        return;
+      }
+      if (!t.empty()) ck(cudaMemcpy(h->arena + off, t.data(), t.size() * sizeof(float2), cudaMemcpyHostToDevice), "twiddle upload");
+    };
+    std::vector<unsigned short> rev;
+    if (r.zw_lines) {
+      inplace(r.d.NN, D.zw_plan, r.off_zw, rev);
+      D.zw_lines = r.zw_lines;
+      D.zw_tw = reinterpret_cast<const float2*>(h->arena + r.off_zw);
+    }
+    if (r.xw_fnb) {
+      const size_t off_rev = align_up(r.off_xw + sizeof(float2) * (size_t)r.d.MM, 256);
+      inplace(r.d.MM, D.xw_plan, r.off_xw, rev);
+      if (!rev.empty()) ck(cudaMemcpy(h->arena + off_rev, rev.data(), rev.size() * sizeof(unsigned short), cudaMemcpyHostToDevice), "order upload");
+      D.xw_fnb = r.xw_fnb; D.xw_inb = r.xw_inb; D.xw_nd = r.xw_nd;
+      D.xw_tw = reinterpret_cast<const float2*>(h->arena + r.off_xw);
+      D.xw_rev = reinterpret_cast<const unsigned short*>(h->arena + off_rev);
+    }
+    if (rc != MWF_OK) break;
     if (r.fx) {
       const RunHost::FxOff fo = r.fx_off();
       std::vector<int4> wX, wZ, tM, tQ, gn(r.d.NN);
-      std::vector<unsigned short> rev, unused;
+      std::vector<unsigned short> unused;
       // the double and the fixed-point tables of X and Z from one evaluation
       auto table = [&](int N, size_t off_d, size_t off_fx, std::vector<int4>& w) {
         const std::vector<long double> v = twiddles<long double>(N);
@@ -979,17 +1165,27 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
       };
       table(r.X, r.off_twX, fo.twX, wX);
       table(r.Z, r.off_twZ, fo.twZ, wZ);
-      if (!make_fx_plan(r.d.MM, wX, D.fx_planM, tM, rev) || !make_fx_plan(r.d.NN, wZ, D.fx_planQ, tQ, unused) ||
+      if (!make_fx_plan(r.d.MM, wX, true, D.fx_planM, tM, rev) || !make_fx_plan(r.d.NN, wZ, true, D.fx_planQ, tQ, unused) ||
           tM.size() > (size_t)r.d.MM || tQ.size() > (size_t)r.d.NN) {
         rc = fail(MWF_ERR_SIZE, "run %d: no fixed-point FFT plan", i);
         break;
       }
-      // gamma n (the FP64 product) = mantissa in [1/2, 1) times 2^exponent
-      for (int n = 0; n < r.d.NN; ++n) {
+      // mantissa in [1/2, 1) and exponent of gamma n and of the powers 0 .. 3 of alpha m
+      auto factor = [](double v) {
         int ex = 0;
-        const long long w = (long long)std::ldexp(std::frexp(r.d.gamma * n, &ex), 62);
+        const long long w = (long long)std::ldexp(std::frexp(v, &ex), 62);
         const int l = (int)(unsigned)w;
-        gn[n] = make_int4((int)((w - l) >> 32), l, ex, 0);
+        return make_int4((int)((w - l) >> 32), l, ex, 0);
+      };
+      std::vector<int4> mp(4 * (size_t)r.d.MM);
+      std::vector<double> ms(2 * (size_t)r.d.MM);
+      for (int n = 0; n < r.d.NN; ++n) gn[n] = factor(r.d.gamma * n);
+      for (int m = 0; m < r.d.MM; ++m) {
+        const double m1 = r.d.alpha * m;
+        double v = 1.0;
+        for (int p = 0; p < 4; ++p, v *= m1) mp[(size_t)p * r.d.MM + m] = factor(v);
+        ms[2 * (size_t)m] = m1 * D.scale;
+        ms[2 * (size_t)m + 1] = m1 * m1 * D.scale;
       }
       auto put = [&](size_t off, const void* p, size_t bytes) {
         if (bytes) ck(cudaMemcpy(h->arena + off, p, bytes, cudaMemcpyHostToDevice), "fixed-point table upload");
@@ -997,6 +1193,8 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
       put(fo.twM, tM.data(), tM.size() * sizeof(int4));
       put(fo.twQ, tQ.data(), tQ.size() * sizeof(int4));
       put(fo.gn, gn.data(), gn.size() * sizeof(int4));
+      put(fo.mp, mp.data(), mp.size() * sizeof(int4));
+      put(fo.ms, ms.data(), ms.size() * 8);
       put(fo.rev, rev.data(), rev.size() * sizeof(unsigned short));
       D.fx = 1;
       D.fx_nb = r.fx_nb; D.fx_xi_nb = r.fx_xi_nb; D.fx_nblk = r.fx_nblk; D.fx_lines = r.fx_lines;
@@ -1005,6 +1203,8 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
       D.fx_twM = reinterpret_cast<const int4*>(h->arena + fo.twM);
       D.fx_twQ = reinterpret_cast<const int4*>(h->arena + fo.twQ);
       D.fx_gn = reinterpret_cast<const int4*>(h->arena + fo.gn);
+      D.fx_mp = reinterpret_cast<const int4*>(h->arena + fo.mp);
+      D.fx_ms = reinterpret_cast<const double2*>(h->arena + fo.ms);
       D.fx_rev = reinterpret_cast<const unsigned short*>(h->arena + fo.rev);
       D.fx_colE = reinterpret_cast<int*>(h->arena + fo.colE);
       D.fx_blkE = reinterpret_cast<int*>(h->arena + fo.blkE);
@@ -1769,6 +1969,8 @@ extern "C" int mwf_step_noalloc(const mwf_run_desc* d, double* c_re, double* c_i
   r.d = *d;
   const char* why = "";
   if (!plan_run(r, why)) return fail(MWF_ERR_SIZE, "mwf_step_noalloc: %s", why);
+  r.fx = false;                // the kernels below need no more than run_bytes' basic arrays
+  r.zw_lines = r.xw_fnb = 0;
   const int prec = d->precision;
   const size_t cb = prec == MWF_FP64 ? 16 : 8;
   // work items of the three passes

@@ -110,6 +110,22 @@ cudaError_t launch_x_forward_fx(int nt, const RunDesc* runs, const WorkItem* ite
 cudaError_t launch_z_fx(int K0, int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st);
 cudaError_t launch_x_inverse_fx(int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st);
 
+// FP32 z pass with a warp per line (mwf_zwarp.cuh): ns z-subsets at once (3 where they fit), in CTAs
+// of 256 threads, two per SM, or of 512.
+// (LS: padded line length, FxPlan).
+constexpr size_t zw_smem(int K0, int Q, int LS, int ns, int L) {
+  const size_t kk = 3 * K0 - 1, nt = (kk + 1) / 2 + kk;
+  return 8 * (nt * ns * L * LS + Q);
+}
+cudaError_t launch_z_warp(int K0, int ns, int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st);
+
+// FP32 x passes with a warp per line (mwf_xwarp.cuh), in CTAs of 256 threads, two (x forward) or three
+// (x inverse) per SM where shared memory allows, or of 512.
+constexpr size_t xw_fsmem(int MM, int LS, int nd, int nb) { return 8 * ((size_t)3 * nd * nb * LS + MM); }
+constexpr size_t xw_ismem(int MM, int LS, int nb) { return 8 * ((size_t)9 * nb * LS + MM); }
+cudaError_t launch_x_forward_warp(int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st);
+cudaError_t launch_x_inverse_warp(int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st);
+
 // Physical-field z transform (one line of length Z <= kPhysVpt * kPhysThreads per CTA).
 constexpr int kPhysThreads = 256;
 constexpr int kPhysVpt = 12;
