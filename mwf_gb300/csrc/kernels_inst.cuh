@@ -116,10 +116,9 @@ cudaError_t MWF_FN(launch_x_inverse)(int nt, const RunDesc* runs, const WorkItem
   return cudaErrorInvalidValue;
 }
 
-cudaError_t MWF_FN(launch_energy)(const RunDesc* runs, int run, double* partial, int nparts, double* out,
-                                  cudaStream_t st) {
-  energy_partial_kernel<MWF_T><<<nparts, 256, 0, st>>>(runs, run, partial);
-  energy_final_kernel<<<1, 32, 0, st>>>(partial, nparts, out);
+cudaError_t MWF_FN(launch_energy)(const RunDesc* runs, int run, double* partial, int nparts, int* flag,
+                                  unsigned* ticket, const int* err, HostOut* out, cudaStream_t st) {
+  energy_kernel<MWF_T><<<nparts, kEnergyThreads, 0, st>>>(runs, run, partial, flag, ticket, err, out);
   return cudaGetLastError();
 }
 
@@ -131,11 +130,19 @@ cudaError_t MWF_FN(launch_ref_to_dev)(const double* re, const double* im, void* 
   return cudaGetLastError();
 }
 
-cudaError_t MWF_FN(launch_dev_to_ref)(const void* in, double* re, double* im, int K, int M, int NN,
-                                      cudaStream_t st) {
+cudaError_t MWF_FN(launch_host_to_dev)(const double* re, const double* im, void* out, int K, int M, int NN,
+                                       cudaStream_t st) {
   const size_t tot = (size_t)K * M * NN;
   const int blocks = (int)((tot + 255) / 256 < 152 * 16 ? (tot + 255) / 256 : 152 * 16);
-  dev_to_ref_kernel<MWF_T><<<blocks, 256, 0, st>>>(reinterpret_cast<const cx<MWF_T>*>(in), re, im, K, M, NN);
+  host_to_dev_kernel<MWF_T><<<blocks, 256, 0, st>>>(re, im, reinterpret_cast<cx<MWF_T>*>(out), K, M, NN);
+  return cudaGetLastError();
+}
+
+cudaError_t MWF_FN(launch_dev_to_ref)(const void* in, double* re, double* im, int K, int M, int NN,
+                                      cudaStream_t st, const int* err, HostOut* out) {
+  const size_t tot = (size_t)K * M * NN;
+  const int blocks = (int)((tot + 255) / 256 < 152 * 16 ? (tot + 255) / 256 : 152 * 16);
+  dev_to_ref_kernel<MWF_T><<<blocks, 256, 0, st>>>(reinterpret_cast<const cx<MWF_T>*>(in), re, im, K, M, NN, err, out);
   return cudaGetLastError();
 }
 
@@ -143,11 +150,6 @@ cudaError_t MWF_FN(launch_imposesym)(const RunDesc* runs, int run, int mode, int
   const size_t tot = (size_t)M * NN;
   const int blocks = (int)((tot + 255) / 256 < 152 * 8 ? (tot + 255) / 256 : 152 * 8);
   imposesym_kernel<MWF_T><<<blocks, 256, 0, st>>>(runs, run, mode);
-  return cudaGetLastError();
-}
-
-cudaError_t MWF_FN(launch_nonfinite)(const RunDesc* runs, int run, int* flag, cudaStream_t st) {
-  nonfinite_kernel<MWF_T><<<152 * 4, 256, 0, st>>>(runs, run, flag);
   return cudaGetLastError();
 }
 

@@ -175,6 +175,14 @@ struct WorkItem {
   int pad; // x-forward: 1 = without the laminar base flow (diagnostics)
 };
 
+// What a call reads back, in host memory that the device writes to.
+struct HostOut {
+  double value;
+  int flag;
+  int err;
+};
+constexpr int kEnergyThreads = 64;   // small blocks spread a small state's FP64 operations over the SMs
+
 // One item of the persistent FP32 step (mwf_persist.cuh): a pass work item and its kind and size,
 // code = kind << 8 | size index (kinds: 0 x forward, 1 z pass of M4, 2 z pass of M6, 3 x inverse;
 // size index of MM or NN in {32, 48, 64, 96, 128, 192, 256}).

@@ -1,5 +1,6 @@
 // C-ABI implementation (include/mwf_gpu.h): plans, FP64 tables, device arena, work lists,
 // CUDA-graph replay of the timestep, state copies and the energy diagnostic.
+#include <cuda.h>
 #include <cmath>
 #include <cstddef>
 #include <cstdarg>
@@ -575,8 +576,9 @@ struct mwf_handle {
   WorkItem* d_diag_items = nullptr;  // scratch for one run's diagnostic work items
   int* d_err = nullptr;
   int* d_flag = nullptr;
+  unsigned* d_ticket = nullptr;  // blocks of the energy kernel that have finished
   double* d_partial = nullptr;
-  double* d_eout = nullptr;
+  HostOut* h_out = nullptr;      // pinned host memory that kernels write a call's outcome to
   double* d_stage = nullptr;     // 2 * max(csz) doubles for state copies
   size_t stage_elems = 0;
   std::vector<Launch> launches;
@@ -593,7 +595,7 @@ struct mwf_handle {
   cudaGraphExec_t graph1 = nullptr;   // one step
   cudaGraphExec_t graphG = nullptr;   // kGraphSteps steps
   static constexpr int kGraphSteps = 16;
-  static constexpr int kEnergyParts = 256;
+  static constexpr int kEnergyParts = 2432;  // blocks of the energy kernel: sixteen per SM
 };
 
 namespace {
@@ -646,12 +648,43 @@ int build_graph(mwf_handle* h, int steps, cudaGraphExec_t* out) {
   return MWF_OK;
 }
 
-int check_device_err(mwf_handle* h) {
-  int herr = 0;
-  CK(cudaMemcpyAsync(&herr, h->d_err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+// Wait for the stream; the error word is in h_out->err by then.
+int finish_call(mwf_handle* h) {
   CK(cudaStreamSynchronize(h->stream));
+  const int herr = h->h_out->err;
   if (herr) return fail(MWF_ERR_DEVICE, "kernel reported internal error flags 0x%x", herr);
   return MWF_OK;
+}
+
+int check_device_err(mwf_handle* h) {
+  CK(cudaMemcpyAsync(&h->h_out->err, h->d_err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  return finish_call(h);
+}
+
+// Whether the device may access the n doubles at p in place: they lie within one pinned host
+// allocation (or registration).
+bool device_reads_host(const double* p, size_t n) {
+  static const auto attr = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      fn = nullptr;
+    return reinterpret_cast<CUresult (*)(void*, CUpointer_attribute, CUdeviceptr)>(fn);
+  }();
+  if (!attr) return false;
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (a.type != cudaMemoryTypeHost || a.devicePointer != (const void*)p) return false;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  if (attr(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, (CUdeviceptr)p) != CUDA_SUCCESS ||
+      attr(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, (CUdeviceptr)p) != CUDA_SUCCESS)
+    return false;
+  return (CUdeviceptr)p >= start && (CUdeviceptr)p + n * sizeof(double) <= start + size;
 }
 
 void free_handle(mwf_handle* h) {
@@ -659,6 +692,7 @@ void free_handle(mwf_handle* h) {
   if (h->graph1) cudaGraphExecDestroy(h->graph1);
   if (h->graphG) cudaGraphExecDestroy(h->graphG);
   if (h->arena) cudaFree(h->arena);
+  if (h->h_out) cudaFreeHost(h->h_out);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
 }
@@ -1017,14 +1051,21 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
   size_t max_diag = 0;
   for (const RunHost& r : h->runs) max_diag = std::max(max_diag, (size_t)(r.n_diag_xf + r.n_diag_z));
   const size_t off_diag = o; o = align_up(o + sizeof(WorkItem) * max_diag, 256);
-  const size_t off_err = o; o = align_up(o + 2 * sizeof(int), 256);
-  const size_t off_part = o; o = align_up(o + sizeof(double) * (mwf_handle::kEnergyParts + 1), 256);
+  const size_t off_err = o; o = align_up(o + 3 * sizeof(int), 256);
+  const size_t off_part = o; o = align_up(o + sizeof(double) * mwf_handle::kEnergyParts, 256);
   const size_t off_stage = o; o = align_up(o + sizeof(double) * 2 * h->stage_elems, 256);
   h->arena_bytes = o;
   if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
     free_handle(h);
     return fail(MWF_ERR_CUDA, "stream creation failed");
   }
+  if (cudaHostAlloc(&h->h_out, sizeof(HostOut), cudaHostAllocMapped) != cudaSuccess) {
+    cudaGetLastError();
+    h->h_out = nullptr;
+    free_handle(h);
+    return fail(MWF_ERR_NOMEM, "cudaHostAlloc failed");
+  }
+  memset(h->h_out, 0, sizeof(HostOut));
   if (cudaMalloc(&h->arena, o) != cudaSuccess) {
     cudaGetLastError();
     h->arena = nullptr;
@@ -1037,7 +1078,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
   h->d_err = reinterpret_cast<int*>(h->arena + off_err);
   h->d_flag = h->d_err + 1;
   h->d_partial = reinterpret_cast<double*>(h->arena + off_part);
-  h->d_eout = h->d_partial + mwf_handle::kEnergyParts;
+  h->d_ticket = reinterpret_cast<unsigned*>(h->d_err + 2);
   h->d_stage = reinterpret_cast<double*>(h->arena + off_stage);
   h->d_pitems = h->arena + off_pitems;
   h->n_pitems = (int)pitems.size();
@@ -1245,19 +1286,51 @@ static int check_run(mwf_handle* h, int run) {
   return MWF_OK;
 }
 
+// State copies between the caller's split arrays (reference layout) and array `off` of run r, queued
+// on the handle's stream.  Pinned arrays are accessed by the conversion kernel itself, in place of
+// two staging copies per direction and the copy of the error word: get_state of a 27 KB, 1.8 MB and
+// 45 MB array pair took 21.8, 42.5 and 536 us with copies and takes 14.0, 33 and 493 us.
+static int state_in(mwf_handle* h, const RunHost& r, size_t off, const double* re, const double* im) {
+  const bool f64 = r.d.precision == MWF_FP64;
+  cudaError_t e;
+  if (device_reads_host(re, r.csz) && device_reads_host(im, r.csz)) {
+    e = f64 ? launch_host_to_dev_f64(re, im, h->arena + off, r.K, r.M, r.d.NN, h->stream)
+            : launch_host_to_dev_f32(re, im, h->arena + off, r.K, r.M, r.d.NN, h->stream);
+  } else {
+    double* sre = h->d_stage;
+    double* sim = h->d_stage + h->stage_elems;
+    CK(cudaMemcpyAsync(sre, re, r.csz * 8, cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync(sim, im, r.csz * 8, cudaMemcpyHostToDevice, h->stream));
+    e = f64 ? launch_ref_to_dev_f64(sre, sim, h->arena + off, r.K, r.M, r.d.NN, h->stream)
+            : launch_ref_to_dev_f32(sre, sim, h->arena + off, r.K, r.M, r.d.NN, h->stream);
+  }
+  if (e != cudaSuccess) return fail(MWF_ERR_CUDA, "state conversion: %s", cudaGetErrorString(e));
+  return MWF_OK;
+}
+
+// The error word follows into h_out (finish_call).
+static int state_out(mwf_handle* h, const RunHost& r, size_t off, double* re, double* im) {
+  const bool f64 = r.d.precision == MWF_FP64;
+  const bool direct = device_reads_host(re, r.csz) && device_reads_host(im, r.csz);
+  double* sre = direct ? re : h->d_stage;
+  double* sim = direct ? im : h->d_stage + h->stage_elems;
+  const cudaError_t e = f64 ? launch_dev_to_ref_f64(h->arena + off, sre, sim, r.K, r.M, r.d.NN, h->stream, h->d_err, h->h_out)
+                            : launch_dev_to_ref_f32(h->arena + off, sre, sim, r.K, r.M, r.d.NN, h->stream, h->d_err, h->h_out);
+  if (e != cudaSuccess) return fail(MWF_ERR_CUDA, "state conversion: %s", cudaGetErrorString(e));
+  if (!direct) {
+    CK(cudaMemcpyAsync(re, sre, r.csz * 8, cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaMemcpyAsync(im, sim, r.csz * 8, cudaMemcpyDeviceToHost, h->stream));
+  }
+  return MWF_OK;
+}
+
 int mwf_set_state(mwf_handle* h, int run, const double* re, const double* im) {
   int rc = check_run(h, run);
   if (rc) return rc;
   if (!re || !im) return fail(MWF_ERR_ARG, "mwf_set_state: null state array");
   const RunHost& r = h->runs[run];
-  double* sre = h->d_stage;
-  double* sim = h->d_stage + h->stage_elems;
-  CK(cudaMemcpyAsync(sre, re, r.csz * 8, cudaMemcpyHostToDevice, h->stream));
-  CK(cudaMemcpyAsync(sim, im, r.csz * 8, cudaMemcpyHostToDevice, h->stream));
-  cudaError_t e = r.d.precision == MWF_FP64
-                      ? launch_ref_to_dev_f64(sre, sim, h->arena + r.off_c, r.K, r.M, r.d.NN, h->stream)
-                      : launch_ref_to_dev_f32(sre, sim, h->arena + r.off_c, r.K, r.M, r.d.NN, h->stream);
-  if (e != cudaSuccess) return fail(MWF_ERR_CUDA, "state conversion: %s", cudaGetErrorString(e));
+  rc = state_in(h, r, r.off_c, re, im);
+  if (rc) return rc;
   CK(cudaStreamSynchronize(h->stream));
   return MWF_OK;
 }
@@ -1267,15 +1340,8 @@ int mwf_get_state(mwf_handle* h, int run, double* re, double* im) {
   if (rc) return rc;
   if (!re || !im) return fail(MWF_ERR_ARG, "mwf_get_state: null state array");
   const RunHost& r = h->runs[run];
-  double* sre = h->d_stage;
-  double* sim = h->d_stage + h->stage_elems;
-  cudaError_t e = r.d.precision == MWF_FP64
-                      ? launch_dev_to_ref_f64(h->arena + r.off_c, sre, sim, r.K, r.M, r.d.NN, h->stream)
-                      : launch_dev_to_ref_f32(h->arena + r.off_c, sre, sim, r.K, r.M, r.d.NN, h->stream);
-  if (e != cudaSuccess) return fail(MWF_ERR_CUDA, "state conversion: %s", cudaGetErrorString(e));
-  CK(cudaMemcpyAsync(re, sre, r.csz * 8, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaMemcpyAsync(im, sim, r.csz * 8, cudaMemcpyDeviceToHost, h->stream));
-  return check_device_err(h);
+  rc = state_out(h, r, r.off_c, re, im);
+  return rc ? rc : finish_call(h);
 }
 
 int mwf_get_history(mwf_handle* h, int run, double* re, double* im, int* euler_next) {
@@ -1283,16 +1349,10 @@ int mwf_get_history(mwf_handle* h, int run, double* re, double* im, int* euler_n
   if (rc) return rc;
   if (!re || !im || !euler_next) return fail(MWF_ERR_ARG, "mwf_get_history: null argument");
   const RunHost& r = h->runs[run];
-  double* sre = h->d_stage;
-  double* sim = h->d_stage + h->stage_elems;
-  cudaError_t e = r.d.precision == MWF_FP64
-                      ? launch_dev_to_ref_f64(h->arena + r.off_onl, sre, sim, r.K, r.M, r.d.NN, h->stream)
-                      : launch_dev_to_ref_f32(h->arena + r.off_onl, sre, sim, r.K, r.M, r.d.NN, h->stream);
-  if (e != cudaSuccess) return fail(MWF_ERR_CUDA, "history conversion: %s", cudaGetErrorString(e));
-  CK(cudaMemcpyAsync(re, sre, r.csz * 8, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaMemcpyAsync(im, sim, r.csz * 8, cudaMemcpyDeviceToHost, h->stream));
+  rc = state_out(h, r, r.off_onl, re, im);
+  if (rc) return rc;
   CK(cudaMemcpyAsync(euler_next, h->arena + r.off_nst, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-  return check_device_err(h);
+  return finish_call(h);
 }
 
 int mwf_set_history(mwf_handle* h, int run, const double* re, const double* im, int euler_next) {
@@ -1300,14 +1360,8 @@ int mwf_set_history(mwf_handle* h, int run, const double* re, const double* im, 
   if (rc) return rc;
   if (!re || !im) return fail(MWF_ERR_ARG, "mwf_set_history: null argument");
   const RunHost& r = h->runs[run];
-  double* sre = h->d_stage;
-  double* sim = h->d_stage + h->stage_elems;
-  CK(cudaMemcpyAsync(sre, re, r.csz * 8, cudaMemcpyHostToDevice, h->stream));
-  CK(cudaMemcpyAsync(sim, im, r.csz * 8, cudaMemcpyHostToDevice, h->stream));
-  cudaError_t e = r.d.precision == MWF_FP64
-                      ? launch_ref_to_dev_f64(sre, sim, h->arena + r.off_onl, r.K, r.M, r.d.NN, h->stream)
-                      : launch_ref_to_dev_f32(sre, sim, h->arena + r.off_onl, r.K, r.M, r.d.NN, h->stream);
-  if (e != cudaSuccess) return fail(MWF_ERR_CUDA, "history conversion: %s", cudaGetErrorString(e));
+  rc = state_in(h, r, r.off_onl, re, im);
+  if (rc) return rc;
   const int v = euler_next ? 1 : 0;
   CK(cudaMemcpyAsync(h->arena + r.off_nst, &v, sizeof(int), cudaMemcpyHostToDevice, h->stream));
   CK(cudaStreamSynchronize(h->stream));
@@ -1439,19 +1493,17 @@ int mwf_energy(mwf_handle* h, int run, double* e) {
   if (rc) return rc;
   if (!e) return fail(MWF_ERR_ARG, "mwf_energy: null output");
   const RunHost& r = h->runs[run];
-  CK(cudaMemsetAsync(h->d_flag, 0, sizeof(int), h->stream));
-  cudaError_t ce = r.d.precision == MWF_FP64 ? launch_nonfinite_f64(h->d_runs, run, h->d_flag, h->stream)
-                                             : launch_nonfinite_f32(h->d_runs, run, h->d_flag, h->stream);
-  if (ce != cudaSuccess) return fail(MWF_ERR_CUDA, "non-finite check: %s", cudaGetErrorString(ce));
-  ce = r.d.precision == MWF_FP64
-           ? launch_energy_f64(h->d_runs, run, h->d_partial, mwf_handle::kEnergyParts, h->d_eout, h->stream)
-           : launch_energy_f32(h->d_runs, run, h->d_partial, mwf_handle::kEnergyParts, h->d_eout, h->stream);
+  const size_t pts = (size_t)r.M * r.d.NN;
+  const int parts = (int)std::min<size_t>(mwf_handle::kEnergyParts, (pts + kEnergyThreads - 1) / kEnergyThreads);
+  const cudaError_t ce =
+      r.d.precision == MWF_FP64
+          ? launch_energy_f64(h->d_runs, run, h->d_partial, parts, h->d_flag, h->d_ticket, h->d_err, h->h_out, h->stream)
+          : launch_energy_f32(h->d_runs, run, h->d_partial, parts, h->d_flag, h->d_ticket, h->d_err, h->h_out, h->stream);
   if (ce != cudaSuccess) return fail(MWF_ERR_CUDA, "energy launch: %s", cudaGetErrorString(ce));
-  int flag = 0;
-  CK(cudaMemcpyAsync(e, h->d_eout, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaMemcpyAsync(&flag, h->d_flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-  rc = check_device_err(h);
+  rc = finish_call(h);
   if (rc) return rc;
+  const int flag = h->h_out->flag;
+  *e = h->h_out->value;
   if (flag) return fail(MWF_ERR_NONFINITE, "run %d: state contains NaN/Inf", run);
   return MWF_OK;
 }

@@ -896,18 +896,28 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 1024 / NT : 512 / NT) x_i
 // w_f = 1 for u_0, w_0 and 1/2 otherwise (epos, velocity.f90:115-126).  FP64 with
 // Neumaier-compensated per-thread sums and a pairwise tree across the block.
 // ---------------------------------------------------------------------------------------
+// The state is checked for NaN and infinities (every coefficient, also the ones no field
+// reads) on the way, and the block that finishes last adds the partials, pairwise in a fixed order, and
+// writes the outcome to the host word `out` (mapped memory): one launch and no copy, where a memset,
+// a separate check, a serial final sum and three copies took 40 us per call.
 template <typename T>
-__global__ void energy_partial_kernel(const RunDesc* __restrict__ runs, int run, double* partial) {
+__global__ void __launch_bounds__(kEnergyThreads) energy_kernel(const RunDesc* __restrict__ runs, int run, double* partial,
+                                                                 int* flag, unsigned* ticket, const int* err, HostOut* out) {
   using C = cx<T>;
   const RunDesc& R = runs[run];
   const C* __restrict__ c = reinterpret_cast<const C*>(R.c);
-  const int M = R.M, NN = R.NN, KK = R.KK, K0 = R.K0, MM = R.MM;
+  const int M = R.M, NN = R.NN, KK = R.KK, K = R.K, K0 = R.K0, MM = R.MM;
   const size_t npt = (size_t)NN * M;
   double sum = 0.0, comp = 0.0;
+  int bad = 0;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < npt; e += (size_t)gridDim.x * blockDim.x) {
     const int n = (int)(e / M);
     const int ms = (int)(e - (size_t)n * M);
     const int m = signed_m(ms, MM, M);
+    for (int k = 0; k < K; ++k) {
+      const C v = c[((size_t)n * K + k) * M + ms];
+      bad |= !isfinite(v.x) || !isfinite(v.y);
+    }
     for (int fs = 0; fs < KK; ++fs) {
       const double w = (fs == 0 || fs == 2 * K0 - 1) ? 1.0 : 0.5;
       const C v = mpt_to_field<T>(R, c, fs, m, n, false);
@@ -925,26 +935,35 @@ __global__ void energy_partial_kernel(const RunDesc* __restrict__ runs, int run,
       sum = y;
     }
   }
-  __shared__ double red[1024];
-  red[threadIdx.x] = sum + comp;
-  __syncthreads();
-  for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
+  __shared__ double red[kEnergyThreads];
+  __shared__ bool last;
+  auto tree = [&](double v) {
+    red[threadIdx.x] = v;
     __syncthreads();
+    for (int h = kEnergyThreads / 2; h > 0; h >>= 1) {
+      if ((int)threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
+      __syncthreads();
+    }
+  };
+  tree(sum + comp);
+  bad = __syncthreads_or(bad);
+  if (threadIdx.x == 0) {
+    partial[blockIdx.x] = red[0];
+    if (bad) atomicOr(flag, 1);
+    __threadfence();
+    last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;      // wraps to 0 for the next call
+    __threadfence();
   }
-  if (threadIdx.x == 0) partial[blockIdx.x] = red[0];
-}
-
-static __global__ void energy_final_kernel(const double* partial, int nparts, double* out) {
-  if (threadIdx.x != 0) return;
-  double sum = 0.0, comp = 0.0;
-  for (int i = 0; i < nparts; ++i) {
-    const double t = partial[i];
-    const double y = sum + t;
-    comp += (fabs(sum) >= fabs(t)) ? (sum - y) + t : (t - y) + sum;
-    sum = y;
+  __syncthreads();
+  if (!last) return;
+  double v = 0.0;
+  for (unsigned i = threadIdx.x; i < gridDim.x; i += kEnergyThreads) v += __ldcg(&partial[i]);
+  tree(v);
+  if (threadIdx.x == 0) {
+    out->value = red[0];
+    out->flag = atomicExch(flag, 0);
+    out->err = *err;
   }
-  *out = sum + comp;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -966,9 +985,26 @@ __global__ void ref_to_dev_kernel(const double* __restrict__ re, const double* _
   }
 }
 
+// The same from host arrays that the device reads in place: it walks the reference layout, so the
+// reads over the host link are contiguous, and scatters into device memory.
+template <typename T>
+__global__ void host_to_dev_kernel(const double* __restrict__ re, const double* __restrict__ im,
+                                   cx<T>* __restrict__ out, int K, int M, int NN) {
+  const size_t tot = (size_t)K * M * NN;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < tot; e += (size_t)gridDim.x * blockDim.x) {
+    const int k = (int)(e % K);
+    const size_t r = e / K;
+    const int m = (int)(r % M);
+    const int n = (int)(r / M);
+    out[((size_t)n * K + k) * M + m] = mk<T>(T(re[e]), T(im[e]));
+  }
+}
+
+// out, err: if given, the device error word is passed to the host with the state.
 template <typename T>
 __global__ void dev_to_ref_kernel(const cx<T>* __restrict__ in, double* __restrict__ re,
-                                  double* __restrict__ im, int K, int M, int NN) {
+                                  double* __restrict__ im, int K, int M, int NN, const int* err, HostOut* out) {
+  if (out && blockIdx.x == 0 && threadIdx.x == 0) out->err = *err;
   const size_t tot = (size_t)K * M * NN;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < tot; e += (size_t)gridDim.x * blockDim.x) {
     // e enumerates the reference layout (k fastest, then m, then n)
@@ -1033,21 +1069,6 @@ __global__ void imposesym_kernel(const RunDesc* __restrict__ runs, int run, int 
       }
     }
   }
-}
-
-// Non-finite check of a run's state: sets *flag to 1 if any coefficient is NaN/Inf.
-template <typename T>
-__global__ void nonfinite_kernel(const RunDesc* __restrict__ runs, int run, int* flag) {
-  using C = cx<T>;
-  const RunDesc& R = runs[run];
-  const C* c = reinterpret_cast<const C*>(R.c);
-  const size_t tot = (size_t)R.K * R.M * R.NN;
-  int bad = 0;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < tot; e += (size_t)gridDim.x * blockDim.x) {
-    const C v = c[e];
-    if (!isfinite((double)v.x) || !isfinite((double)v.y)) bad = 1;
-  }
-  if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(flag, 1);
 }
 
 }  // namespace mwf

@@ -146,14 +146,17 @@ inline size_t xpass_smem(int prec, size_t n) {
   cudaError_t launch_x_inverse_##SUF(int nt, const RunDesc* runs, const WorkItem* items, int n,      \
                                      size_t smem, int* err, cudaStream_t st);                        \
   cudaError_t launch_energy_##SUF(const RunDesc* runs, int run, double* partial, int nparts,         \
-                                  double* out, cudaStream_t st);                                     \
+                                  int* flag, unsigned* ticket, const int* err, HostOut* out,        \
+                                  cudaStream_t st);                                                  \
   cudaError_t launch_ref_to_dev_##SUF(const double* re, const double* im, void* out, int K, int M,   \
                                       int NN, cudaStream_t st);                                      \
+  cudaError_t launch_host_to_dev_##SUF(const double* re, const double* im, void* out, int K, int M,  \
+                                       int NN, cudaStream_t st);                                     \
   cudaError_t launch_dev_to_ref_##SUF(const void* in, double* re, double* im, int K, int M, int NN,  \
-                                      cudaStream_t st);                                              \
+                                      cudaStream_t st, const int* err = nullptr,                    \
+                                      HostOut* out = nullptr);                                       \
   cudaError_t launch_imposesym_##SUF(const RunDesc* runs, int run, int mode, int M, int NN,          \
                                      cudaStream_t st);                                               \
-  cudaError_t launch_nonfinite_##SUF(const RunDesc* runs, int run, int* flag, cudaStream_t st);    \
   cudaError_t launch_phys_z_##SUF(const RunDesc* runs, int run, int X, int KK, const FftPlanDev& planZ, \
                                   size_t smem, double* out, int* err, cudaStream_t st);              \
   cudaError_t launch_spectrum_##SUF(const RunDesc* runs, int run, int M, int NN,                     \
