@@ -235,8 +235,16 @@ template <bool INV, int R> __device__ __forceinline__ void fx_dft(longlong2 (&v)
     v[1] = cadd(e1, o1); v[5] = csub(e1, o1);
     v[2] = cadd(e2, o2); v[6] = csub(e2, o2);
     v[3] = cadd(e3, o3); v[7] = csub(e3, o3);
+  } else if constexpr (R == 6) {
+    // 6 = 2 x 3 by the prime-factor map: no twiddles
+    longlong2 a0 = v[0], a1 = v[2], a2 = v[4], b0 = v[3], b1 = v[5], b2 = v[1];
+    fx_dft3<INV>(a0, a1, a2);
+    fx_dft3<INV>(b0, b1, b2);
+    v[0] = cadd(a0, b0); v[3] = csub(a0, b0);
+    v[4] = cadd(a1, b1); v[1] = csub(a1, b1);
+    v[2] = cadd(a2, b2); v[5] = csub(a2, b2);
   } else {
-    static_assert(R == 9, "radices 2, 3, 4, 8, 9");
+    static_assert(R == 9, "radices 2, 3, 4, 6, 8, 9");
     // 3 x 3: x[3 a + b] -> X[k + 3 l], twiddles W9^{b k}
     fx_dft3<INV>(v[0], v[3], v[6]);
     fx_dft3<INV>(v[1], v[4], v[7]);
@@ -332,7 +340,7 @@ __device__ __forceinline__ void fx_fft(longlong2* buf, int base, int G, const Fx
     const bool unit = s == pl.nst - 1;
 #define MWF_FX(R_) case R_: if (unit) fx_stage<INV, R_, true>(buf, base, G, pl, s, t, aux); else fx_stage<INV, R_, false>(buf, base, G, pl, s, t, aux); break;
     switch (pl.radix[s]) {
-      MWF_FX(8) MWF_FX(4) MWF_FX(2) MWF_FX(3) MWF_FX(9)
+      MWF_FX(8) MWF_FX(6) MWF_FX(4) MWF_FX(2) MWF_FX(3) MWF_FX(9)
       default: break;
     }
 #undef MWF_FX

@@ -56,33 +56,50 @@ __device__ __forceinline__ FxNorm fx_norm_add(FxNorm a, FxNorm b) {
 // ---------------------------------------------------------------------------------------
 
 // Sum over the M slots of a row of |re| + |im| times |m|^p0 (S0) and |m|^p1 (S1), each as a float times
-// 2^E; nan: a NaN or an infinity in the row.  One warp; the high words are enough (truncated by
-// less than 2^-20, which the caller covers).
+// 2^E; nan: a NaN or an infinity in the row.  One warp, one pass, eight loads of a lane in flight; each
+// lane keeps its sums relative to its largest exponent so far.  The high words are enough (truncated
+// by less than 2^-20, which the caller covers); zeros and subnormals count as zeros.
 __device__ __forceinline__ void fx_row_moments(const double2* __restrict__ row, int M, int MM, int p0, int p1,
                                                float& S0, float& S1, int& E, int& nan) {
   const int lane = threadIdx.x & 31;
   int top = 0;
-  for (int ms = lane; ms < M; ms += 32) {
-    const double2 v = row[ms];
-    top = max(top, max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff));
-  }
-  top = __reduce_max_sync(0xffffffffu, top) >> 20;
-  nan = top >= 0x7ff;
   float a = 0.f, b = 0.f;
-  for (int ms = lane; ms < M; ms += 32) {
-    const double2 v = row[ms];
-    auto part = [&](double x) {
-      const int h = (__double2hiint(x) & 0x7fffffff) - (top - 127) * (1 << 20);   // exponent relative to the largest
-      return h < (1 << 20) ? 0.f : __int_as_float(h << 3);
+  for (int m0 = 0; m0 < M; m0 += 256) {
+    int hx[8], hy[8], t = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int ms = m0 + 32 * i + lane;
+      const double2 v = ms < M ? row[ms] : make_double2(0.0, 0.0);
+      hx[i] = __double2hiint(v.x) & 0x7fffffff;
+      hy[i] = __double2hiint(v.y) & 0x7fffffff;
+      t = max(t, max(hx[i], hy[i]));
+    }
+    t >>= 20;
+    if (t > top) {
+      const float k = fx_pow2(max(top - t, -127));
+      a *= k;
+      b *= k;
+      top = t;
+    }
+    auto part = [&](int h) {                          // relative to the largest exponent
+      const int q = h - (top - 127) * (1 << 20);
+      return q < (1 << 20) || h < (1 << 20) ? 0.f : __int_as_float(q << 3);
     };
-    const float t = part(v.x) + part(v.y);
-    const float m = (float)(ms < MM ? ms : M - ms);
-    a += t * (p0 == 0 ? 1.f : p0 == 1 ? m : p0 == 2 ? m * m : m * m * m);
-    b += t * (p1 == 0 ? 1.f : p1 == 1 ? m : m * m);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int ms = m0 + 32 * i + lane;
+      const float v = part(hx[i]) + part(hy[i]);
+      const float m = (float)(ms < MM ? ms : M - ms);
+      a += v * (p0 == 0 ? 1.f : p0 == 1 ? m : p0 == 2 ? m * m : m * m * m);
+      b += v * (p1 == 0 ? 1.f : p1 == 1 ? m : m * m);
+    }
   }
-  S0 = top ? fx_warp_sum(a) : 0.f;                   // (zeros and subnormals count as zeros)
-  S1 = top ? fx_warp_sum(b) : 0.f;
-  E = top - 1023;
+  const int all = __reduce_max_sync(0xffffffffu, top);
+  const float k = fx_pow2(max(top - all, -127));
+  S0 = fx_warp_sum(a * k);
+  S1 = fx_warp_sum(b * k);
+  E = all - 1023;
+  nan = all >= 0x7ff;
 }
 
 template <int NT>
@@ -109,48 +126,47 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDes
 
   // Column scales from bounds on the columns' L1 norms: u = i(-n1 psi + k1 m1 phi), w = i(m1 psi +
   // k1 n1 phi), v = (m1^2 + n1^2) phi and the same times m1 (m1 = alpha m, n1 = gamma n)
-  for (int l = warp; l < nb; l += NT / 32) {
-    const int n = n0 + l;
-    const double a1 = fabs(R.alpha), g1 = fabs(R.gamma * n), k1 = fabs(kbeta<double>(k));
-    const int d = deriv ? 1 : 0;
-    double L = 0.0;
-    int nan = 0;
-    const double2* col = c + (size_t)n * K * M;
-    if (comp != 1) {                                  // psi: u needs m^d, w m^(d+1)
-      float s0, s1;
-      int E, bad;
-      fx_row_moments(col + (size_t)k * M, M, MM, comp == 0 ? d : d + 1, 0, s0, s1, E, bad);
-      nan |= bad;
-      L += scalbn((comp == 0 ? g1 : a1) * (double)s0, E);
-      if (n == 0 && !deriv) {                         // the mean flow u_k = psi_k, and the base flow
-        const double2 v = col[(size_t)k * M];
-        L += fabs(v.x) + fabs(v.y) + (k == 1 ? 1.0 : 0.0);
+  __shared__ float mom[2][2][kFxMaxCols];             // [psi, phi][sum]
+  __shared__ int momE[2][kFxMaxCols], momN[2][kFxMaxCols];
+  {
+    const int dd = deriv ? 1 : 0;
+    for (int i = warp; i < 2 * nb; i += NT / 32) {
+      const int l = i >> 1, phi = i & 1;
+      float s0 = 0.f, s1 = 0.f;
+      int E = 0, bad = 0;
+      // psi: u needs m^d, w m^(d+1); phi: u m^(d+1), w m^d, v m^(d+2) and m^d
+      if (phi ? k >= 1 : comp != 1) {
+        const int p0 = phi ? (comp == 0 ? dd + 1 : comp == 2 ? dd : dd + 2) : (comp == 0 ? dd : dd + 1);
+        fx_row_moments(c + ((size_t)(n0 + l) * K + (phi ? k + K0 - 1 : k)) * M, M, MM, p0, dd, s0, s1, E, bad);
+      }
+      if (lane == 0) {
+        mom[phi][0][l] = s0;
+        mom[phi][1][l] = s1;
+        momE[phi][l] = E;
+        momN[phi][l] = bad;
       }
     }
-    if (k >= 1) {                                     // phi: u m^(d+1), w m^d, v m^(d+2) and m^d
-      float s0, s1;
-      int E, bad;
-      fx_row_moments(col + (size_t)(k + K0 - 1) * M, M, MM, comp == 0 ? d + 1 : comp == 2 ? d : d + 2, d, s0, s1, E, bad);
-      nan |= bad;
-      if (comp == 0) L += scalbn(k1 * a1 * (double)s0, E);
-      else if (comp == 2) L += scalbn(k1 * g1 * (double)s0, E);
-      else L += scalbn(a1 * a1 * (double)s0, E) + scalbn(g1 * g1 * (double)s1, E);
-      if (comp == 2 && n == 0 && !deriv) {            // the mean flow w_k = phi_k
-        const double2 v = col[(size_t)(k + K0 - 1) * M];
-        L += fabs(v.x) + fabs(v.y);
-      }
+  }
+  __syncthreads();
+  if (threadIdx.x < nb) {
+    const int l = threadIdx.x, n = n0 + l;
+    const double a1 = fabs(R.alpha), n1 = R.gamma * n, g1 = fabs(n1), kb = kbeta<double>(k), k1 = fabs(kb);
+    const double s0 = scalbn((double)mom[0][0][l], momE[0][l]);
+    const double t0 = scalbn((double)mom[1][0][l], momE[1][l]), t1 = scalbn((double)mom[1][1][l], momE[1][l]);
+    double L = comp == 0 ? g1 * s0 + k1 * a1 * t0 : comp == 2 ? a1 * s0 + k1 * g1 * t0 : a1 * a1 * t0 + g1 * g1 * t1;
+    if (n == 0 && !deriv && comp != 1) {              // the mean flows u_k = psi_k, w_k = phi_k, and the base flow
+      const double2 v = c[(size_t)(comp == 0 || k == 0 ? k : k + K0 - 1) * M];
+      L += fabs(v.x) + fabs(v.y) + (k == 1 ? 1.0 : 0.0);
     }
     if (deriv) L *= a1;
     L *= 1.0001;
     const int ex = (int)(fx_bits(L) >> 52) & 0x7ff;
-    const int e = nan || ex == 0x7ff ? kFxNan : (L == 0.0 ? kFxZero : 61 - (ex - 1022));
-    if (lane == 0) {
-      colE[l] = e;
-      R.fx_colE[(size_t)f * NN + n] = e;
-      const double n1 = R.gamma * n, kb = kbeta<double>(k), sg = deriv ? -1.0 : 1.0;
-      colN[0][l] = fx_factor(comp == 0 ? -sg * n1 : comp == 2 ? sg : 1.0);
-      colN[1][l] = fx_factor(comp == 0 ? sg * kb : comp == 2 ? sg * (kb * n1) : n1 * n1);
-    }
+    const int e = momN[0][l] || momN[1][l] || ex == 0x7ff ? kFxNan : (L == 0.0 ? kFxZero : 61 - (ex - 1022));
+    colE[l] = e;
+    R.fx_colE[(size_t)f * NN + n] = e;
+    const double sg = deriv ? -1.0 : 1.0;
+    colN[0][l] = fx_factor(comp == 0 ? -sg * n1 : comp == 2 ? sg : 1.0);
+    colN[1][l] = fx_factor(comp == 0 ? sg * kb : comp == 2 ? sg * (kb * n1) : n1 * n1);
   }
   __syncthreads();
 
@@ -367,7 +383,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) z_fx_kernel(const RunDesc* __res
     float* nZ = nS + 2 * KK * L;
     int* nE = reinterpret_cast<int*>(nZ + 2 * KK * L);
     int W = 1;
-    while (W < 32 && 2 * W < R.fx_nblk) W <<= 1;
+    while (W < 32 && 4 * W < R.fx_nblk) W <<= 1;     // four blocks of a lane in flight
     const int sub = lane / W, seg = 32 / W;
     for (int i0 = warp * seg; i0 < 2 * KK * L; i0 += NW * seg) {
       const int i = min(i0 + sub, 2 * KK * L - 1);

@@ -129,27 +129,16 @@ int4 fx_twiddle(const long double* v) {
   return make_int4(out[0], out[1], out[2], out[3]);
 }
 
-// Radices of the in-place transforms of length N.  Fixed point: 8s (of 16 two 4s), then 9s and 3s; a
-// butterfly of 12 or 16 would not leave 128 registers a thread.  FP32: the fewest stages of radices up
-// to 16, the balanced choice among them.
+// Radices of the in-place transforms of length N: the fewest stages, with radices up to 9 in fixed
+// point (a butterfly of 12 or 16 would not leave 128 registers a thread) and up to 16 in FP32.
 std::vector<int> inplace_radices(int N, bool fx) {
-  std::vector<int> rad;
-  if (fx) {
-    int rest = N;
-    auto take = [&](int r) { rad.push_back(r); rest /= r; };
-    while (rest % 8 == 0 && rest != 16) take(8);
-    while (rest % 4 == 0) take(4);
-    while (rest % 2 == 0) take(2);
-    while (rest % 9 == 0) take(9);
-    while (rest % 3 == 0) take(3);
-    return rad;
-  }
   static const int all[] = {16, 12, 9, 8, 6, 4, 3, 2};
   std::vector<int> cur, best;
   int best_sum = 0;
-  // depth-first over non-increasing radices: fewest stages, then the least padding (the last radix,
-  // below), then the smallest sum
-  auto padding = [](const std::vector<int>& r) {
+  // depth-first over non-increasing radices: fewest stages, then (FP32) the least padding (the last
+  // radix, below), then the smallest sum
+  auto padding = [&](const std::vector<int>& r) {
+    if (fx) return 0;
     for (int v : r)
       if (v % 2) return 0;
     return 48 / r[0];
@@ -173,7 +162,8 @@ std::vector<int> inplace_radices(int N, bool fx) {
         cur.pop_back();
       }
   };
-  go(go, N, 0);
+  go(go, N, fx ? 2 : 0);
+  if (fx) return best;
   // last: an odd radix, which needs no padding (mwf_zwarp.cuh), else the largest
   size_t last = 0;
   for (size_t k = 0; k < best.size(); ++k)
@@ -480,14 +470,27 @@ bool plan_run(RunHost& r, const char*& why) {
     while (r.fx_xi_nb > 1 && (fx_xi_smem(d.MM, r.fx_xi_nb) > (r.fx_xi_nb == 2 ? whole : half) ||
                               (r.fx_xi_nb > 2 && items(r.fx_xi_nb, d.K0) < slots))) r.fx_xi_nb /= 2;
     r.fx_xi_nt = fx_xi_smem(d.MM, r.fx_xi_nb) <= half ? 256 : 512;
-    // enough lines that a warp's butterflies fill its lanes, twice as many where that leaves two
-    // waves of items
-    r.fx_z_nt = fx_z_smem(d.K0, d.NN, 1) <= zb_smem_budget(2) ? 256 : 512;
-    const size_t zbud = zb_smem_budget(r.fx_z_nt == 256 ? 2 : 1);
+    // z pass: lines per item and block size (256 threads, two CTAs per SM, or 512) by the rounds that
+    // a CTA's warps make over its lines, transforms and points, times the waves of CTAs; enough
+    // lines come together that a warp's butterflies fill its lanes, and two such groups at most
     const int g = std::max(1, 256 / d.NN);
-    int L = std::min(r.X / (2 * g) * 3 >= 2 * slots ? 2 * g : g, r.X);
-    while (L > 1 && fx_z_smem(d.K0, d.NN, L) > zbud) --L;
-    r.fx_lines = L;
+    const int ntr = (3 * r.KK + 1) / 2, npair = (r.KK + 1) / 2;
+    long best = -1;
+    for (int nt : {256, 512}) {
+      const size_t zbud = zb_smem_budget(nt == 256 ? 2 : 1);
+      for (int L = 1; L <= 2 * g && L <= r.X; ++L) {
+        if (fx_z_smem(d.K0, d.NN, L) > zbud) continue;
+        const long warps = nt / 32, groups = (L + g - 1) / g, ctas = (long)((r.X + L - 1) / L) * 3;
+        auto rounds = [&](long tasks) { return (tasks + warps - 1) / warps; };
+        const long per_cta = 4 * rounds(ntr * groups) + 3 * rounds(npair * groups) + 3 * ((L * d.NN + nt - 1) / nt) + 3;
+        const long cost = per_cta * ((ctas + 152 * 512 / nt - 1) / (152 * 512 / nt));
+        if (best < 0 || cost < best || (cost == best && nt == r.fx_z_nt)) {
+          best = cost;
+          r.fx_z_nt = nt;
+          r.fx_lines = L;
+        }
+      }
+    }
   }
   r.n_diag_xf = ((d.NN + r.xf_nb - 1) / r.xf_nb) * r.KK;
   r.n_diag_z = ((r.X + r.z_lx - 1) / r.z_lx) * 3;
