@@ -595,6 +595,7 @@ struct mwf_handle {
   int persist_grid = 0;
   bool persist_mode = false;         // step with the persistent kernel (mwf_set_persistent)
   bool any_sym = false;
+  bool euler_pending = true;          // a run's Euler-start flag may be set: the next step clears it
   cudaGraphExec_t graph1 = nullptr;   // one step
   cudaGraphExec_t graphG = nullptr;   // kGraphSteps steps
   static constexpr int kGraphSteps = 16;
@@ -603,7 +604,10 @@ struct mwf_handle {
 
 namespace {
 
-int enqueue_step(mwf_handle* h) {
+// One step on the handle's stream; clear_euler: with the reset of the runs' Euler-start flags, which
+// only the first step after a flag was set needs (the graphs leave it out: a memset node cost a
+// small run's step about 2 us).
+int enqueue_step(mwf_handle* h, bool clear_euler) {
   cudaStream_t st = h->stream;
   if (h->any_sym) {
     for (size_t i = 0; i < h->runs.size(); ++i) {
@@ -632,8 +636,10 @@ int enqueue_step(mwf_handle* h) {
     if (e != cudaSuccess) return fail(MWF_ERR_CUDA, "pass %d launch: %s", L.kind, cudaGetErrorString(e));
   }
   // the Euler start applies to one step only (velocity.f90:24-27)
-  cudaError_t e = cudaMemsetAsync(h->arena + h->off_nst_all, 0, sizeof(int) * h->runs.size(), st);
-  if (e != cudaSuccess) return fail(MWF_ERR_CUDA, "nst reset: %s", cudaGetErrorString(e));
+  if (clear_euler) {
+    const cudaError_t e = cudaMemsetAsync(h->arena + h->off_nst_all, 0, sizeof(int) * h->runs.size(), st);
+    if (e != cudaSuccess) return fail(MWF_ERR_CUDA, "nst reset: %s", cudaGetErrorString(e));
+  }
   return MWF_OK;
 }
 
@@ -641,7 +647,7 @@ int build_graph(mwf_handle* h, int steps, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   int rc = MWF_OK;
-  for (int s = 0; s < steps && rc == MWF_OK; ++s) rc = enqueue_step(h);
+  for (int s = 0; s < steps && rc == MWF_OK; ++s) rc = enqueue_step(h, false);
   cudaError_t e = cudaStreamEndCapture(h->stream, &g);
   if (rc != MWF_OK) { if (g) cudaGraphDestroy(g); return rc; }
   if (e != cudaSuccess) return fail(MWF_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
@@ -1366,6 +1372,7 @@ int mwf_set_history(mwf_handle* h, int run, const double* re, const double* im, 
   rc = state_in(h, r, r.off_onl, re, im);
   if (rc) return rc;
   const int v = euler_next ? 1 : 0;
+  if (v) h->euler_pending = true;
   CK(cudaMemcpyAsync(h->arena + r.off_nst, &v, sizeof(int), cudaMemcpyHostToDevice, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   return MWF_OK;
@@ -1389,6 +1396,12 @@ int mwf_step_async(mwf_handle* h, int nsteps) {
   if (nsteps < 0) return fail(MWF_ERR_ARG, "nsteps < 0");
   if (cudaSetDevice(h->device) != cudaSuccess) return fail(MWF_ERR_CUDA, "cudaSetDevice failed");
   int s = nsteps;
+  if (s > 0 && h->euler_pending) {
+    const int rc = enqueue_step(h, true);
+    if (rc) return rc;
+    h->euler_pending = false;
+    --s;
+  }
   while (s >= mwf_handle::kGraphSteps) {
     CK(cudaGraphLaunch(h->graphG, h->stream));
     s -= mwf_handle::kGraphSteps;
@@ -1413,6 +1426,7 @@ int mwf_reset_history(mwf_handle* h, int run) {
   int rc = check_run(h, run);
   if (rc) return rc;
   const int one = 1;
+  h->euler_pending = true;
   CK(cudaMemcpyAsync(h->arena + h->runs[run].off_nst, &one, sizeof(int), cudaMemcpyHostToDevice, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   return MWF_OK;
@@ -1611,6 +1625,7 @@ int mwf_history(mwf_handle* h, int run, double y, int n_probes, double* H) {
 
 static int set_nst(mwf_handle* h, const RunHost& r) {
   const int one = 1;
+  h->euler_pending = true;
   CK(cudaMemcpyAsync(h->arena + r.off_nst, &one, sizeof(int), cudaMemcpyHostToDevice, h->stream));
   return MWF_OK;
 }
@@ -1721,6 +1736,7 @@ int mwf_profile_passes(mwf_handle* h, int nreps, double* ms_per_pass) {
     }
     CK(cudaMemsetAsync(h->arena + h->off_nst_all, 0, sizeof(int) * h->runs.size(), h->stream));
   }
+  h->euler_pending = false;
   if (rc == MWF_OK) {
     CK(cudaStreamSynchronize(h->stream));
     double acc[3] = {0, 0, 0};
