@@ -205,8 +205,8 @@ cudaError_t MWF_FN(launch_spec_x_forward)(const RunDesc* runs, int run, int X, i
 
 cudaError_t MWF_FN(launch_spectrum)(const RunDesc* runs, int run, int M, int NN, unsigned long long* mx,
                                     cudaStream_t st) {
-  const dim3 grid((M + 255) / 256, (NN + kSpecRows - 1) / kSpecRows);
-  spectrum_kernel<MWF_T><<<grid, 256, 0, st>>>(runs, run, mx);
+  const dim3 grid((M + kSpecThreads - 1) / kSpecThreads, (NN + kSpecRows - 1) / kSpecRows);
+  spectrum_kernel<MWF_T><<<grid, kSpecThreads, 0, st>>>(runs, run, mx);
   return cudaGetLastError();
 }
 

@@ -8,6 +8,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <map>
 #include <vector>
 #include <algorithm>
 
@@ -89,30 +90,63 @@ bool make_plan(int N, FftPlanDev& pl, int maxr) {
   return ns == N;
 }
 
+// cos and sin of 2 pi t / N in long double, the argument folded into [0, pi/4]: with 4t = q N + r the
+// angle is (q + r/N) quarter turns, and r > N/2 swaps the two.  first(r), r <= N/2, gives them for
+// r/N of a quarter turn.
+template <typename F>
+void unit_root(int N, int t, F&& first, long double& c, long double& s) {
+  const int q = (int)(4LL * t / N), r = (int)(4LL * t - (long long)q * N);
+  long double a, b;                            // cos, sin of r/N quarter turns
+  if (2 * r <= N) first(r, a, b);
+  else first(N - r, b, a);
+  switch (q & 3) {
+    case 0: c = a; s = b; break;
+    case 1: c = -b; s = a; break;
+    case 2: c = -a; s = -b; break;
+    default: c = b; s = -a; break;
+  }
+}
+void first_octant(int N, int r, long double& c, long double& s) {
+  const long double h = 0.707106781186547524400844362104849039L, quarter = 1.570796326794896619231321691639751442L;
+  if (r == 0) { c = 1.0L; s = 0.0L; return; }
+  if (2 * r == N) { c = s = h; return; }
+  const long double a = quarter * (long double)r / (long double)N;
+  c = cosl(a);
+  s = sinl(a);
+}
+
 // tw[t] = exp(-2 pi i t / N) for t in [t0, t0 + cnt), evaluated in long double and rounded
 // once; out receives 2*cnt values (re, im interleaved).
 template <typename T>
 void twiddles_into(int N, int t0, int cnt, T* out) {
-  const long double two_pi = 6.283185307179586476925286766559005768L;
   for (int t = t0; t < t0 + cnt; ++t) {
-    // reduce by symmetry so the argument stays in [0, pi/4]
     long double c, s;
-    const int q8 = 8 * t;               // angle = 2 pi t/N = (pi/4) * (8t/N)
-    if (q8 % N == 0) {
-      const int oct = q8 / N;           // exact multiples of pi/4
-      const long double h = 0.707106781186547524400844362104849039L;
-      static const int cs[8][2] = {{2, 0}, {1, 1}, {0, 2}, {-1, 1}, {-2, 0}, {-1, -1}, {0, -2}, {1, -1}};
-      auto val = [&](int v) -> long double { return v == 2 ? 1.0L : v == -2 ? -1.0L : v * h; };
-      c = val(cs[oct][0]);
-      s = val(cs[oct][1]);
-    } else {
-      const long double a = two_pi * (long double)t / (long double)N;
-      c = cosl(a);
-      s = sinl(a);
-    }
+    unit_root(N, t, [&](int r, long double& a, long double& b) { first_octant(N, r, a, b); }, c, s);
     out[2 * (size_t)(t - t0)] = (T)c;
     out[2 * (size_t)(t - t0) + 1] = (T)(-s);
   }
+}
+
+// The whole table in long double; each first-octant value is evaluated once (N/8 of them where
+// 4 divides N: long double functions take 0.7 us on the Grace host).
+std::vector<long double> twiddles(int N) {
+  std::vector<long double> out(2 * (size_t)N), oct(2 * ((size_t)N / 2 + 1));
+  std::vector<char> have((size_t)N / 2 + 1, 0);
+  auto first = [&](int r, long double& a, long double& b) {
+    if (!have[r]) {
+      first_octant(N, r, oct[2 * (size_t)r], oct[2 * (size_t)r + 1]);
+      have[r] = 1;
+    }
+    a = oct[2 * (size_t)r];
+    b = oct[2 * (size_t)r + 1];
+  };
+  for (int t = 0; t < N; ++t) {
+    long double c, s;
+    unit_root(N, t, first, c, s);
+    out[2 * (size_t)t] = c;
+    out[2 * (size_t)t + 1] = -s;
+  }
+  return out;
 }
 
 // A twiddle (re, im) times 2^62 as two 32-bit limbs per part (FxConst: high, signed low), the low
@@ -218,13 +252,6 @@ bool make_fx_plan(int N, const std::vector<W>& w, bool fx, FxPlan& pl, std::vect
     rev[p] = (unsigned short)q;
   }
   return span == 1;
-}
-
-template <typename T>
-std::vector<T> twiddles(int N) {
-  std::vector<T> out(2 * (size_t)N);
-  twiddles_into<T>(N, 0, N, out.data());
-  return out;
 }
 
 // var_precompute tables (variables.f90:516-531) and var_LHSRHS (variables.f90:565-597) in
@@ -1110,6 +1137,12 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
   // for the handle's non-blocking stream: finish the clear first, or it can land after them
   // and zero the tables of the first runs.
   ck(cudaStreamSynchronize(h->stream), "arena clear");
+  std::map<int, std::vector<long double>> root_tables;   // one per length, for all runs
+  auto roots = [&](int N) -> const std::vector<long double>& {
+    std::vector<long double>& v = root_tables[N];
+    if (v.empty()) v = twiddles(N);
+    return v;
+  };
   std::vector<RunDesc> rds(n_runs);
   for (int i = 0; i < n_runs && rc == MWF_OK; ++i) {
     RunHost& r = h->runs[i];
@@ -1163,11 +1196,12 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
       ck(cudaMemcpy(h->arena + r.off_rhs, b.data(), b.size() * 4, cudaMemcpyHostToDevice), "table upload");
     }
     auto up = [&](size_t off, int N) {
+      const std::vector<long double>& v = roots(N);
       if (r.d.precision == MWF_FP64) {
-        std::vector<double> t = twiddles<double>(N);
+        const std::vector<double> t(v.begin(), v.end());
         ck(cudaMemcpy(h->arena + off, t.data(), t.size() * 8, cudaMemcpyHostToDevice), "twiddle upload");
       } else {
-        std::vector<float> t = twiddles<float>(N);
+        const std::vector<float> t(v.begin(), v.end());
         ck(cudaMemcpy(h->arena + off, t.data(), t.size() * 4, cudaMemcpyHostToDevice), "twiddle upload");
       }
     };
@@ -1176,9 +1210,9 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
     if (!r.fx) up(r.off_twZ, r.Z);
     // in-place FP32 transforms of length N, their stage twiddles at off
     auto inplace = [&](int N, FxPlan& pl, size_t off, std::vector<unsigned short>& rev) {
-      const std::vector<float> v = twiddles<float>(3 * N);
+      const std::vector<long double>& v = roots(3 * N);
       std::vector<float2> w(3 * (size_t)N), t;
-      for (size_t j = 0; j < w.size(); ++j) w[j] = make_float2(v[2 * j], v[2 * j + 1]);
+      for (size_t j = 0; j < w.size(); ++j) w[j] = make_float2((float)v[2 * j], (float)v[2 * j + 1]);
       if (!make_fx_plan(N, w, false, pl, t, rev) || t.size() > (size_t)N) {
         rc = fail(MWF_ERR_SIZE, "run %d: no in-place FFT plan", i);
         return;
@@ -1206,7 +1240,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
       std::vector<unsigned short> unused;
       // the double and the fixed-point tables of X and Z from one evaluation
       auto table = [&](int N, size_t off_d, size_t off_fx, std::vector<int4>& w) {
-        const std::vector<long double> v = twiddles<long double>(N);
+        const std::vector<long double>& v = roots(N);
         const std::vector<double> t(v.begin(), v.end());
         w.resize(N);
         for (int j = 0; j < N; ++j) w[j] = fx_twiddle(&v[2 * (size_t)j]);
@@ -1819,7 +1853,8 @@ int transform_setup(const mwf_run_desc* desc, const char* who, TransformCall& tc
   D.twX = tc.mem + off_twX;
   D.twZ = tc.mem + off_twZ;
   D.active = 1;
-  const std::vector<double> twx = twiddles<double>(r.X), twz = twiddles<double>(r.Z);
+  const std::vector<long double> lx = twiddles(r.X), lz = twiddles(r.Z);
+  const std::vector<double> twx(lx.begin(), lx.end()), twz(lz.begin(), lz.end());
   CK(cudaMemcpy(tc.d, &D, sizeof D, cudaMemcpyHostToDevice));
   CK(cudaMemset(tc.err, 0, sizeof(int)));
   CK(cudaMemcpy(tc.mem + off_twX, twx.data(), twx.size() * 8, cudaMemcpyHostToDevice));

@@ -164,18 +164,21 @@ __global__ void __launch_bounds__(NT) spec_x_forward_kernel(const RunDesc* __res
 // sqrt(re^2 + im^2) over the KK spectral coefficients of u, v, w (no base flow); folded
 // into mx[0..MM-1] by |m| and mx[MM..MM+NN-1] by n.  The moduli are non-negative, so their
 // bit patterns order like the values and one 64-bit atomicMax keeps each maximum.
-// Grid: (ceil(M / 256), ceil(NN / kSpecRows)); one thread per column slot m.
+// The largest square is kept and rooted once: the rounded root is monotonic, so the maximum of the
+// roots is the root of the maximum.  Grid: (ceil(M / 128), ceil(NN / kSpecRows)); one thread per column
+// slot m.  (Sixteen rows of 256 slots with a root per coefficient left a 96 x 191 state six CTAs and took
+// 240 us.)
 // ---------------------------------------------------------------------------------------
-constexpr int kSpecRows = 16;
+constexpr int kSpecRows = 2, kSpecThreads = 128;
 
 template <typename T>
-__global__ void __launch_bounds__(256) spectrum_kernel(const RunDesc* __restrict__ runs, int run,
+__global__ void __launch_bounds__(kSpecThreads) spectrum_kernel(const RunDesc* __restrict__ runs, int run,
                                                         unsigned long long* mx) {
   using C = cx<T>;
   const RunDesc& R = runs[run];
   const C* __restrict__ c = reinterpret_cast<const C*>(R.c);
   const int M = R.M, MM = R.MM, NN = R.NN, KK = R.KK;
-  const int ms = blockIdx.x * 256 + threadIdx.x;
+  const int ms = blockIdx.x * kSpecThreads + threadIdx.x;
   const int n0 = blockIdx.y * kSpecRows;
   const bool live = ms < M;
   const int m = live ? signed_m(ms, MM, M) : 0;
@@ -187,9 +190,10 @@ __global__ void __launch_bounds__(256) spectrum_kernel(const RunDesc* __restrict
       for (int fs = 0; fs < KK; ++fs) {
         const C v = mpt_to_field<T>(R, c, fs, m, n, false);
         const double re = (double)v.x, im = (double)v.y;
-        d = fmax(d, sqrt(__dadd_rn(__dmul_rn(re, re), __dmul_rn(im, im))));
+        d = fmax(d, __dadd_rn(__dmul_rn(re, re), __dmul_rn(im, im)));
       }
     }
+    d = sqrt(d);
     mcol = fmax(mcol, d);
     for (int o = 16; o > 0; o >>= 1) d = fmax(d, __shfl_xor_sync(0xffffffffu, d, o));
     if ((threadIdx.x & 31) == 0) atomicMax(&mx[MM + n], (unsigned long long)__double_as_longlong(d));
