@@ -26,8 +26,9 @@ cudaError_t launch_x_forward_fx(int nt, const RunDesc* runs, const WorkItem* ite
 
 cudaError_t launch_z_fx(int K0, int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st) {
   if (K0 == 4)
-    return nt == 256 ? fx_launch(z_fx_kernel<4, 256>, nt, runs, items, n, smem, st)
-                     : fx_launch(z_fx_kernel<4, 512>, nt, runs, items, n, smem, st);
+    return nt == 256   ? fx_launch(z_fx_kernel<4, 256>, nt, runs, items, n, smem, st)
+           : nt == 512 ? fx_launch(z_fx_kernel<4, 512>, nt, runs, items, n, smem, st)
+                       : fx_launch(z_fx_kernel<4, 544>, nt, runs, items, n, smem, st);
   return nt == 256 ? fx_launch(z_fx_kernel<6, 256>, nt, runs, items, n, smem, st)
                    : fx_launch(z_fx_kernel<6, 512>, nt, runs, items, n, smem, st);
 }

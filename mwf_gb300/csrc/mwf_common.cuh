@@ -158,6 +158,8 @@ struct RunDesc {
   // element of the digit-reversed x lines; the scales of what the passes store
   int fx;
   int fx_nb, fx_xi_nb, fx_nblk, fx_lines;
+  int fx_group;                 // x lines of a warp's task in the z pass
+  int fx_tab;                   // tables of NN entries that the z pass copies to shared memory: 0 ... 2
   const int4 *fx_twX, *fx_twZ, *fx_twM, *fx_twQ, *fx_gn, *fx_mp;
   const double2* fx_ms;
   const unsigned short* fx_rev;

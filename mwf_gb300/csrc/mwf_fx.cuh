@@ -38,7 +38,18 @@ constexpr i64 kFxQuarterPi = 3622009729038561421ll;  // pi/4
 __host__ __device__ constexpr i64 fx_c9(int i) { return i == 0 ? 3532756447825785444ll : i == 1 ? 800810873071977681ll : -4333567320897763126ll; }
 __host__ __device__ constexpr i64 fx_s9(int i) { return i == 0 ? 2964334632409774423ll : i == 1 ? 4541624145405292212ll : 1577289512995517789ll; }
 
-__host__ __device__ __forceinline__ i64 fx_madw(int a, int b, i64 c) { return (i64)a * b + c; }
+// a b + c.  (Written as one instruction: from (i64)a * b + c the compiler made a product and an
+// addition where it saw sums of several, and a coupling section of 54 such triples took 4180 cycles
+// instead of 2570.)
+__host__ __device__ __forceinline__ i64 fx_madw(int a, int b, i64 c) {
+#ifdef __CUDA_ARCH__
+  i64 r;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+  return r;
+#else
+  return (i64)a * b + c;
+#endif
+}
 
 // x = h 2^32 + l with l signed.
 __host__ __device__ __forceinline__ FxConst fx_split(i64 x) {

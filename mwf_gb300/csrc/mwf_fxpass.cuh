@@ -265,6 +265,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDes
   const float wgt = (ce >= kFxZero || er <= kFxNan) ? 0.f : fx_pow2(max(er - ce, -127));
   longlong2* __restrict__ T = reinterpret_cast<longlong2*>(R.T) + (size_t)f * X * NN;
   float* __restrict__ P = R.fx_rowP + (size_t)f * X * nblk;
+#pragma unroll 4
   for (int e0 = 0; e0 < (X << lw); e0 += NT) {
     const int sp = (e0 + threadIdx.x) >> lw;          // s MM + position
     const bool on = sp < X;
@@ -288,6 +289,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDes
 // z pass
 // ---------------------------------------------------------------------------------------
 
+constexpr int kFxFlight = 5;   // 128 blocks and the column n = 0 are 129 entries for 32 lanes
+
 // Sums of moduli of row (f, x), and of the moduli times the z wavenumber index (an upper bound: the
 // block's largest), over the W lanes (a power of two) of a warp's segment; lane = place in it.
 __device__ __forceinline__ void fx_row_norm(const RunDesc& R, int f, int x, int W, int lane, float& S, float& Z, int& E, int& bad) {
@@ -297,17 +300,17 @@ __device__ __forceinline__ void fx_row_norm(const RunDesc& R, int f, int x, int 
   int ref = -(1 << 29);
   bad = 0;
   float s = 0.f, z = 0.f;
-  for (int b0 = 0; b0 < nblk; b0 += 4 * W) {          // four blocks of a lane in flight
-    float p[4];
-    int e[4], top = -(1 << 29);
+  for (int b0 = 0; b0 < nblk; b0 += kFxFlight * W) {  // kFxFlight blocks of a lane in flight
+    float p[kFxFlight];
+    int e[kFxFlight], top = -(1 << 29);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < kFxFlight; ++i) {
       const int b = b0 + i * W + lane;
       p[i] = b < nblk ? P[b] : 0.f;
       e[i] = b < nblk ? EB[b] : kFxZero;
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < kFxFlight; ++i) {
       bad |= e[i] <= kFxNan;
       if (p[i] > 0.f) top = max(top, -e[i]);
     }
@@ -322,7 +325,7 @@ __device__ __forceinline__ void fx_row_norm(const RunDesc& R, int f, int x, int 
       ref = top;
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < kFxFlight; ++i)
       if (p[i] > 0.f) {
         const float v = p[i] * fx_pow2(max(-e[i] - ref, -127));
         s += v;
@@ -348,7 +351,7 @@ template <int K0> __host__ __device__ constexpr int fx_first(int comp) { return 
 template <int K0> __host__ __device__ constexpr int fx_count(int comp) { return comp == 1 ? K0 - 1 : K0; }
 
 template <int K0, int NT>
-__global__ void __launch_bounds__(NT, 512 / NT) z_fx_kernel(const RunDesc* __restrict__ runs, const WorkItem* __restrict__ items) {
+__global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) z_fx_kernel(const RunDesc* __restrict__ runs, const WorkItem* __restrict__ items) {
   constexpr int KK = 3 * K0 - 1, NPAIR = (KK + 1) / 2, NTR = NPAIR + KK;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const WorkItem wi = items[blockIdx.x];
@@ -367,12 +370,20 @@ __global__ void __launch_bounds__(NT, 512 / NT) z_fx_kernel(const RunDesc* __res
   int* eo = ge + kFxGroups * L;                                  // [3 L] exponents of the products
   int* sh = eo + 3 * L;                                          // [NPAIR L] forward line shifts
   int* bad = sh + NPAIR * L;                                     // [L] NaN lines
+  // Where they fit (RunDesc::fx_tab): the subset's twiddles e^{-2 pi i ns/Z}, then gamma n, which the fill
+  // would wait for in every slot
+  int4* const tab = reinterpret_cast<int4*>(smem_raw + (((unsigned char*)(bad + L) - smem_raw + 15) & ~15));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int NW = NT / 32;
   const longlong2* __restrict__ T = reinterpret_cast<const longlong2*>(R.T);
   const size_t fstride = (size_t)X * Q;
 
-  for (int i = threadIdx.x; i < Q; i += NT) tw[i] = R.fx_twQ[i];
+  const int ntab = R.fx_tab;
+  for (int i = threadIdx.x; i < Q; i += NT) {
+    tw[i] = R.fx_twQ[i];
+    if (ntab > 0) tab[i] = R.fx_twZ[i * s];
+    if (ntab > 1) tab[Q + i] = R.fx_gn[i];
+  }
   for (int i = threadIdx.x; i < 2 * NTR * L; i += NT) mx[i] = 0;
   for (int i = threadIdx.x; i < L; i += NT) bad[i] = 0;
   __syncthreads();
@@ -383,7 +394,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) z_fx_kernel(const RunDesc* __res
     float* nZ = nS + 2 * KK * L;
     int* nE = reinterpret_cast<int*>(nZ + 2 * KK * L);
     int W = 1;
-    while (W < 32 && 4 * W < R.fx_nblk) W <<= 1;     // four blocks of a lane in flight
+    while (W < 32 && kFxFlight * W < R.fx_nblk) W <<= 1;
     const int sub = lane / W, seg = 32 / W;
     for (int i0 = warp * seg; i0 < 2 * KK * L; i0 += NW * seg) {
       const int i = min(i0 + sub, 2 * KK * L - 1);
@@ -416,9 +427,10 @@ __global__ void __launch_bounds__(NT, 512 / NT) z_fx_kernel(const RunDesc* __res
   // H[Q-n] = w' (U' + eps V'), w' = e^{2 pi i (Q-n)s/Z}, where U = a + i b at n, V = conj a + i conj b
   // at Q-n, and U', V' the same with n and Q-n exchanged.  Slot n < (Q+1)/2 of a line is the pair
   // (n, Q-n); slot 0 is n = 0 with, for even Q, n = Q/2 (its own partner).
-  const int4* __restrict__ om = R.fx_twZ;             // e^{-2 pi i t/Z}
+  const int4* om = ntab > 0 ? tab : R.fx_twZ;         // e^{-2 pi i ns/Z} at n os
+  const int os = ntab > 0 ? 1 : s;
   const int* __restrict__ colE = R.fx_colE;
-  const int4* __restrict__ gn = R.fx_gn;              // gamma n as (h, l, exponent)
+  const int4* gn = ntab > 1 ? tab + Q : R.fx_gn;      // gamma n as (h, l, exponent)
   constexpr FxConst s3 = fx_const(kFxSqrt34);
   auto times_eps = [&](longlong2 a) {                 // eps a for this subset (s = 1, 2)
     const i64 rx = fx_mulc(a.x, s3), ry = fx_mulc(a.y, s3);
@@ -427,7 +439,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) z_fx_kernel(const RunDesc* __res
     r.y = s == 1 ? -(a.y >> 1) - rx : -(a.y >> 1) + rx;
     return r;
   };
-  const int G = max(1, min(L, 256 / Q));
+  const int G = min(L, R.fx_group);
   const int groups = (L + G - 1) / G;
   const int slots = (Q + 1) / 2;
   const bool even = (Q & 1) == 0;
@@ -503,8 +515,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) z_fx_kernel(const RunDesc* __res
         Hn = cadd(U, V);
         Hq = cadd(U2, V2);
       } else {
-        Hn = fx_cmul<true>(cadd(U, times_eps(V)), om[n * s]);
-        Hq = fx_cmul<true>(cadd(U2, times_eps(V2)), om[nq * s]);
+        Hn = fx_cmul<true>(cadd(U, times_eps(V)), om[n * os]);
+        Hq = fx_cmul<true>(cadd(U2, times_eps(V2)), om[nq * os]);
       }
       if (sl || even) buf[fx_at(base + n)] = Hn;
       if (sl) buf[fx_at(base + nq)] = Hq;
@@ -644,7 +656,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) z_fx_kernel(const RunDesc* __res
       A.x = g.x + m.x; A.y = g.y - m.y;
       B.x = g.y + m.y; B.y = m.x - g.x;
       if (s != 0) {
-        const int4 w = om[n * s];
+        const int4 w = om[n * os];
         A = fx_cmul<false>(A, w);
         B = fx_cmul<false>(B, w);
       }

@@ -323,7 +323,7 @@ struct RunHost {
   // FP64 in fixed point (mwf_fxpass.cuh): columns and block sizes of the x passes, lines and block
   // size of the z pass
   bool fx = false;
-  int fx_nb = 0, fx_xi_nb = 0, fx_lines = 0, fx_nblk = 0;
+  int fx_nb = 0, fx_xi_nb = 0, fx_lines = 0, fx_nblk = 0, fx_tab = 0, fx_group = 0;
   int fx_xf_nt = 0, fx_z_nt = 0, fx_xi_nt = 0;
   size_t off_fx = 0;
   struct FxOff { size_t twX, twZ, twM, twQ, gn, mp, ms, rev, colE, blkE, rowE, minE, rowP, end; };
@@ -497,27 +497,39 @@ bool plan_run(RunHost& r, const char*& why) {
     while (r.fx_xi_nb > 1 && (fx_xi_smem(d.MM, r.fx_xi_nb) > (r.fx_xi_nb == 2 ? whole : half) ||
                               (r.fx_xi_nb > 2 && items(r.fx_xi_nb, d.K0) < slots))) r.fx_xi_nb /= 2;
     r.fx_xi_nt = fx_xi_smem(d.MM, r.fx_xi_nb) <= half ? 256 : 512;
-    // z pass: lines per item and block size (256 threads, two CTAs per SM, or 512) by the rounds that
-    // a CTA's warps make over its lines, transforms and points, times the waves of CTAs; enough
-    // lines come together that a warp's butterflies fill its lanes, and two such groups at most
-    const int g = std::max(1, 256 / d.NN);
-    const int ntr = (3 * r.KK + 1) / 2, npair = (r.KK + 1) / 2;
-    long best = -1;
-    for (int nt : {256, 512}) {
-      const size_t zbud = zb_smem_budget(nt == 256 ? 2 : 1);
-      for (int L = 1; L <= 2 * g && L <= r.X; ++L) {
-        if (fx_z_smem(d.K0, d.NN, L) > zbud) continue;
-        const long warps = nt / 32, groups = (L + g - 1) / g, ctas = (long)((r.X + L - 1) / L) * 3;
-        auto rounds = [&](long tasks) { return (tasks + warps - 1) / warps; };
-        const long per_cta = 4 * rounds(ntr * groups) + 3 * rounds(npair * groups) + 3 * ((L * d.NN + nt - 1) / nt) + 3;
-        const long cost = per_cta * ((ctas + 152 * 512 / nt - 1) / (152 * 512 / nt));
-        if (best < 0 || cost < best || (cost == best && nt == r.fx_z_nt)) {
-          best = cost;
-          r.fx_z_nt = nt;
-          r.fx_lines = L;
+    // z pass: block size (256 threads, two CTAs per SM; 512; for M4 also 544, a warp for each of its 17
+    // lines), lines per item and lines of a warp's task, by an estimate of a CTA's time -- the rounds
+    // that its warps make over fill, transforms and points, in thousands of cycles as measured on
+    // NN = 48 and 512 -- times the waves of CTAs
+    const int ntr = (3 * r.KK + 1) / 2, npair = (r.KK + 1) / 2, zslots = (d.NN + 1) / 2;
+    const std::vector<int> rad = inplace_radices(d.NN, true);
+    const int g0 = std::max(1, 256 / d.NN);
+    auto up = [](long a, long b) { return (a + b - 1) / b; };
+    double best = -1.0;
+    for (int nt : {256, 512, 544}) {
+      if (nt == 544 && d.K0 != 4) continue;
+      const long warps = nt / 32, per_sm = nt == 256 ? 2 : 1;
+      for (int L = 1; L <= 2 * g0 + 1 && L <= r.X; ++L) {
+        if (fx_z_smem(d.K0, d.NN, L) > zb_smem_budget((int)per_sm)) continue;
+        for (int G = 1; G <= std::min(L, g0 + 1); ++G) {
+          const long groups = up(L, G), fill = up((long)G * zslots, 32);
+          double fft = 0.0;                     // a butterfly of radix 8 as the unit
+          for (int q : rad) fft += up((long)G * d.NN / q, 32) * (q / 8.0 + 0.2);
+          const double cta = up(ntr * groups, warps) * (2.0 * fill + 2.2 * fft) +
+                             up(npair * groups, warps) * (1.0 * fill + 2.0 * fft + 2.0) +
+                             up((long)L * d.NN, nt) * (d.K0 == 4 ? 10.0 : 30.0) + 8.0;
+          const double cost = cta * up(up(r.X, L) * 3, 152 * per_sm);
+          if (best < 0.0 || cost < best) {
+            best = cost;
+            r.fx_z_nt = nt;
+            r.fx_lines = L;
+            r.fx_group = G;
+          }
         }
       }
     }
+    r.fx_tab = 2;
+    while (r.fx_tab > 0 && fx_z_smem(d.K0, d.NN, r.fx_lines, r.fx_tab) > zb_smem_budget(r.fx_z_nt == 256 ? 2 : 1)) --r.fx_tab;
   }
   r.n_diag_xf = ((d.NN + r.xf_nb - 1) / r.xf_nb) * r.KK;
   r.n_diag_z = ((r.X + r.z_lx - 1) / r.z_lx) * 3;
@@ -811,7 +823,7 @@ int mwf_describe_run(const mwf_run_desc* d, mwf_run_plan* out) {
     p.z_items = (r.X + r.zw_lines - 1) / r.zw_lines;
   } else if (r.fx) {
     p.z_lines = r.fx_lines;
-    p.z_smem = (long long)fx_z_smem(d->K0, d->NN, r.fx_lines);
+    p.z_smem = (long long)fx_z_smem(d->K0, d->NN, r.fx_lines, r.fx_tab);
     p.z_items = ((r.X + r.fx_lines - 1) / r.fx_lines) * 3;
   } else {
     p.z_lines = r.z_lx;
@@ -989,7 +1001,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
   // FP64 runs in fixed point: one launch per pass and block size (and model, for the z pass)
   for (int kind = 0; kind < 3; ++kind)
     for (int K0 : {4, 6})
-      for (int nt : {256, 512}) {
+      for (int nt : {256, 512, 544}) {
         if (kind != 1 && K0 == 6) continue;
         Launch L{kind, 0, K0, 0, nt, 0, items.size(), 0};
         L.fx = true;
@@ -1003,7 +1015,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
           } else if (kind == 1 && r.fx_z_nt == nt && r.d.K0 == K0) {
             for (int x0 = 0; x0 < r.X; x0 += r.fx_lines)
               for (int sub = 0; sub < 3; ++sub) items.push_back(WorkItem{i, x0, sub, 0});
-            L.smem = std::max(L.smem, fx_z_smem(K0, r.d.NN, r.fx_lines));
+            L.smem = std::max(L.smem, fx_z_smem(K0, r.d.NN, r.fx_lines, r.fx_tab));
           } else if (kind == 2 && r.fx_xi_nt == nt) {
             for (int n0 = 0; n0 < r.d.NN; n0 += r.fx_xi_nb)
               for (int k = 0; k < r.d.K0; ++k) items.push_back(WorkItem{i, n0, k, 0});
@@ -1281,7 +1293,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
       put(fo.ms, ms.data(), ms.size() * 8);
       put(fo.rev, rev.data(), rev.size() * sizeof(unsigned short));
       D.fx = 1;
-      D.fx_nb = r.fx_nb; D.fx_xi_nb = r.fx_xi_nb; D.fx_nblk = r.fx_nblk; D.fx_lines = r.fx_lines;
+      D.fx_nb = r.fx_nb; D.fx_xi_nb = r.fx_xi_nb; D.fx_nblk = r.fx_nblk; D.fx_lines = r.fx_lines; D.fx_tab = r.fx_tab; D.fx_group = r.fx_group;
       D.fx_twX = reinterpret_cast<const int4*>(h->arena + fo.twX);
       D.fx_twZ = reinterpret_cast<const int4*>(h->arena + fo.twZ);
       D.fx_twM = reinterpret_cast<const int4*>(h->arena + fo.twM);
