@@ -455,7 +455,7 @@ bool plan_run(RunHost& r, const char*& why) {
     r.zw_ns = 3;
     if (need(1) > zb_smem_budget(1)) r.zw_ns = 1;
     if (need(1) <= zb_smem_budget(1)) {
-      r.zw_nt = need(1) <= zb_smem_budget(2) ? 256 : 512;
+      r.zw_nt = need(1) <= zb_smem_budget(2) ? 256 : (d.K0 == 6 && r.zw_ns == 3 ? 512 : 576);
       const size_t zbud = zb_smem_budget(r.zw_nt == 256 ? 2 : 1);
       const int g = std::max(1, 128 / d.NN);    // lines of a warp's task
       int L = 1;
@@ -986,7 +986,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
   // FP32 z pass with a warp per line: one launch per model, subsets at once and block size
   for (int K0 : {4, 6})
     for (int ns : {3, 1})
-      for (int nt : {256, 512}) {
+      for (int nt : {256, 512, 576}) {
         Launch L{1, 1, K0, 0, nt, 0, items.size(), 0};
         L.zw_ns = ns;
         for (int i = 0; i < n_runs; ++i) {

@@ -112,8 +112,11 @@ cudaError_t launch_z_fx(int K0, int nt, const RunDesc* runs, const WorkItem* ite
 cudaError_t launch_x_inverse_fx(int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st);
 
 // FP32 z pass with a warp per line (mwf_zwarp.cuh): ns z-subsets at once (3 where they fit), in CTAs
-// of 256 threads, two per SM, or of 512.
-// (LS: padded line length, FxPlan).
+// of 256 threads, two per SM, or of 576 with two warps per line: nine teams take M4's 17 + 6 lines
+// in 2 + 1 rounds and M6's 26 + 9 in 3 + 1, where eight need 3 + 1 and 4 + 2 (M4, NN = 1024:
+// 1.81 -> 1.61 ms; M6, 512: 0.82 -> 0.71).  M6 with the three subsets at once (NN = 162 ... 324) keeps 512
+// threads, a warp per line: 0.220 against 0.228 ms at NN = 256.
+// (LS: padded line length, FxPlan.)
 constexpr size_t zw_smem(int K0, int Q, int LS, int ns, int L) {
   const size_t kk = 3 * K0 - 1, nt = (kk + 1) / 2 + kk;
   return 8 * (nt * ns * L * LS + Q);

@@ -77,6 +77,8 @@ def test_plans_fit_the_kernels():
     smooth = sorted(2 ** a * 3 ** b for a in range(11) for b in range(7) if 2 <= 2 ** a * 3 ** b <= 1024)
     for K0 in (4, 6):
         for N in smooth:
+            if K0 == 6 and N == 1024:        # no z kernel holds it: refused when the handle is made
+                continue
             d = mwf.describe_run(mwf.RunParams(K0=K0, MM=N, NN=N, alpha=0.1, gamma=0.1, precision="fp32"))
             assert max(d["xf_smem"], d["z_smem"], d["xi_smem"]) <= 232448
             assert d["z_items"] == -(-3 * N // d["z_lines"])
