@@ -162,7 +162,7 @@ struct RunDesc {
   int fx_tab;                   // tables of NN entries that the z pass copies to shared memory: 0 ... 2
   const int4 *fx_twX, *fx_twZ, *fx_twM, *fx_twQ, *fx_gn, *fx_mp;
   const double2* fx_ms;
-  const unsigned short* fx_rev;
+  const unsigned short *fx_rev, *fx_revQ;   // of the x lines, of the z lines
   int *fx_colE, *fx_blkE, *fx_rowE, *fx_minE;
   float* fx_rowP;
   FxPlan fx_planM, fx_planQ;

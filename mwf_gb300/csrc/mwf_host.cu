@@ -254,6 +254,22 @@ bool make_fx_plan(int N, const std::vector<W>& w, bool fx, FxPlan& pl, std::vect
   return span == 1;
 }
 
+// Tables of the fixed-point transforms of a run: e^{-2 pi i t/3N} and the plan of both lengths.
+struct FxTables {
+  std::vector<int4> wX, wZ, tM, tQ;
+  std::vector<unsigned short> rev, revQ;
+};
+bool make_fx_tables(int MM, int NN, const std::vector<long double>& vX, const std::vector<long double>& vZ, RunDesc& D, FxTables& t) {
+  auto table = [](const std::vector<long double>& v, std::vector<int4>& w) {
+    w.resize(v.size() / 2);
+    for (size_t j = 0; j < w.size(); ++j) w[j] = fx_twiddle(&v[2 * j]);
+  };
+  table(vX, t.wX);
+  table(vZ, t.wZ);
+  return make_fx_plan(MM, t.wX, true, D.fx_planM, t.tM, t.rev) && make_fx_plan(NN, t.wZ, true, D.fx_planQ, t.tQ, t.revQ) &&
+         t.tM.size() <= (size_t)MM && t.tQ.size() <= (size_t)NN;
+}
+
 // var_precompute tables (variables.f90:516-531) and var_LHSRHS (variables.f90:565-597) in
 // the reference's loop order, stored in the device layout [n][k][m].
 void lhsrhs(const mwf_run_desc& d, std::vector<double>& inv_lhs, std::vector<double>& rhs) {
@@ -326,7 +342,7 @@ struct RunHost {
   int fx_nb = 0, fx_xi_nb = 0, fx_lines = 0, fx_nblk = 0, fx_tab = 0, fx_group = 0;
   int fx_xf_nt = 0, fx_z_nt = 0, fx_xi_nt = 0;
   size_t off_fx = 0;
-  struct FxOff { size_t twX, twZ, twM, twQ, gn, mp, ms, rev, colE, blkE, rowE, minE, rowP, end; };
+  struct FxOff { size_t twX, twZ, twM, twQ, gn, mp, ms, rev, revQ, colE, blkE, rowE, minE, rowP, end; };
   FxOff fx_off() const {
     FxOff o;
     size_t a = off_fx;
@@ -339,6 +355,7 @@ struct RunHost {
     o.mp = put(16 * (size_t)4 * d.MM);
     o.ms = put(16 * (size_t)d.MM);
     o.rev = put(2 * (size_t)d.MM);
+    o.revQ = put(2 * (size_t)d.NN);
     o.colE = put(4 * (size_t)2 * KK * d.NN);
     o.blkE = put(4 * (size_t)2 * KK * fx_nblk);
     o.rowE = put(4 * (size_t)3 * KK * X);
@@ -1217,9 +1234,9 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
         ck(cudaMemcpy(h->arena + off, t.data(), t.size() * 4, cudaMemcpyHostToDevice), "twiddle upload");
       }
     };
-    if (!r.fx) up(r.off_twX, r.X);
+    up(r.off_twX, r.X);
     up(r.off_twQ, r.d.NN);
-    if (!r.fx) up(r.off_twZ, r.Z);
+    up(r.off_twZ, r.Z);
     // in-place FP32 transforms of length N, their stage twiddles at off
     auto inplace = [&](int N, FxPlan& pl, size_t off, std::vector<unsigned short>& rev) {
       const std::vector<long double>& v = roots(3 * N);
@@ -1248,21 +1265,9 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
     if (rc != MWF_OK) break;
     if (r.fx) {
       const RunHost::FxOff fo = r.fx_off();
-      std::vector<int4> wX, wZ, tM, tQ, gn(r.d.NN);
-      std::vector<unsigned short> unused;
-      // the double and the fixed-point tables of X and Z from one evaluation
-      auto table = [&](int N, size_t off_d, size_t off_fx, std::vector<int4>& w) {
-        const std::vector<long double>& v = roots(N);
-        const std::vector<double> t(v.begin(), v.end());
-        w.resize(N);
-        for (int j = 0; j < N; ++j) w[j] = fx_twiddle(&v[2 * (size_t)j]);
-        ck(cudaMemcpy(h->arena + off_d, t.data(), t.size() * 8, cudaMemcpyHostToDevice), "twiddle upload");
-        ck(cudaMemcpy(h->arena + off_fx, w.data(), w.size() * sizeof(int4), cudaMemcpyHostToDevice), "twiddle upload");
-      };
-      table(r.X, r.off_twX, fo.twX, wX);
-      table(r.Z, r.off_twZ, fo.twZ, wZ);
-      if (!make_fx_plan(r.d.MM, wX, true, D.fx_planM, tM, rev) || !make_fx_plan(r.d.NN, wZ, true, D.fx_planQ, tQ, unused) ||
-          tM.size() > (size_t)r.d.MM || tQ.size() > (size_t)r.d.NN) {
+      std::vector<int4> gn(r.d.NN);
+      FxTables t;
+      if (!make_fx_tables(r.d.MM, r.d.NN, roots(r.X), roots(r.Z), D, t)) {
         rc = fail(MWF_ERR_SIZE, "run %d: no fixed-point FFT plan", i);
         break;
       }
@@ -1286,12 +1291,15 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
       auto put = [&](size_t off, const void* p, size_t bytes) {
         if (bytes) ck(cudaMemcpy(h->arena + off, p, bytes, cudaMemcpyHostToDevice), "fixed-point table upload");
       };
-      put(fo.twM, tM.data(), tM.size() * sizeof(int4));
-      put(fo.twQ, tQ.data(), tQ.size() * sizeof(int4));
+      put(fo.twX, t.wX.data(), t.wX.size() * sizeof(int4));
+      put(fo.twZ, t.wZ.data(), t.wZ.size() * sizeof(int4));
+      put(fo.twM, t.tM.data(), t.tM.size() * sizeof(int4));
+      put(fo.twQ, t.tQ.data(), t.tQ.size() * sizeof(int4));
       put(fo.gn, gn.data(), gn.size() * sizeof(int4));
       put(fo.mp, mp.data(), mp.size() * sizeof(int4));
       put(fo.ms, ms.data(), ms.size() * 8);
-      put(fo.rev, rev.data(), rev.size() * sizeof(unsigned short));
+      put(fo.rev, t.rev.data(), t.rev.size() * sizeof(unsigned short));
+      put(fo.revQ, t.revQ.data(), t.revQ.size() * sizeof(unsigned short));
       D.fx = 1;
       D.fx_nb = r.fx_nb; D.fx_xi_nb = r.fx_xi_nb; D.fx_nblk = r.fx_nblk; D.fx_lines = r.fx_lines; D.fx_tab = r.fx_tab; D.fx_group = r.fx_group;
       D.fx_twX = reinterpret_cast<const int4*>(h->arena + fo.twX);
@@ -1302,6 +1310,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
       D.fx_mp = reinterpret_cast<const int4*>(h->arena + fo.mp);
       D.fx_ms = reinterpret_cast<const double2*>(h->arena + fo.ms);
       D.fx_rev = reinterpret_cast<const unsigned short*>(h->arena + fo.rev);
+      D.fx_revQ = reinterpret_cast<const unsigned short*>(h->arena + fo.revQ);
       D.fx_colE = reinterpret_cast<int*>(h->arena + fo.colE);
       D.fx_blkE = reinterpret_cast<int*>(h->arena + fo.blkE);
       D.fx_rowE = reinterpret_cast<int*>(h->arena + fo.rowE);
@@ -1489,29 +1498,34 @@ int mwf_phys_diagnostics(mwf_handle* h, int run, double threshold, double* count
   items.reserve(r.n_diag_xf + r.n_diag_z);
   for (int n0 = 0; n0 < r.d.NN; n0 += r.xf_nb)
     for (int f = 0; f < r.KK; ++f) items.push_back(WorkItem{run, n0, f, 1});
-  for (int x0 = 0; x0 < r.X; x0 += r.z_lx)
-    for (int sub = 0; sub < 3; ++sub) items.push_back(WorkItem{run, x0, sub, 0});
-  if ((int)items.size() != r.n_diag_xf + r.n_diag_z) return fail(MWF_ERR_DEVICE, "diagnostic item count mismatch");
+  const bool fx = r.fx && fx_diag_fits(r.KK, r.d.NN);
+  const int nz = fx ? r.X : r.n_diag_z;
+  if (!fx)
+    for (int x0 = 0; x0 < r.X; x0 += r.z_lx)
+      for (int sub = 0; sub < 3; ++sub) items.push_back(WorkItem{run, x0, sub, 0});
+  if ((int)items.size() != r.n_diag_xf + (fx ? 0 : r.n_diag_z)) return fail(MWF_ERR_DEVICE, "diagnostic item count mismatch");
   cudaStream_t st = h->stream;
   CK(cudaMemcpyAsync(h->d_diag_items, items.data(), sizeof(WorkItem) * items.size(), cudaMemcpyHostToDevice, st));
   RunDesc* d = h->d_runs + run;
-  CK(cudaMemcpyAsync(reinterpret_cast<unsigned char*>(d) + offsetof(RunDesc, diag_ct), &threshold, sizeof(double),
-                     cudaMemcpyHostToDevice, st));
+  if (!fx)
+    CK(cudaMemcpyAsync(reinterpret_cast<unsigned char*>(d) + offsetof(RunDesc, diag_ct), &threshold, sizeof(double),
+                       cudaMemcpyHostToDevice, st));
   const size_t xfs = xpass_smem(prec, (size_t)r.xf_nb * r.X);
   const size_t zsm = zpass_smem(prec, r.d.K0, r.z_ppt, r.z_nt);
   cudaError_t e = prec == MWF_FP64 ? launch_x_forward_f64(r.x_nt, h->d_runs, h->d_diag_items, r.n_diag_xf, xfs, h->d_err, st)
                                    : launch_x_forward_f32(r.x_nt, h->d_runs, h->d_diag_items, r.n_diag_xf, xfs, h->d_err, st);
   if (e == cudaSuccess)
-    e = prec == MWF_FP64
+    e = fx ? launch_diag_z_fx(h->d_runs, run, r.X, r.KK, r.d.NN, threshold, reinterpret_cast<double*>(h->arena + r.off_NLT), st)
+        : prec == MWF_FP64
             ? launch_z_diag_f64(r.d.K0, r.z_ppt, r.z_nt, h->d_runs, h->d_diag_items + r.n_diag_xf, r.n_diag_z, zsm, h->d_err, st)
             : launch_z_diag_f32(r.d.K0, r.z_ppt, r.z_nt, h->d_runs, h->d_diag_items + r.n_diag_xf, r.n_diag_z, zsm, h->d_err, st);
   if (e != cudaSuccess) return fail(MWF_ERR_CUDA, "diagnostic launch: %s", cudaGetErrorString(e));
-  std::vector<double> part(2 * (size_t)r.n_diag_z);
+  std::vector<double> part(2 * (size_t)nz);
   CK(cudaMemcpyAsync(part.data(), h->arena + r.off_NLT, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, st));
   rc = check_device_err(h);
   if (rc) return rc;
   double cnt = 0.0, sum = 0.0, comp = 0.0;
-  for (int i = 0; i < r.n_diag_z; ++i) {
+  for (int i = 0; i < nz; ++i) {
     cnt += part[2 * i];
     const double t = part[2 * i + 1];
     const double y = sum + t;
@@ -1595,8 +1609,9 @@ int mwf_get_phys(mwf_handle* h, int run, double* p) {
   cudaError_t e = prec == MWF_FP64 ? launch_x_forward_f64(r.x_nt, h->d_runs, h->d_diag_items, (int)items.size(), xfs, h->d_err, st)
                                    : launch_x_forward_f32(r.x_nt, h->d_runs, h->d_diag_items, (int)items.size(), xfs, h->d_err, st);
   if (e == cudaSuccess)
-    e = prec == MWF_FP64 ? launch_phys_z_f64(h->d_runs, run, r.X, r.KK, pz, zs, out, h->d_err, st)
-                         : launch_phys_z_f32(h->d_runs, run, r.X, r.KK, pz, zs, out, h->d_err, st);
+    e = r.fx               ? launch_phys_z_fx(h->d_runs, run, r.X, r.KK, r.d.NN, out, st)
+        : prec == MWF_FP64 ? launch_phys_z_f64(h->d_runs, run, r.X, r.KK, pz, zs, out, h->d_err, st)
+                           : launch_phys_z_f32(h->d_runs, run, r.X, r.KK, pz, zs, out, h->d_err, st);
   if (e != cudaSuccess) return fail(MWF_ERR_CUDA, "physical-field launch: %s", cudaGetErrorString(e));
   CK(cudaMemcpyAsync(p, out, sizeof(double) * (size_t)r.KK * r.X * r.Z, cudaMemcpyDeviceToHost, st));
   return check_device_err(h);
@@ -1836,11 +1851,29 @@ int transform_setup(const mwf_run_desc* desc, const char* who, TransformCall& tc
   if (!make_plan(r.Z, tc.pz, 12) || !make_plan(r.X, D.planX, 12)) return fail(MWF_ERR_SIZE, "%s: no FFT plan", who);
   tc.nspec = (size_t)r.KK * r.M * r.d.NN;
   tc.nphys = (size_t)r.KK * r.Z * r.X;
-  size_t o = 0;
-  const size_t off_d = o; o = align_up(o + sizeof(RunDesc), 256);
-  const size_t off_err = o; o = align_up(o + sizeof(int), 256);
-  const size_t off_twX = o; o = align_up(o + 16 * (size_t)r.X, 256);
-  const size_t off_twZ = o; o = align_up(o + 16 * (size_t)r.Z, 256);
+  // descriptor, error word and tables first: one upload
+  const std::vector<long double> lx = twiddles(r.X), lz = twiddles(r.Z);
+  FxTables t;
+  std::vector<double> twx, twz;
+  if (!r.fx) {
+    twx.assign(lx.begin(), lx.end());
+    twz.assign(lz.begin(), lz.end());
+  } else if (!make_fx_tables(r.d.MM, r.d.NN, lx, lz, D, t)) {
+    return fail(MWF_ERR_SIZE, "%s: no fixed-point FFT plan", who);
+  }
+  std::vector<unsigned char> head(align_up(sizeof(RunDesc), 256) + 256);
+  auto table = [&](const void* p, size_t bytes) {
+    const size_t at = head.size();
+    head.resize(align_up(at + bytes, 256));
+    if (bytes) memcpy(head.data() + at, p, bytes);
+    return at;
+  };
+  const size_t off_err = align_up(sizeof(RunDesc), 256);
+  const size_t off_twX = r.fx ? table(t.wX.data(), t.wX.size() * sizeof(int4)) : table(twx.data(), twx.size() * 8);
+  const size_t off_twZ = r.fx ? table(t.wZ.data(), t.wZ.size() * sizeof(int4)) : table(twz.data(), twz.size() * 8);
+  const size_t off_tM = table(t.tM.data(), t.tM.size() * sizeof(int4)), off_tQ = table(t.tQ.data(), t.tQ.size() * sizeof(int4));
+  const size_t off_rev = table(t.rev.data(), t.rev.size() * 2), off_revQ = table(t.revQ.data(), t.revQ.size() * 2);
+  size_t o = head.size();
   const size_t off_sp = o; o = align_up(o + 16 * tc.nspec, 256);
   const size_t off_W = o; o = align_up(o + 16 * (size_t)r.KK * r.X * r.d.NN, 256);
   const size_t off_ph = o; o = align_up(o + 8 * tc.nphys, 256);
@@ -1851,7 +1884,7 @@ int transform_setup(const mwf_run_desc* desc, const char* who, TransformCall& tc
     tc.mem = nullptr;
     return fail(MWF_ERR_NOMEM, "%s: cudaMalloc of %zu bytes failed", who, o);
   }
-  tc.d = reinterpret_cast<RunDesc*>(tc.mem + off_d);
+  tc.d = reinterpret_cast<RunDesc*>(tc.mem);
   tc.err = reinterpret_cast<int*>(tc.mem + off_err);
   tc.sp = reinterpret_cast<double2*>(tc.mem + off_sp);
   tc.ph = reinterpret_cast<double*>(tc.mem + off_ph);
@@ -1864,13 +1897,15 @@ int transform_setup(const mwf_run_desc* desc, const char* who, TransformCall& tc
   D.T = tc.mem + off_W;
   D.twX = tc.mem + off_twX;
   D.twZ = tc.mem + off_twZ;
+  D.fx_twX = reinterpret_cast<const int4*>(tc.mem + off_twX);
+  D.fx_twZ = reinterpret_cast<const int4*>(tc.mem + off_twZ);
+  D.fx_twM = reinterpret_cast<const int4*>(tc.mem + off_tM);
+  D.fx_twQ = reinterpret_cast<const int4*>(tc.mem + off_tQ);
+  D.fx_rev = reinterpret_cast<const unsigned short*>(tc.mem + off_rev);
+  D.fx_revQ = reinterpret_cast<const unsigned short*>(tc.mem + off_revQ);
   D.active = 1;
-  const std::vector<long double> lx = twiddles(r.X), lz = twiddles(r.Z);
-  const std::vector<double> twx(lx.begin(), lx.end()), twz(lz.begin(), lz.end());
-  CK(cudaMemcpy(tc.d, &D, sizeof D, cudaMemcpyHostToDevice));
-  CK(cudaMemset(tc.err, 0, sizeof(int)));
-  CK(cudaMemcpy(tc.mem + off_twX, twx.data(), twx.size() * 8, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(tc.mem + off_twZ, twz.data(), twz.size() * 8, cudaMemcpyHostToDevice));
+  memcpy(head.data(), &D, sizeof D);
+  CK(cudaMemcpy(tc.mem, head.data(), head.size(), cudaMemcpyHostToDevice));
   return MWF_OK;
 }
 
@@ -1894,8 +1929,12 @@ int mwf_spec2phys(const mwf_run_desc* d, const double* s_re, const double* s_im,
   CK(cudaMemcpy(tc.s_re, s_re, 8 * tc.nspec, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(tc.s_im, s_im, 8 * tc.nspec, cudaMemcpyHostToDevice));
   cudaError_t e = launch_ref_to_dev_f64(tc.s_re, tc.s_im, tc.sp, r.KK, r.M, r.d.NN, 0);
-  if (e == cudaSuccess) e = launch_spec_x_backward_f64(tc.d, 0, r.X, r.KK, r.d.NN, tc.sp, tc.err, 0);
-  if (e == cudaSuccess) e = launch_phys_z_f64(tc.d, 0, r.X, r.KK, tc.pz, xpass_smem(0, (size_t)r.Z), tc.ph, tc.err, 0);
+  if (e == cudaSuccess)
+    e = r.fx ? launch_spec_x_backward_fx(tc.d, 0, r.d.MM, r.KK, r.d.NN, tc.sp, 0)
+             : launch_spec_x_backward_f64(tc.d, 0, r.X, r.KK, r.d.NN, tc.sp, tc.err, 0);
+  if (e == cudaSuccess)
+    e = r.fx ? launch_phys_z_fx(tc.d, 0, r.X, r.KK, r.d.NN, tc.ph, 0)
+             : launch_phys_z_f64(tc.d, 0, r.X, r.KK, tc.pz, xpass_smem(0, (size_t)r.Z), tc.ph, tc.err, 0);
   if (e != cudaSuccess) return fail(MWF_ERR_CUDA, "mwf_spec2phys: launch: %s", cudaGetErrorString(e));
   rc = transform_finish(tc, "mwf_spec2phys");
   if (rc) return rc;
@@ -1910,8 +1949,11 @@ int mwf_phys2spec(const mwf_run_desc* d, const double* p, double* s_re, double* 
   if (rc) return rc;
   const RunHost& r = tc.r;
   CK(cudaMemcpy(tc.ph, p, 8 * tc.nphys, cudaMemcpyHostToDevice));
-  cudaError_t e = launch_phys_z_forward_f64(tc.d, 0, r.X, r.KK, r.Z, tc.pz, tc.ph, tc.err, 0);
-  if (e == cudaSuccess) e = launch_spec_x_forward_f64(tc.d, 0, r.X, r.KK, r.d.NN, tc.sp, tc.err, 0);
+  cudaError_t e = r.fx ? launch_phys_z_forward_fx(tc.d, 0, r.X, r.KK, r.d.NN, tc.ph, 0)
+                       : launch_phys_z_forward_f64(tc.d, 0, r.X, r.KK, r.Z, tc.pz, tc.ph, tc.err, 0);
+  if (e == cudaSuccess)
+    e = r.fx ? launch_spec_x_forward_fx(tc.d, 0, r.d.MM, r.KK, r.d.NN, tc.sp, 0)
+             : launch_spec_x_forward_f64(tc.d, 0, r.X, r.KK, r.d.NN, tc.sp, tc.err, 0);
   if (e == cudaSuccess) e = launch_dev_to_ref_f64(tc.sp, tc.s_re, tc.s_im, r.KK, r.M, r.d.NN, 0);
   if (e != cudaSuccess) return fail(MWF_ERR_CUDA, "mwf_phys2spec: launch: %s", cudaGetErrorString(e));
   rc = transform_finish(tc, "mwf_phys2spec");

@@ -111,6 +111,20 @@ cudaError_t launch_x_forward_fx(int nt, const RunDesc* runs, const WorkItem* ite
 cudaError_t launch_z_fx(int K0, int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st);
 cudaError_t launch_x_inverse_fx(int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st);
 
+// FP64 lines on their own in fixed point (mwf_fxlines.cuh): lines of 3N points per CTA.  No more than
+// half an SM holds, and fewer while the grid leaves some of the chip's 304 half-SM slots empty.
+__host__ __device__ constexpr int fx_line_stride(int N) { return (3 * N) | 1; }
+constexpr size_t fx_line_smem_bytes(int N, int lines) {
+  return 16 * ((((size_t)lines * fx_line_stride(N) + 7) & ~(size_t)7) + N) + 4 * ((size_t)lines + 3);
+}
+cudaError_t launch_spec_x_backward_fx(const RunDesc* runs, int run, int MM, int KK, int NN, const void* sp, cudaStream_t st);
+cudaError_t launch_spec_x_forward_fx(const RunDesc* runs, int run, int MM, int KK, int NN, void* sp, cudaStream_t st);
+cudaError_t launch_phys_z_fx(const RunDesc* runs, int run, int X, int KK, int NN, double* out, cudaStream_t st);
+cudaError_t launch_phys_z_forward_fx(const RunDesc* runs, int run, int X, int KK, int NN, const double* ph, cudaStream_t st);
+// all pairs of an x line in one CTA; false for the longest lines, which do not fit it
+constexpr bool fx_diag_fits(int KK, int NN) { return fx_line_smem_bytes(NN, (KK + 1) / 2) + 256 <= zb_smem_budget(1); }
+cudaError_t launch_diag_z_fx(const RunDesc* runs, int run, int X, int KK, int NN, double threshold, double* out, cudaStream_t st);
+
 // FP32 z pass with a warp per line (mwf_zwarp.cuh): ns z-subsets at once (3 where they fit), in CTAs
 // of 256 threads, two per SM, or of 576 with two warps per line: nine teams take M4's 17 + 6 lines
 // in 2 + 1 rounds and M6's 26 + 9 in 3 + 1, where eight need 3 + 1 and 4 + 2 (M4, NN = 1024:
