@@ -59,8 +59,10 @@ static cudaError_t fx_line_launch(K k, long grid, int N, int lines, cudaStream_t
 
 cudaError_t launch_spec_x_backward_fx(const RunDesc* runs, int run, int MM, int KK, int NN, const void* sp, cudaStream_t st) {
   const int nb = fx_line_tile(MM, NN, 8, KK);
-  return fx_line_launch(spec_x_backward_fx_kernel, (long)KK * ((NN + nb - 1) / nb), MM, nb, st, runs, run, nb,
-                        reinterpret_cast<const double2*>(sp));
+  const long grid = (long)KK * ((NN + nb - 1) / nb);
+  const double2* in = reinterpret_cast<const double2*>(sp);
+  return in ? fx_line_launch(spec_x_backward_fx_kernel<false>, grid, MM, nb, st, runs, run, nb, in)
+            : fx_line_launch(spec_x_backward_fx_kernel<true>, grid, MM, nb, st, runs, run, nb, in);
 }
 
 cudaError_t launch_spec_x_forward_fx(const RunDesc* runs, int run, int MM, int KK, int NN, void* sp, cudaStream_t st) {

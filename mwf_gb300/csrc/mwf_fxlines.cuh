@@ -120,7 +120,9 @@ __device__ __forceinline__ FxLineSmem fx_line_smem(unsigned char* p, int N, int 
   return s;
 }
 
-// x backward: field f, columns n0 ... n0 + nb - 1 of sp[n][f][ms] -> W[f][x][n].
+// x backward: field f, columns n0 ... n0 + nb - 1 of sp[n][f][ms] -> W[f][x][n].  STATE: of the
+// perturbation fields of the run's state (var_mpt2spec) in the place of sp.
+template <bool STATE>
 __global__ void __launch_bounds__(kFxLineThreads) spec_x_backward_fx_kernel(const RunDesc* __restrict__ runs, int run, int nb,
                                                                             const double2* __restrict__ sp) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -131,8 +133,17 @@ __global__ void __launch_bounds__(kFxLineThreads) spec_x_backward_fx_kernel(cons
   const FastDiv f2 = make_fastdiv(2 * MM), fMM = make_fastdiv(MM);
   for (int i = threadIdx.x; i < cols * 2 * MM; i += kFxLineThreads) {
     const int l = f2.div(i), ms = i - l * 2 * MM;     // slot MM is the m = -MM that no field has
-    const double2* __restrict__ row = sp + ((size_t)(n0 + l) * KK + f) * M;
-    fx_put_raw(S.buf, l * S.PS + ms, ms == MM ? make_double2(0.0, 0.0) : row[ms < MM ? ms : ms - 1]);
+    double2 v = make_double2(0.0, 0.0);
+    if (ms != MM) {
+      if constexpr (STATE) {
+        const int n = n0 + l, m = ms < MM ? ms : ms - 2 * MM;
+        v = mpt_to_field_w<double>(R, reinterpret_cast<const double2*>(R.c), f, m, n, false, R.alpha * m, R.gamma * n,
+                                   kbeta<double>(field_k(f, R.K0)));
+      } else {
+        v = sp[((size_t)(n0 + l) * KK + f) * M + (ms < MM ? ms : ms - 1)];
+      }
+    }
+    fx_put_raw(S.buf, l * S.PS + ms, v);
   }
   __syncthreads();
   for (int l = threadIdx.x >> 5; l < cols; l += kFxLineThreads / 32) {

@@ -713,6 +713,25 @@ int build_graph(mwf_handle* h, int steps, cudaGraphExec_t* out) {
   return MWF_OK;
 }
 
+// x forward of the run's perturbation fields (without the base flow) by the kernels of the timestep;
+// with_z: the items of the diagnostic z pass go up behind its own.
+int diag_x_forward(mwf_handle* h, int run, bool with_z, cudaError_t& e) {
+  const RunHost& r = h->runs[run];
+  std::vector<WorkItem> items;
+  items.reserve(r.n_diag_xf + r.n_diag_z);
+  for (int n0 = 0; n0 < r.d.NN; n0 += r.xf_nb)
+    for (int f = 0; f < r.KK; ++f) items.push_back(WorkItem{run, n0, f, 1});
+  if (with_z)
+    for (int x0 = 0; x0 < r.X; x0 += r.z_lx)
+      for (int sub = 0; sub < 3; ++sub) items.push_back(WorkItem{run, x0, sub, 0});
+  if ((int)items.size() != r.n_diag_xf + (with_z ? r.n_diag_z : 0)) return fail(MWF_ERR_DEVICE, "diagnostic item count mismatch");
+  CK(cudaMemcpyAsync(h->d_diag_items, items.data(), sizeof(WorkItem) * items.size(), cudaMemcpyHostToDevice, h->stream));
+  const size_t xfs = xpass_smem(r.d.precision, (size_t)r.xf_nb * r.X);
+  e = r.d.precision == MWF_FP64 ? launch_x_forward_f64(r.x_nt, h->d_runs, h->d_diag_items, r.n_diag_xf, xfs, h->d_err, h->stream)
+                                : launch_x_forward_f32(r.x_nt, h->d_runs, h->d_diag_items, r.n_diag_xf, xfs, h->d_err, h->stream);
+  return MWF_OK;
+}
+
 // Wait for the stream; the error word is in h_out->err by then.
 int finish_call(mwf_handle* h) {
   CK(cudaStreamSynchronize(h->stream));
@@ -1494,31 +1513,26 @@ int mwf_phys_diagnostics(mwf_handle* h, int run, double threshold, double* count
   const RunHost& r = h->runs[run];
   if (!r.active) return fail(MWF_ERR_ARG, "run %d is not active", run);
   const int prec = r.d.precision;
-  std::vector<WorkItem> items;
-  items.reserve(r.n_diag_xf + r.n_diag_z);
-  for (int n0 = 0; n0 < r.d.NN; n0 += r.xf_nb)
-    for (int f = 0; f < r.KK; ++f) items.push_back(WorkItem{run, n0, f, 1});
   const bool fx = r.fx && fx_diag_fits(r.KK, r.d.NN);
   const int nz = fx ? r.X : r.n_diag_z;
-  if (!fx)
-    for (int x0 = 0; x0 < r.X; x0 += r.z_lx)
-      for (int sub = 0; sub < 3; ++sub) items.push_back(WorkItem{run, x0, sub, 0});
-  if ((int)items.size() != r.n_diag_xf + (fx ? 0 : r.n_diag_z)) return fail(MWF_ERR_DEVICE, "diagnostic item count mismatch");
   cudaStream_t st = h->stream;
-  CK(cudaMemcpyAsync(h->d_diag_items, items.data(), sizeof(WorkItem) * items.size(), cudaMemcpyHostToDevice, st));
   RunDesc* d = h->d_runs + run;
-  if (!fx)
+  cudaError_t e;
+  if (fx) {
+    e = launch_spec_x_backward_fx(h->d_runs, run, r.d.MM, r.KK, r.d.NN, nullptr, st);
+    if (e == cudaSuccess)
+      e = launch_diag_z_fx(h->d_runs, run, r.X, r.KK, r.d.NN, threshold, reinterpret_cast<double*>(h->arena + r.off_NLT), st);
+  } else {
+    rc = diag_x_forward(h, run, true, e);
+    if (rc) return rc;
     CK(cudaMemcpyAsync(reinterpret_cast<unsigned char*>(d) + offsetof(RunDesc, diag_ct), &threshold, sizeof(double),
                        cudaMemcpyHostToDevice, st));
-  const size_t xfs = xpass_smem(prec, (size_t)r.xf_nb * r.X);
-  const size_t zsm = zpass_smem(prec, r.d.K0, r.z_ppt, r.z_nt);
-  cudaError_t e = prec == MWF_FP64 ? launch_x_forward_f64(r.x_nt, h->d_runs, h->d_diag_items, r.n_diag_xf, xfs, h->d_err, st)
-                                   : launch_x_forward_f32(r.x_nt, h->d_runs, h->d_diag_items, r.n_diag_xf, xfs, h->d_err, st);
-  if (e == cudaSuccess)
-    e = fx ? launch_diag_z_fx(h->d_runs, run, r.X, r.KK, r.d.NN, threshold, reinterpret_cast<double*>(h->arena + r.off_NLT), st)
-        : prec == MWF_FP64
-            ? launch_z_diag_f64(r.d.K0, r.z_ppt, r.z_nt, h->d_runs, h->d_diag_items + r.n_diag_xf, r.n_diag_z, zsm, h->d_err, st)
-            : launch_z_diag_f32(r.d.K0, r.z_ppt, r.z_nt, h->d_runs, h->d_diag_items + r.n_diag_xf, r.n_diag_z, zsm, h->d_err, st);
+    const size_t zsm = zpass_smem(prec, r.d.K0, r.z_ppt, r.z_nt);
+    if (e == cudaSuccess)
+      e = prec == MWF_FP64
+              ? launch_z_diag_f64(r.d.K0, r.z_ppt, r.z_nt, h->d_runs, h->d_diag_items + r.n_diag_xf, r.n_diag_z, zsm, h->d_err, st)
+              : launch_z_diag_f32(r.d.K0, r.z_ppt, r.z_nt, h->d_runs, h->d_diag_items + r.n_diag_xf, r.n_diag_z, zsm, h->d_err, st);
+  }
   if (e != cudaSuccess) return fail(MWF_ERR_CUDA, "diagnostic launch: %s", cudaGetErrorString(e));
   std::vector<double> part(2 * (size_t)nz);
   CK(cudaMemcpyAsync(part.data(), h->arena + r.off_NLT, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, st));
@@ -1597,21 +1611,20 @@ int mwf_get_phys(mwf_handle* h, int run, double* p) {
   FftPlanDev pz{};
   if (!make_plan(r.Z, pz, prec == MWF_FP64 ? 12 : 16) || r.Z > kPhysVpt * kPhysThreads)
     return fail(MWF_ERR_SIZE, "no z plan for Z = %d", r.Z);
-  std::vector<WorkItem> items;
-  items.reserve(r.n_diag_xf);
-  for (int n0 = 0; n0 < r.d.NN; n0 += r.xf_nb)
-    for (int f = 0; f < r.KK; ++f) items.push_back(WorkItem{run, n0, f, 1});
   cudaStream_t st = h->stream;
-  CK(cudaMemcpyAsync(h->d_diag_items, items.data(), sizeof(WorkItem) * items.size(), cudaMemcpyHostToDevice, st));
-  const size_t xfs = xpass_smem(prec, (size_t)r.xf_nb * r.X);
   const size_t zs = xpass_smem(prec, (size_t)r.Z);
   double* out = reinterpret_cast<double*>(h->arena + r.off_NLT);   // KK*X*Z doubles fit the NLT scratch
-  cudaError_t e = prec == MWF_FP64 ? launch_x_forward_f64(r.x_nt, h->d_runs, h->d_diag_items, (int)items.size(), xfs, h->d_err, st)
-                                   : launch_x_forward_f32(r.x_nt, h->d_runs, h->d_diag_items, (int)items.size(), xfs, h->d_err, st);
-  if (e == cudaSuccess)
-    e = r.fx               ? launch_phys_z_fx(h->d_runs, run, r.X, r.KK, r.d.NN, out, st)
-        : prec == MWF_FP64 ? launch_phys_z_f64(h->d_runs, run, r.X, r.KK, pz, zs, out, h->d_err, st)
+  cudaError_t e;
+  if (r.fx) {
+    e = launch_spec_x_backward_fx(h->d_runs, run, r.d.MM, r.KK, r.d.NN, nullptr, st);
+    if (e == cudaSuccess) e = launch_phys_z_fx(h->d_runs, run, r.X, r.KK, r.d.NN, out, st);
+  } else {
+    rc = diag_x_forward(h, run, false, e);
+    if (rc) return rc;
+    if (e == cudaSuccess)
+      e = prec == MWF_FP64 ? launch_phys_z_f64(h->d_runs, run, r.X, r.KK, pz, zs, out, h->d_err, st)
                            : launch_phys_z_f32(h->d_runs, run, r.X, r.KK, pz, zs, out, h->d_err, st);
+  }
   if (e != cudaSuccess) return fail(MWF_ERR_CUDA, "physical-field launch: %s", cudaGetErrorString(e));
   CK(cudaMemcpyAsync(p, out, sizeof(double) * (size_t)r.KK * r.X * r.Z, cudaMemcpyDeviceToHost, st));
   return check_device_err(h);

@@ -117,6 +117,7 @@ __host__ __device__ constexpr int fx_line_stride(int N) { return (3 * N) | 1; }
 constexpr size_t fx_line_smem_bytes(int N, int lines) {
   return 16 * ((((size_t)lines * fx_line_stride(N) + 7) & ~(size_t)7) + N) + 4 * ((size_t)lines + 3);
 }
+// sp = nullptr: the fields of the run's state
 cudaError_t launch_spec_x_backward_fx(const RunDesc* runs, int run, int MM, int KK, int NN, const void* sp, cudaStream_t st);
 cudaError_t launch_spec_x_forward_fx(const RunDesc* runs, int run, int MM, int KK, int NN, void* sp, cudaStream_t st);
 cudaError_t launch_phys_z_fx(const RunDesc* runs, int run, int X, int KK, int NN, double* out, cudaStream_t st);
