@@ -368,6 +368,31 @@ struct RunHost {
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
+// Items of one launch: each takes up to *width of a run's `lines`, `per` times.
+struct ItemWidth {
+  int* width;
+  int lines, per;
+  bool fixed;        // by a tuning knob
+};
+// plan_run takes the widest items that fit, which read and set up the least per line.  A launch whose runs
+// together give fewer than `slots` of them leaves SMs without one while each item takes its lines
+// in turn, so there the narrowest width that still makes one round is taken.
+void spread_items(std::vector<ItemWidth>& v, int slots, bool pow2) {
+  int widest = 1;
+  for (const ItemWidth& x : v) widest = std::max(widest, *x.width);
+  int w = 1;
+  for (; w < widest; w = pow2 ? 2 * w : w + 1) {
+    long items = 0;
+    for (const ItemWidth& x : v) {
+      const int own = x.fixed ? *x.width : std::min(w, *x.width);
+      items += (long)((x.lines + own - 1) / own) * x.per;
+    }
+    if (items <= slots) break;
+  }
+  for (const ItemWidth& x : v)
+    if (!x.fixed) *x.width = std::min(w, *x.width);
+}
+
 // Tiling of one run; returns false if the run does not fit the kernels' shapes.
 bool plan_run(RunHost& r, const char*& why) {
   const mwf_run_desc& d = r.d;
@@ -911,6 +936,30 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
 #ifndef MWF_NO_PERSIST
   for (RunHost& r : h->runs) r.persist = r.d.precision == MWF_FP32 && r.xbf_nb && r.zb_lx && r.xbi_nb;
 #endif
+  // FP32 items by what their launch holds.  One run, us a step with the widest items and with these: M4,
+  // 32 x 32 18.5 and 13.3, 64 x 64 23.8 and 16.5, 36 x 36 40.5 and 22.8, 72 x 72 54.2 and 28.9; M6, 64 x 64
+  // 25.2 and 21.1, 72 x 72 54.4 and 39.1; eight M4 36 x 36 43.5 and 37.  Full launches keep the widest.
+  {
+    std::map<std::vector<int>, std::vector<ItemWidth>> xf, z, xi, xwf, xwi, zw;
+    for (RunHost& r : h->runs) {
+      const mwf_run_desc& d = r.d;
+      const int pset = r.persist ? 1 : 0;
+      if (r.xbf_nb) xf[{pset, d.MM}].push_back({&r.xbf_nb, d.NN, d.K0, d.xf_cols != 0});
+      if (r.xbi_nb) xi[{pset, d.MM}].push_back({&r.xbi_nb, d.NN, d.K0, d.xi_cols != 0});
+      if (r.zb_lx) z[{pset, d.K0, d.NN}].push_back({&r.zb_lx, r.X, 1, d.z_lines != 0});
+      if (r.xw_fnb) xwf[{r.xw_fnt}].push_back({&r.xw_fnb, d.NN, d.K0, false});
+      if (r.xw_inb) xwi[{r.xw_int}].push_back({&r.xw_inb, d.NN, d.K0, false});
+      if (r.zw_lines) zw[{d.K0, r.zw_ns, r.zw_nt}].push_back({&r.zw_lines, r.X, 1, false});
+    }
+    // rounds that the resident CTAs make; past these the narrower items' setup costs more (at
+    // M4 128 x 128 modes and 228 x forward items 33.7 us, with 128 of them 30.0)
+    for (auto& g : xf) spread_items(g.second, 152, false);
+    for (auto& g : xi) spread_items(g.second, 304, false);
+    for (auto& g : z) spread_items(g.second, 304, false);
+    for (auto& g : xwf) spread_items(g.second, 304, true);
+    for (auto& g : xwi) spread_items(g.second, 456, true);
+    for (auto& g : zw) spread_items(g.second, 304, false);
+  }
   // launch groups of the other runs and of the runs that can step in the persistent kernel
   auto build_groups = [&](bool pset) {
   for (int prec = 0; prec < 2; ++prec) {

@@ -84,3 +84,22 @@ def test_plans_fit_the_kernels():
             assert d["z_items"] == -(-3 * N // d["z_lines"])
             if not d["batched_x"]:
                 assert d["xf_items"] == -(-N // d["xf_cols"]) * K0 and d["xi_items"] == -(-N // d["xi_cols"]) * K0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K0,MM,NN", [(4, 32, 32), (6, 64, 48), (4, 27, 36), (6, 72, 18), (4, 64, 54), (4, 128, 2)])
+def test_a_run_alone_and_among_many(built_lib, K0, MM, NN):
+    """A launch that its runs do not fill takes narrower items: the same sums in the same order for each
+    line, so a run steps alike alone and among as many as fill the launch, to the rounding of differently
+    contracted products (a few 6e-8 of the state's norm in three steps)."""
+    p = mwf.RunParams(K0=K0, MM=MM, NN=NN, alpha=3.0 / MM, gamma=3.0 / NN, dt=0.01, precision="fp32")
+    c0 = mwf.ic.gaussian_ic(p, seed=3)
+    out = []
+    for n in (1, 5, 40):
+        with mwf.Ensemble([p] * n) as ens:
+            for i in range(n):
+                ens.set_state(i, c0)
+            ens.step(3)
+            out += [ens.get_state(0), ens.get_state(n - 1)]
+    for g in out[1:]:
+        assert np.linalg.norm(g - out[0]) <= 1e-6 * np.linalg.norm(out[0])
