@@ -164,7 +164,7 @@ struct RunDesc {
   const double2* fx_ms;
   const unsigned short *fx_rev, *fx_revQ;   // of the x lines, of the z lines
   int *fx_colE, *fx_blkE, *fx_rowE, *fx_minE;
-  float* fx_rowP;
+  unsigned* fx_rowP;
   FxPlan fx_planM, fx_planQ;
 };
 

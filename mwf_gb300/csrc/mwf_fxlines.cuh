@@ -11,8 +11,7 @@
 // What bounds them: latency -- a few hundred small CTAs run once.  The kernels before took one line
 // to a CTA of 256 or 512 threads, of which N/12 had a butterfly, and wrote 8 of every 88 or 136 bytes:
 // M6, 64 x 64 modes: x backward 47 us, z backward 119, z forward 118, x forward 47.
-// Error: the rounding of the line transforms is 2^-62 of the line's L1 norm per stage, below that
-// of FP64 arithmetic (mwf_fx.cuh).
+// Error against 80-bit arithmetic, sizes 9 ... 128: 0.3 ... 0.6 of that of the FP64-arithmetic kernels.
 #pragma once
 #include "mwf_fxpass.cuh"
 
@@ -34,7 +33,8 @@ __device__ __forceinline__ void fx_put_raw(longlong2* buf, int i, double2 v) {
 
 // Exponent e with 2^extra sum(|re| + |im|) 2^e <= 2^61 over the `count` values from place `base`, by
 // one warp: the largest high word first, then the sum relative to it, as in fx_row_moments.
-__device__ __forceinline__ int fx_line_exponent(const longlong2* buf, int base, int count, int extra) {
+// fine: fx_fine of the line, of which a value of a subset line is a sum of 2^(extra + 1) values backward, one forward.
+__device__ __forceinline__ int fx_line_exponent(const longlong2* buf, int base, int count, int extra, const FxPlan& pl, bool inv, int& fine) {
   const int lane = threadIdx.x & 31;
   int t = 0;
   for (int i = lane; i < count; i += 32) {
@@ -42,18 +42,23 @@ __device__ __forceinline__ int fx_line_exponent(const longlong2* buf, int base, 
     t = max(t, max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff));
   }
   const int top = __reduce_max_sync(0xffffffffu, t) >> 20;
+  fine = 0;
   if (top == 0) return kFxZero;
   if (top >= 0x7ff) return kFxNan;
   auto part = [&](double x) {
     const int h = __double2hiint(x) & 0x7fffffff, q = h - (top - 127) * (1 << 20);
     return q < (1 << 20) || h < (1 << 20) ? 0.f : __int_as_float(q << 3);
   };
-  float a = 0.f;
+  float a = 0.f, m = 0.f;
   for (int i = lane; i < count; i += 32) {
     const double2 v = fx_raw(buf, base + i);
-    a += part(v.x) + part(v.y);
+    const float b = part(v.x) + part(v.y);
+    a += b;
+    m = fmaxf(m, b);
   }
-  return 61 - (fx_bits_above(fx_warp_sum(a) * 1.001f) + top - 1023 + extra);
+  const int e = 61 - (fx_bits_above(fx_warp_sum(a) * 1.001f) + top - 1023 + extra);
+  fine = fx_fine(pl, inv, fx_warp_max(m), top - 1023 + (inv ? extra + 1 : 0), e);
+  return e;
 }
 
 __device__ __forceinline__ longlong2 fx_from_double2(double2 v, int e) {
@@ -73,8 +78,8 @@ __device__ __forceinline__ void fx_put_subsets(longlong2* buf, int base, int N, 
   constexpr FxConst s3 = fx_const(kFxSqrt34);
   const i64 rx = fx_mulc(b.x, s3), ry = fx_mulc(b.y, s3);
   longlong2 h, p, q;
-  h.x = a.x - (b.x >> 1);
-  h.y = a.y - (b.y >> 1);
+  h.x = a.x - fx_half(b.x);
+  h.y = a.y - fx_half(b.y);
   p.x = h.x + ry; p.y = h.y - rx;
   q.x = h.x - ry; q.y = h.y + rx;
   buf[fx_at(base + j)] = cadd(a, b);
@@ -89,22 +94,13 @@ __device__ __forceinline__ longlong2 fx_join_subsets(const longlong2* buf, int b
   return cadd(cadd(f0, fx_cmul<NEG>(f1, om[j])), fx_cmul<NEG>(f2, om[2 * j]));
 }
 
-// All subsets of `lines` lines PS apart: a warp per subset, or per line where the three are short.
-template <bool INV>
-__device__ __forceinline__ void fx_line_ffts(longlong2* buf, int lines, int PS, const FxPlan& pl, const int4* tw, int* zero) {
-  const int per = pl.N <= 85 ? 1 : 3;
-  for (int t = threadIdx.x >> 5; t < lines * per; t += kFxLineThreads / 32) {
-    const int l = per == 1 ? t : t / 3;
-    fx_fft<INV>(buf, l * PS + (t - l * per) * pl.N, per == 1 ? 3 : 1, pl, tw, INV ? nullptr : zero);
-  }
-}
-
 // Shared memory of the line kernels: lines (odd stride, so that lanes on neighbouring lines spread
 // over the banks), stage twiddles, one exponent per line.
 struct FxLineSmem {
   longlong2* buf;
   int4* tw;
   int* e;
+  int* fine;        // three times, for the subsets
   int* zero;        // the shift of the forward transforms' first stage
   int PS;
 };
@@ -114,10 +110,26 @@ __device__ __forceinline__ FxLineSmem fx_line_smem(unsigned char* p, int N, int 
   s.buf = reinterpret_cast<longlong2*>(p);
   s.tw = reinterpret_cast<int4*>(s.buf + ((lines * s.PS + 7) & ~7));
   s.e = reinterpret_cast<int*>(s.tw + N);
-  s.zero = s.e + lines;
+  s.fine = s.e + lines;
+  s.zero = s.fine + 3 * lines;
   for (int i = threadIdx.x; i < N; i += kFxLineThreads) s.tw[i] = stage[i];
   if (threadIdx.x < 3) s.zero[threadIdx.x] = 0;
   return s;
+}
+
+// All subsets of `lines` lines: a warp per subset, or per line where the three are short.
+template <bool INV>
+__device__ __forceinline__ void fx_line_ffts(const FxLineSmem& S, int lines, const FxPlan& pl) {
+  const int per = pl.N <= 85 ? 1 : 3;
+  for (int t = threadIdx.x >> 5; t < lines * per; t += kFxLineThreads / 32) {
+    const int l = per == 1 ? t : t / 3;
+    fx_fft<INV>(S.buf, l * S.PS + (t - l * per) * pl.N, per == 1 ? 3 : 1, pl, S.tw, INV ? nullptr : S.zero, S.fine + 3 * l, 1);
+  }
+}
+
+__device__ __forceinline__ void fx_line_scale(const FxLineSmem& S, int l, int e, int g) {
+  S.e[l] = e;
+  for (int i = 0; i < 3; ++i) S.fine[3 * l + i] = g;
 }
 
 // x backward: field f, columns n0 ... n0 + nb - 1 of sp[n][f][ms] -> W[f][x][n].  STATE: of the
@@ -147,18 +159,20 @@ __global__ void __launch_bounds__(kFxLineThreads) spec_x_backward_fx_kernel(cons
   }
   __syncthreads();
   for (int l = threadIdx.x >> 5; l < cols; l += kFxLineThreads / 32) {
-    const int e = fx_line_exponent(S.buf, l * S.PS, 2 * MM, 0);
-    if ((threadIdx.x & 31) == 0) S.e[l] = e;
+    int g;
+    const int e = fx_line_exponent(S.buf, l * S.PS, 2 * MM, 0, R.fx_planM, true, g);
+    if ((threadIdx.x & 31) == 0) fx_line_scale(S, l, e, g);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < cols * MM; i += kFxLineThreads) {
     const int l = fMM.div(i), j = i - l * MM, base = l * S.PS;
-    const longlong2 a = fx_from_double2(fx_raw(S.buf, base + j), S.e[l]);
-    const longlong2 b = fx_from_double2(fx_raw(S.buf, base + MM + j), S.e[l]);
+    const int e = S.e[l] + fx_fine_bits(S.fine[3 * l]);
+    const longlong2 a = fx_from_double2(fx_raw(S.buf, base + j), e);
+    const longlong2 b = fx_from_double2(fx_raw(S.buf, base + MM + j), e);
     fx_put_subsets(S.buf, base, MM, j, a, b, R.fx_twX);
   }
   __syncthreads();
-  fx_line_ffts<true>(S.buf, cols, S.PS, R.fx_planM, S.tw, S.zero);
+  fx_line_ffts<true>(S, cols, R.fx_planM);
   __syncthreads();
   double2* __restrict__ W = reinterpret_cast<double2*>(R.T) + (size_t)f * X * NN;
   const FastDiv fc = make_fastdiv(cols);
@@ -186,16 +200,17 @@ __global__ void __launch_bounds__(kFxLineThreads) spec_x_forward_fx_kernel(const
   }
   __syncthreads();
   for (int l = threadIdx.x >> 5; l < cols; l += kFxLineThreads / 32) {
-    const int e = fx_line_exponent(S.buf, l * S.PS, X, 0);
-    if ((threadIdx.x & 31) == 0) S.e[l] = e;
+    int g;
+    const int e = fx_line_exponent(S.buf, l * S.PS, X, 0, R.fx_planM, false, g);
+    if ((threadIdx.x & 31) == 0) fx_line_scale(S, l, e, g);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < cols * X; i += kFxLineThreads) {
     const int l = fX.div(i), at = l * S.PS + i - l * X;
-    S.buf[fx_at(at)] = fx_from_double2(fx_raw(S.buf, at), S.e[l]);
+    S.buf[fx_at(at)] = fx_from_double2(fx_raw(S.buf, at), S.e[l] + fx_fine_bits(S.fine[3 * l]));
   }
   __syncthreads();
-  fx_line_ffts<false>(S.buf, cols, S.PS, R.fx_planM, S.tw, S.zero);
+  fx_line_ffts<false>(S, cols, R.fx_planM);
   __syncthreads();
   for (int i = threadIdx.x; i < cols * M; i += kFxLineThreads) {
     const int l = fM.div(i), ms = i - l * M, m = signed_m(ms, MM, M), e = S.e[l];
@@ -221,14 +236,15 @@ __device__ __forceinline__ void fx_z_backward(const RunDesc& R, const FxLineSmem
   }
   __syncthreads();
   for (int l = threadIdx.x >> 5; l < pairs; l += kFxLineThreads / 32) {
-    const int e = fx_line_exponent(S.buf, l * S.PS, 2 * NN, 1);
-    if ((threadIdx.x & 31) == 0) S.e[l] = e;
+    int g;
+    const int e = fx_line_exponent(S.buf, l * S.PS, 2 * NN, 1, R.fx_planQ, true, g);
+    if ((threadIdx.x & 31) == 0) fx_line_scale(S, l, e, g);
   }
   __syncthreads();
   const int slots = NN / 2 + 1;                       // j and NN - j together: each needs the other's input
   const FastDiv fS = make_fastdiv(slots);
   for (int i = threadIdx.x; i < pairs * slots; i += kFxLineThreads) {
-    const int l = fS.div(i), j = i - l * slots, jq = NN - j, base = l * S.PS, e = S.e[l];
+    const int l = fS.div(i), j = i - l * slots, jq = NN - j, base = l * S.PS, e = S.e[l] + fx_fine_bits(S.fine[3 * l]);
     const longlong2 a = fx_from_double2(fx_raw(S.buf, base + j), e), b = fx_from_double2(fx_raw(S.buf, base + NN + j), e);
     longlong2 u, v;
     u.x = a.x - b.y; u.y = a.y + b.x;                 // coefficient at j
@@ -245,7 +261,7 @@ __device__ __forceinline__ void fx_z_backward(const RunDesc& R, const FxLineSmem
     if (j != jq) fx_put_subsets(S.buf, base, NN, jq, uq, v, R.fx_twZ);
   }
   __syncthreads();
-  fx_line_ffts<true>(S.buf, pairs, S.PS, R.fx_planQ, S.tw, S.zero);
+  fx_line_ffts<true>(S, pairs, R.fx_planQ);
   __syncthreads();
 }
 
@@ -329,16 +345,17 @@ __global__ void __launch_bounds__(kFxLineThreads) phys_z_forward_fx_kernel(const
   }
   __syncthreads();
   for (int l = threadIdx.x >> 5; l < pairs; l += kFxLineThreads / 32) {
-    const int e = fx_line_exponent(S.buf, l * S.PS, Z, 0);
-    if ((threadIdx.x & 31) == 0) S.e[l] = e;
+    int g;
+    const int e = fx_line_exponent(S.buf, l * S.PS, Z, 0, R.fx_planQ, false, g);
+    if ((threadIdx.x & 31) == 0) fx_line_scale(S, l, e, g);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < pairs * Z; i += kFxLineThreads) {
     const int l = fZ.div(i), at = l * S.PS + i - l * Z;
-    S.buf[fx_at(at)] = fx_from_double2(fx_raw(S.buf, at), S.e[l]);
+    S.buf[fx_at(at)] = fx_from_double2(fx_raw(S.buf, at), S.e[l] + fx_fine_bits(S.fine[3 * l]));
   }
   __syncthreads();
-  fx_line_ffts<false>(S.buf, pairs, S.PS, R.fx_planQ, S.tw, S.zero);
+  fx_line_ffts<false>(S, pairs, R.fx_planQ);
   __syncthreads();
   double2* __restrict__ W = reinterpret_cast<double2*>(R.T);
   const double sc = R.scale;

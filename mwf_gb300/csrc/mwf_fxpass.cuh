@@ -14,9 +14,10 @@
 //
 // What is stored between the passes (RunDesc, fx_*):
 //   T     longlong2[2KK][X][NN], column (f, n) scaled by 2^colE[f][n]
-//   rowP  float[2KK][X][nblk] and blkE int[2KK][nblk]: for row (f, x) and column block b, the sum of
-//         |re| + |im| over the block is rowP 2^(32 - blkE), the last entry being column n = 0, which
-//         block 0 leaves out; the z pass scales its lines by the sums
+//   rowP  unsigned[2KK][X][nblk] and blkE int[2KK][nblk]: for row (f, x) and column block b, the sum
+//         and the largest of |re| + |im| over the block as two bfloat16 (rounded up; sum in the high
+//         half) times 2^(32 - blkE), the last entry being column n = 0, which block 0 leaves out;
+//         the z pass scales its lines by them
 //   NLT   longlong2[3][KK][X][NN], row (s, f, x) scaled by 2^rowE[s][f][x]; minE[f] = the smallest
 //         of field f, the scale at which the x inverse adds the partials
 // Values are unnormalised; the 1/(3MM 3NN) of the forward transform is applied in the update.
@@ -27,8 +28,6 @@
 
 namespace mwf {
 
-// The e with 2^(e-1) <= v < 2^e, for a normal v > 0.
-__device__ __forceinline__ int fx_bits_above(float v) { return (int)((__float_as_uint(v) >> 23) & 255) - 126; }
 // 2^k for k <= 0, zero below the float range.
 __device__ __forceinline__ float fx_pow2(int k) { return k < -126 ? 0.f : __int_as_float((k + 127) << 23); }
 // Number of bits of values whose largest high word is hi (at least 32).
@@ -38,6 +37,14 @@ __device__ __forceinline__ float fx_warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
+}
+
+__device__ __forceinline__ float fx_warp_max(float v) {
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));   // v >= 0
+}
+// Two floats >= 0 as bfloat16, rounded up.
+__device__ __forceinline__ unsigned fx_pack2(float hi, float lo) {
+  return ((__float_as_uint(hi) + 0xffffu) & 0xffff0000u) | ((__float_as_uint(lo) + 0xffffu) >> 16);
 }
 
 // A sum of moduli S 2^E; S = 0: nothing but zeros.
@@ -55,15 +62,15 @@ __device__ __forceinline__ FxNorm fx_norm_add(FxNorm a, FxNorm b) {
 // x forward
 // ---------------------------------------------------------------------------------------
 
-// Sum over the M slots of a row of |re| + |im| times |m|^p0 (S0) and |m|^p1 (S1), each as a float times
-// 2^E; nan: a NaN or an infinity in the row.  One warp, one pass, eight loads of a lane in flight; each
+// Sum and largest over the M slots of a row of |re| + |im| times |m|^p0 (S0, T0) and |m|^p1 (S1, T1),
+// each as a float times 2^E; nan: a NaN or an infinity in the row.  One warp, one pass, eight loads of a lane in flight; each
 // lane keeps its sums relative to its largest exponent so far.  The high words are enough (truncated
 // by less than 2^-20, which the caller covers); zeros and subnormals count as zeros.
 __device__ __forceinline__ void fx_row_moments(const double2* __restrict__ row, int M, int MM, int p0, int p1,
-                                               float& S0, float& S1, int& E, int& nan) {
+                                               float& S0, float& S1, float& T0, float& T1, int& E, int& nan) {
   const int lane = threadIdx.x & 31;
   int top = 0;
-  float a = 0.f, b = 0.f;
+  float a = 0.f, b = 0.f, ta = 0.f, tb = 0.f;
   for (int m0 = 0; m0 < M; m0 += 256) {
     int hx[8], hy[8], t = 0;
 #pragma unroll
@@ -79,6 +86,8 @@ __device__ __forceinline__ void fx_row_moments(const double2* __restrict__ row, 
       const float k = fx_pow2(max(top - t, -127));
       a *= k;
       b *= k;
+      ta *= k;
+      tb *= k;
       top = t;
     }
     auto part = [&](int h) {                          // relative to the largest exponent
@@ -90,14 +99,20 @@ __device__ __forceinline__ void fx_row_moments(const double2* __restrict__ row, 
       const int ms = m0 + 32 * i + lane;
       const float v = part(hx[i]) + part(hy[i]);
       const float m = (float)(ms < MM ? ms : M - ms);
-      a += v * (p0 == 0 ? 1.f : p0 == 1 ? m : p0 == 2 ? m * m : m * m * m);
-      b += v * (p1 == 0 ? 1.f : p1 == 1 ? m : m * m);
+      const float va = v * (p0 == 0 ? 1.f : p0 == 1 ? m : p0 == 2 ? m * m : m * m * m);
+      const float vb = v * (p1 == 0 ? 1.f : p1 == 1 ? m : m * m);
+      a += va;
+      b += vb;
+      ta = fmaxf(ta, va);
+      tb = fmaxf(tb, vb);
     }
   }
   const int all = __reduce_max_sync(0xffffffffu, top);
   const float k = fx_pow2(max(top - all, -127));
   S0 = fx_warp_sum(a * k);
   S1 = fx_warp_sum(b * k);
+  T0 = fx_warp_max(ta * k);
+  T1 = fx_warp_max(tb * k);
   E = all - 1023;
   nan = all >= 0x7ff;
 }
@@ -126,22 +141,25 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDes
 
   // Column scales from bounds on the columns' L1 norms: u = i(-n1 psi + k1 m1 phi), w = i(m1 psi +
   // k1 n1 phi), v = (m1^2 + n1^2) phi and the same times m1 (m1 = alpha m, n1 = gamma n)
-  __shared__ float mom[2][2][kFxMaxCols];             // [psi, phi][sum]
+  __shared__ float mom[2][4][kFxMaxCols];             // [psi, phi][sums, largest]
+  __shared__ int fine[3 * kFxMaxCols];                // finer scale of the first stages, by subset line
   __shared__ int momE[2][kFxMaxCols], momN[2][kFxMaxCols];
   {
     const int dd = deriv ? 1 : 0;
     for (int i = warp; i < 2 * nb; i += NT / 32) {
       const int l = i >> 1, phi = i & 1;
-      float s0 = 0.f, s1 = 0.f;
+      float s0 = 0.f, s1 = 0.f, t0 = 0.f, t1 = 0.f;
       int E = 0, bad = 0;
       // psi: u needs m^d, w m^(d+1); phi: u m^(d+1), w m^d, v m^(d+2) and m^d
       if (phi ? k >= 1 : comp != 1) {
         const int p0 = phi ? (comp == 0 ? dd + 1 : comp == 2 ? dd : dd + 2) : (comp == 0 ? dd : dd + 1);
-        fx_row_moments(c + ((size_t)(n0 + l) * K + (phi ? k + K0 - 1 : k)) * M, M, MM, p0, dd, s0, s1, E, bad);
+        fx_row_moments(c + ((size_t)(n0 + l) * K + (phi ? k + K0 - 1 : k)) * M, M, MM, p0, dd, s0, s1, t0, t1, E, bad);
       }
       if (lane == 0) {
         mom[phi][0][l] = s0;
         mom[phi][1][l] = s1;
+        mom[phi][2][l] = t0;
+        mom[phi][3][l] = t1;
         momE[phi][l] = E;
         momN[phi][l] = bad;
       }
@@ -151,17 +169,26 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDes
   if (threadIdx.x < nb) {
     const int l = threadIdx.x, n = n0 + l;
     const double a1 = fabs(R.alpha), n1 = R.gamma * n, g1 = fabs(n1), kb = kbeta<double>(k), k1 = fabs(kb);
-    const double s0 = scalbn((double)mom[0][0][l], momE[0][l]);
-    const double t0 = scalbn((double)mom[1][0][l], momE[1][l]), t1 = scalbn((double)mom[1][1][l], momE[1][l]);
-    double L = comp == 0 ? g1 * s0 + k1 * a1 * t0 : comp == 2 ? a1 * s0 + k1 * g1 * t0 : a1 * a1 * t0 + g1 * g1 * t1;
-    if (n == 0 && !deriv && comp != 1) {              // the mean flows u_k = psi_k, w_k = phi_k, and the base flow
-      const double2 v = c[(size_t)(comp == 0 || k == 0 ? k : k + K0 - 1) * M];
-      L += fabs(v.x) + fabs(v.y) + (k == 1 ? 1.0 : 0.0);
-    }
-    if (deriv) L *= a1;
-    L *= 1.0001;
+    auto bound = [&](int i) {                         // i = 0: of the sum, 2: of the largest
+      const double s0 = scalbn((double)mom[0][i][l], momE[0][l]);
+      const double t0 = scalbn((double)mom[1][i][l], momE[1][l]), t1 = scalbn((double)mom[1][i + 1][l], momE[1][l]);
+      double L = comp == 0 ? g1 * s0 + k1 * a1 * t0 : comp == 2 ? a1 * s0 + k1 * g1 * t0 : a1 * a1 * t0 + g1 * g1 * t1;
+      if (n == 0 && !deriv && comp != 1) {            // the mean flows u_k = psi_k, w_k = phi_k, and the base flow
+        const double2 v = c[(size_t)(comp == 0 || k == 0 ? k : k + K0 - 1) * M];
+        L += fabs(v.x) + fabs(v.y) + (k == 1 ? 1.0 : 0.0);
+      }
+      if (deriv) L *= a1;
+      return L * 1.0001;
+    };
+    const double L = bound(0);
     const int ex = (int)(fx_bits(L) >> 52) & 0x7ff;
     const int e = momN[0][l] || momN[1][l] || ex == 0x7ff ? kFxNan : (L == 0.0 ? kFxZero : 61 - (ex - 1022));
+    // a value of the subset lines is the sum of two coefficients
+    const double most = bound(2);
+    const int mx = (int)(fx_bits(most) >> 52) & 0x7ff;
+    const int fg = mx == 0 || mx == 0x7ff ? 0
+        : fx_fine(R.fx_planM, true, (float)fx_value((fx_bits(most) & 0xfffffffffffffull) | (1024ull << 52)), mx - 1023, e);
+    for (int s = 0; s < 3; ++s) fine[3 * l + s] = fg;
     colE[l] = e;
     R.fx_colE[(size_t)f * NN + n] = e;
     const double sg = deriv ? -1.0 : 1.0;
@@ -188,7 +215,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDes
   for (int e = threadIdx.x; e < nb * MM; e += NT) {
     const int l = fMM.div(e);
     const int j = e - l * MM;
-    const int ce = colE[l];
+    const int ce = colE[l] + fx_fine_bits(fine[3 * l]);
     const FxFactor na = colN[0][l], nbf = colN[1][l];
     const double2* __restrict__ col = c + (size_t)(n0 + l) * K * M;
     const int jn = j == 0 ? 0 : MM - j;               // -m of the negative wavenumber
@@ -230,8 +257,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDes
     constexpr FxConst s3 = fx_const(kFxSqrt34);
     const i64 rx = fx_mulc(b.x, s3), ry = fx_mulc(b.y, s3);
     longlong2 h, p, q;
-    h.x = a.x - (b.x >> 1);
-    h.y = a.y - (b.y >> 1);
+    h.x = a.x - fx_half(b.x);
+    h.y = a.y - fx_half(b.y);
     p.x = h.x + ry; p.y = h.y - rx;                   // a + e^{-2 pi i/3} b
     q.x = h.x - ry; q.y = h.y + rx;                   // a + e^{-4 pi i/3} b
     buf[fx_at(base + MM)] = fx_cmul<true>(p, xm[j]);
@@ -243,7 +270,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDes
     const int lines = 3 * nb;
     const int G = max(1, min(lines, 256 / MM));
     for (int t = warp * G; t < lines; t += (NT / 32) * G)
-      fx_fft<true>(buf, t * MM, min(G, lines - t), R.fx_planM, tw, nullptr);
+      fx_fft<true>(buf, t * MM, min(G, lines - t), R.fx_planM, tw, nullptr, fine + t, 1);
   }
   __syncthreads();
 
@@ -264,7 +291,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDes
   const int er = apart ? ce : eb;
   const float wgt = (ce >= kFxZero || er <= kFxNan) ? 0.f : fx_pow2(max(er - ce, -127));
   longlong2* __restrict__ T = reinterpret_cast<longlong2*>(R.T) + (size_t)f * X * NN;
-  float* __restrict__ P = R.fx_rowP + (size_t)f * X * nblk;
+  unsigned* __restrict__ P = R.fx_rowP + (size_t)f * X * nblk;
 #pragma unroll 4
   for (int e0 = 0; e0 < (X << lw); e0 += NT) {
     const int sp = (e0 + threadIdx.x) >> lw;          // s MM + position
@@ -278,10 +305,14 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDes
       T[(size_t)x * NN + n0 + l] = v;
       part = ((float)fx_abs_hi(v.x) + (float)fx_abs_hi(v.y) + 2.f) * wgt;
     }
-    if (on && apart) P[(size_t)x * nblk + nblk - 1] = part;
+    if (on && apart) P[(size_t)x * nblk + nblk - 1] = fx_pack2(part, part);
     if (apart) part = 0.f;
-    for (int o = 1; o < nbw; o <<= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if (on && l == 0) P[(size_t)x * nblk + blk] = part;
+    float top = part;
+    for (int o = 1; o < nbw; o <<= 1) {
+      part += __shfl_xor_sync(0xffffffffu, part, o);
+      top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    }
+    if (on && l == 0) P[(size_t)x * nblk + blk] = fx_pack2(part, top);
   }
 }
 
@@ -291,55 +322,65 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDes
 
 constexpr int kFxFlight = 5;   // 128 blocks and the column n = 0 are 129 entries for 32 lanes
 
-// Sums of moduli of row (f, x), and of the moduli times the z wavenumber index (an upper bound: the
-// block's largest), over the W lanes (a power of two) of a warp's segment; lane = place in it.
-__device__ __forceinline__ void fx_row_norm(const RunDesc& R, int f, int x, int W, int lane, float& S, float& Z, int& E, int& bad) {
+// Sums (S) and largest (m) of the moduli of row (f, x), and of the moduli times the z wavenumber index
+// (Z, mz: upper bounds with the block's largest index), times 2^E, over the W lanes (a power of two)
+// of a warp's segment; lane = place in it.
+struct FxRow { float S, Z, m, mz; int E, bad; };
+__device__ __forceinline__ FxRow fx_row_norm(const RunDesc& R, int f, int x, int W, int lane) {
   const int nblk = R.fx_nblk;
-  const float* __restrict__ P = R.fx_rowP + ((size_t)f * R.X + x) * nblk;
+  const unsigned* __restrict__ P = R.fx_rowP + ((size_t)f * R.X + x) * nblk;
   const int* __restrict__ EB = R.fx_blkE + (size_t)f * nblk;
   int ref = -(1 << 29);
-  bad = 0;
-  float s = 0.f, z = 0.f;
+  FxRow o{0.f, 0.f, 0.f, 0.f, 0, 0};
   for (int b0 = 0; b0 < nblk; b0 += kFxFlight * W) {  // kFxFlight blocks of a lane in flight
-    float p[kFxFlight];
+    unsigned p[kFxFlight];
     int e[kFxFlight], top = -(1 << 29);
 #pragma unroll
     for (int i = 0; i < kFxFlight; ++i) {
       const int b = b0 + i * W + lane;
-      p[i] = b < nblk ? P[b] : 0.f;
+      p[i] = b < nblk ? P[b] : 0u;
       e[i] = b < nblk ? EB[b] : kFxZero;
     }
 #pragma unroll
     for (int i = 0; i < kFxFlight; ++i) {
-      bad |= e[i] <= kFxNan;
-      if (p[i] > 0.f) top = max(top, -e[i]);
+      o.bad |= e[i] <= kFxNan;
+      if (p[i]) top = max(top, -e[i]);
     }
-    for (int o = 1; o < W; o <<= 1) {
-      top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
-      bad |= __shfl_xor_sync(0xffffffffu, bad, o);
+    for (int d = 1; d < W; d <<= 1) {
+      top = max(top, __shfl_xor_sync(0xffffffffu, top, d));
+      o.bad |= __shfl_xor_sync(0xffffffffu, o.bad, d);
     }
     if (top > ref) {                                  // the same for the whole segment
       const float k = fx_pow2(max(ref - top, -127));
-      s *= k;
-      z *= k;
+      o.S *= k;
+      o.Z *= k;
+      o.m *= k;
+      o.mz *= k;
       ref = top;
     }
 #pragma unroll
     for (int i = 0; i < kFxFlight; ++i)
-      if (p[i] > 0.f) {
-        const float v = p[i] * fx_pow2(max(-e[i] - ref, -127));
-        s += v;
+      if (p[i]) {
+        const float k = fx_pow2(max(-e[i] - ref, -127));
+        const float v = __uint_as_float(p[i] & 0xffff0000u) * k, t = __uint_as_float(p[i] << 16) * k;
+        o.S += v;
+        o.m = fmaxf(o.m, t);
         const int b = b0 + i * W + lane;
-        if (b < nblk - 1) z += v * (float)((b + 1) * R.fx_nb - 1);    // the last entry is n = 0
+        if (b < nblk - 1) {                           // the last entry is n = 0
+          const float n = (float)((b + 1) * R.fx_nb - 1);
+          o.Z += v * n;
+          o.mz = fmaxf(o.mz, t * n);
+        }
       }
   }
-  for (int o = 1; o < W; o <<= 1) {
-    s += __shfl_xor_sync(0xffffffffu, s, o);
-    z += __shfl_xor_sync(0xffffffffu, z, o);
+  for (int d = 1; d < W; d <<= 1) {
+    o.S += __shfl_xor_sync(0xffffffffu, o.S, d);
+    o.Z += __shfl_xor_sync(0xffffffffu, o.Z, d);
+    o.m = fmaxf(o.m, __shfl_xor_sync(0xffffffffu, o.m, d));
+    o.mz = fmaxf(o.mz, __shfl_xor_sync(0xffffffffu, o.mz, d));
   }
-  S = s;
-  Z = z;
-  E = ref + 32;
+  o.E = ref + 32;
+  return o;
 }
 
 // Groups of values with one scale in the coupling: the velocity components, and their x and z
@@ -365,7 +406,8 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) z_fx_kernel(const RunDe
   longlong2* buf = reinterpret_cast<longlong2*>(smem_raw);
   int4* tw = reinterpret_cast<int4*>(buf + (size_t)NTR * TS);    // [Q] stage twiddles
   int* eL = reinterpret_cast<int*>(tw + Q);                      // [NTR L] line exponents
-  int* mx = eL + NTR * L;                                        // [2 NTR L] largest high words (re, im), then shifts
+  int* mx = eL + NTR * L;                                        // [2 NTR L] the lines' finer first scale, then largest
+                                                                 // high words (re, im), then shifts, then the finer scale
   int* ge = mx + 2 * NTR * L;                                    // [kFxGroups L] group exponents
   int* eo = ge + kFxGroups * L;                                  // [3 L] exponents of the products
   int* sh = eo + 3 * L;                                          // [NPAIR L] forward line shifts
@@ -390,34 +432,34 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) z_fx_kernel(const RunDe
 
   // ---- line scales: the rows' norms, a warp segment each (in the lines' space, not yet in use) ----
   {
-    float* nS = reinterpret_cast<float*>(smem_raw);              // [2KK L]
-    float* nZ = nS + 2 * KK * L;
-    int* nE = reinterpret_cast<int*>(nZ + 2 * KK * L);
+    FxRow* rows = reinterpret_cast<FxRow*>(smem_raw);            // [2KK L]
     int W = 1;
     while (W < 32 && kFxFlight * W < R.fx_nblk) W <<= 1;
     const int sub = lane / W, seg = 32 / W;
     for (int i0 = warp * seg; i0 < 2 * KK * L; i0 += NW * seg) {
       const int i = min(i0 + sub, 2 * KK * L - 1);
       const int f = i / L, l = i - f * L;
-      float a, z;
-      int e, nan;
-      fx_row_norm(R, f, x0 + l, W, lane & (W - 1), a, z, e, nan);
+      FxRow v = fx_row_norm(R, f, x0 + l, W, lane & (W - 1));
       if ((lane & (W - 1)) == 0) {
-        nS[i] = a;
-        nZ[i] = z * fabsf(R.gamma_f);
-        nE[i] = e;
-        if (nan) bad[l] = 1;
+        v.Z *= fabsf(R.gamma_f);
+        v.mz *= fabsf(R.gamma_f);
+        rows[i] = v;
+        if (v.bad) bad[l] = 1;
       }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < NTR * L; i += NT) {
       const int t = i / L, l = i - t * L;
-      const int a = (t < NPAIR ? 2 * t : KK + t - NPAIR) * L + l;
-      const int b = (t < NPAIR ? 2 * t + 1 : t - NPAIR) * L + l;
       const bool two = t >= NPAIR || 2 * t + 1 < KK;
-      const FxNorm v = fx_norm_add(FxNorm{nS[a], nE[a]}, FxNorm{two ? (t < NPAIR ? nS[b] : nZ[b]) : 0.f, two ? nE[b] : 0});
-      // the Hermitian extension doubles every coefficient: the line's norm is below 2 S 2^E
-      eL[i] = v.S > 0.f ? 61 - (v.E + 1 + fx_bits_above(v.S * 1.001f)) : kFxZero;
+      const FxRow a = rows[(t < NPAIR ? 2 * t : KK + t - NPAIR) * L + l];
+      const FxRow b = rows[(t < NPAIR ? 2 * t + (two ? 1 : 0) : t - NPAIR) * L + l];
+      const FxNorm v = fx_norm_add(FxNorm{a.S, a.E}, FxNorm{two ? (t < NPAIR ? b.S : b.Z) : 0.f, b.E});
+      const FxNorm m = fx_norm_add(FxNorm{a.m, a.E}, FxNorm{two ? (t < NPAIR ? b.m : b.mz) : 0.f, b.E});
+      // the Hermitian extension doubles every coefficient: the line's norm is below 2 S 2^E, and a
+      // value of a subset line is the sum of two of its coefficients
+      const int e = v.S > 0.f ? 61 - (v.E + 1 + fx_bits_above(v.S * 1.001f)) : kFxZero;
+      eL[i] = e;
+      mx[2 * i] = fx_fine(R.fx_planQ, true, m.S, m.E + 1, e);
     }
   }
   __syncthreads();
@@ -435,8 +477,8 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) z_fx_kernel(const RunDe
   auto times_eps = [&](longlong2 a) {                 // eps a for this subset (s = 1, 2)
     const i64 rx = fx_mulc(a.x, s3), ry = fx_mulc(a.y, s3);
     longlong2 r;
-    r.x = s == 1 ? -(a.x >> 1) + ry : -(a.x >> 1) - ry;
-    r.y = s == 1 ? -(a.y >> 1) - rx : -(a.y >> 1) + rx;
+    r.x = s == 1 ? -fx_half(a.x) + ry : -fx_half(a.x) - ry;
+    r.y = s == 1 ? -fx_half(a.y) - rx : -fx_half(a.y) + rx;
     return r;
   };
   const int G = min(L, R.fx_group);
@@ -474,7 +516,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) z_fx_kernel(const RunDe
       if (idx + 32 < total) nx = load(idx + 32);      // the next slot's rows while this one is formed
       const int l = fSl.div(idx), sl = idx - l * slots;
       const int n = sl ? sl : (even ? Q / 2 : 0), nq = sl ? Q - sl : n;
-      const int e = eL[t * L + l0 + l], base = t * TS + (l0 + l) * Q;
+      const int e = eL[t * L + l0 + l] + fx_fine_bits(mx[2 * (t * L + l0 + l)]), base = t * TS + (l0 + l) * Q;
       const longlong2 Pa = fx_shift2(v.Pa, e - v.ea);
       longlong2 Ra = fx_shift2(v.Ra, e - v.ra), Pb, Rb;
       if (der) {
@@ -522,7 +564,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) z_fx_kernel(const RunDe
       if (sl) buf[fx_at(base + nq)] = Hq;
     }
     __syncwarp();
-    fx_fft<true>(buf, t * TS + l0 * Q, nl, R.fx_planQ, tw, mx + 2 * (t * L + l0));
+    fx_fft<true>(buf, t * TS + l0 * Q, nl, R.fx_planQ, tw, mx + 2 * (t * L + l0), mx + 2 * (t * L + l0), 2);
   }
   __syncthreads();
 
@@ -630,17 +672,26 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) z_fx_kernel(const RunDe
     const int first = (NPAIR + t) * TS + l0 * Q;
     // scale each line so that its norm just fits (from the high words, rounded up)
     for (int l = lane / WQ; l - lane / WQ < nl; l += 32 / WQ) {
-      float a = 0.f;
+      float a = 0.f, m = 0.f;
       if (l < nl)
         for (int n = lane & (WQ - 1); n < Q; n += WQ) {
           const longlong2 v = buf[fx_at(first + l * Q + n)];
-          a += (float)fx_abs_hi(v.x) + (float)fx_abs_hi(v.y) + 2.f;
+          const float b = (float)fx_abs_hi(v.x) + (float)fx_abs_hi(v.y) + 2.f;
+          a += b;
+          m = fmaxf(m, b);
         }
-      for (int o = 1; o < WQ; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-      if (l < nl && (lane & (WQ - 1)) == 0) sh[t * L + l0 + l] = 61 - 32 - fx_bits_above(a * 1.001f);
+      for (int o = 1; o < WQ; o <<= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      }
+      if (l < nl && (lane & (WQ - 1)) == 0) {
+        const int i = t * L + l0 + l, e = 61 - 32 - fx_bits_above(a * 1.001f), g = fx_fine(R.fx_planQ, false, m, 32, e);
+        sh[i] = e + fx_fine_bits(g);
+        mx[2 * i] = g;
+      }
     }
     __syncwarp();
-    fx_fft<false>(buf, first, nl, R.fx_planQ, tw, sh + t * L + l0);
+    fx_fft<false>(buf, first, nl, R.fx_planQ, tw, sh + t * L + l0, mx + 2 * (t * L + l0), 2);
     const int ka = 2 * t;
     const bool two = ka + 1 < KK;
     longlong2* __restrict__ oa = NLT + (size_t)ka * fstride + (size_t)(x0 + l0) * Q;
@@ -682,7 +733,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) z_fx_kernel(const RunDe
       const int l = l0 + (j >> 1), f = ka + (j & 1);
       if (f >= KK) continue;
       // the coupling is 2 nl, the split another factor of two
-      int e = eo[fx_comp<K0>(f) * L + l] + sh[t * L + l] + 2;
+      int e = eo[fx_comp<K0>(f) * L + l] + sh[t * L + l] - fx_fine_bits(mx[2 * (t * L + l)]) + 2;
       if (bad[l]) e = kFxNan;
       R.fx_rowE[((size_t)s * KK + f) * X + x0 + l] = e;
       atomicMin(&R.fx_minE[f], e);
@@ -699,6 +750,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_inverse_fx_kernel(const RunDes
   longlong2* buf = reinterpret_cast<longlong2*>(smem_raw);       // line (comp, l, s) at ((comp nb + l) 3 + s) MM
   __shared__ u64 norm[9 * kFxMaxCols];
   __shared__ int sh[9 * kFxMaxCols];
+  __shared__ int fine[9 * kFxMaxCols];                // largest values' bits, then the finer scale of the first stages
   __shared__ double colw[3][kFxMaxCols];              // gamma n, (-1)^k k b gamma n and (gamma n)^2, times the scale
   const WorkItem wi = items[blockIdx.x];
   const RunDesc& R = runs[wi.run];
@@ -755,13 +807,19 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_inverse_fx_kernel(const RunDes
   }
   __syncthreads();
   for (int i = warp; i < 9 * nb; i += NW) {
-    u64 a = 0;
+    u64 a = 0, m = 0;
     for (int p = lane; p < MM; p += 32) {
       const longlong2 v = buf[fx_at(i * MM + p)];
-      a += ((u64)(v.x ^ (v.x >> 63)) >> 13) + ((u64)(v.y ^ (v.y >> 63)) >> 13) + 2;
+      const u64 b = ((u64)(v.x ^ (v.x >> 63)) >> 13) + ((u64)(v.y ^ (v.y >> 63)) >> 13) + 2;
+      a += b;
+      m |= b;                                         // an upper bound by less than a factor of two
     }
     for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if (lane == 0) norm[i] = a;
+    const unsigned hi = __reduce_or_sync(0xffffffffu, (unsigned)(m >> 32)), lo = __reduce_or_sync(0xffffffffu, (unsigned)m);
+    if (lane == 0) {
+      norm[i] = a;
+      fine[i] = hi ? 64 - __clz((int)hi) : 32 - __clz((int)lo);
+    }
   }
   __syncthreads();
   // the three subsets of a line share a scale: their combined norm is below 2^61
@@ -770,11 +828,20 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_inverse_fx_kernel(const RunDes
     sh[i] = 61 - 13 - (64 - __clzll((i64)(norm[b] + norm[b + 1] + norm[b + 2])));
   }
   __syncthreads();
+  for (int i = threadIdx.x; i < 3 * nb; i += NT) {
+    const int most = max(fine[3 * i], max(fine[3 * i + 1], fine[3 * i + 2]));
+    const int g = fx_fine(R.fx_planM, false, 1.f, most + 13, sh[3 * i]);
+    for (int s = 0; s < 3; ++s) {
+      fine[3 * i + s] = g;
+      sh[3 * i + s] += fx_fine_bits(g);
+    }
+  }
+  __syncthreads();
   {
     const int lines = 9 * nb;
     const int G = max(1, min(lines, 256 / MM));
     for (int t = warp * G; t < lines; t += NW * G)
-      fx_fft<false>(buf, t * MM, min(G, lines - t), R.fx_planM, tw, sh + t);
+      fx_fft<false>(buf, t * MM, min(G, lines - t), R.fx_planM, tw, sh + t, fine + t, 1);
   }
   __syncthreads();
 
@@ -796,7 +863,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_inverse_fx_kernel(const RunDes
     const int ms = o - l * M;
     const int n = n0 + l;
     const double n1 = colw[0][l], kn = colw[1][l], n2 = colw[2][l];
-    const int eu = ref[0] + sh[l * 3], ev = ref[1] + sh[(nb + l) * 3], ew = ref[2] + sh[(2 * nb + l) * 3];
+    auto scale = [&](int c) { return ref[c] + sh[(c * nb + l) * 3] - fx_fine_bits(fine[(c * nb + l) * 3]); };
+    const int eu = scale(0), ev = scale(1), ew = scale(2);
     const int m = signed_m(ms, MM, M);
     const size_t i0 = ((size_t)n * K + k) * M + ms;
     const size_t i1 = i0 + (size_t)(K0 - 1) * M;

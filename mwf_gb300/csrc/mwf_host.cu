@@ -527,7 +527,7 @@ bool plan_run(RunHost& r, const char*& why) {
   r.fx = d.precision == MWF_FP64 && !d.xf_cols && !d.xi_cols && !d.z_lines && !d.x_radix && !d.z_radix &&
          fx_z_smem(d.K0, d.NN, 1) <= zb_smem_budget(1);
   if (r.fx) {
-    const size_t half = zb_smem_budget(2) - 1024, whole = zb_smem_budget(1) - 1024;   // the x passes' static arrays
+    const size_t half = zb_smem_budget(2) - 1408, whole = zb_smem_budget(1) - 1408;   // the x passes' static arrays
     const int slots = 2 * 152;                // CTAs of 256 threads that the chip holds
     auto items = [&](int nb, int per) { return (d.NN + nb - 1) / nb * per; };
     // widest column blocks (whole sectors of T) that still give every slot an item
@@ -1383,7 +1383,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
       D.fx_blkE = reinterpret_cast<int*>(h->arena + fo.blkE);
       D.fx_rowE = reinterpret_cast<int*>(h->arena + fo.rowE);
       D.fx_minE = reinterpret_cast<int*>(h->arena + fo.minE);
-      D.fx_rowP = reinterpret_cast<float*>(h->arena + fo.rowP);
+      D.fx_rowP = reinterpret_cast<unsigned*>(h->arena + fo.rowP);
     }
     const int one = 1;
     ck(cudaMemcpy(h->arena + r.off_nst, &one, sizeof(int), cudaMemcpyHostToDevice), "nst init");

@@ -115,7 +115,7 @@ cudaError_t launch_x_inverse_fx(int nt, const RunDesc* runs, const WorkItem* ite
 // half an SM holds, and fewer while the grid leaves some of the chip's 304 half-SM slots empty.
 __host__ __device__ constexpr int fx_line_stride(int N) { return (3 * N) | 1; }
 constexpr size_t fx_line_smem_bytes(int N, int lines) {
-  return 16 * ((((size_t)lines * fx_line_stride(N) + 7) & ~(size_t)7) + N) + 4 * ((size_t)lines + 3);
+  return 16 * ((((size_t)lines * fx_line_stride(N) + 7) & ~(size_t)7) + N) + 4 * ((size_t)4 * lines + 3);
 }
 // sp = nullptr: the fields of the run's state
 cudaError_t launch_spec_x_backward_fx(const RunDesc* runs, int run, int MM, int KK, int NN, const void* sp, cudaStream_t st);
