@@ -21,6 +21,14 @@ template <typename C> __device__ __forceinline__ C rot90(C a, bool inv) {
   return r;
 }
 
+// a + rot90(b), a - rot90(b): parts of b change places, which two scalar additions do for nothing
+template <typename C> __device__ __forceinline__ C cadd_rot(C a, C b, bool inv) {
+  C r;
+  if (inv) { r.x = a.x - b.y; r.y = a.y + b.x; } else { r.x = a.x + b.y; r.y = a.y - b.x; }
+  return r;
+}
+template <typename C> __device__ __forceinline__ C csub_rot(C a, C b, bool inv) { return cadd_rot(a, b, !inv); }
+
 template <typename T, typename C> __device__ __forceinline__ void dft2(C* v) {
   C a = v[0];
   v[0] = cadd(a, v[1]);
@@ -52,11 +60,11 @@ template <typename T, typename C> __device__ __forceinline__ void dft4(C* v, boo
   C t0 = cadd(v[0], v[2]);
   C t1 = csub(v[0], v[2]);
   C t2 = cadd(v[1], v[3]);
-  C t3 = rot90(csub(v[1], v[3]), inv);
+  C t3 = csub(v[1], v[3]);
   v[0] = cadd(t0, t2);
   v[2] = csub(t0, t2);
-  v[1] = cadd(t1, t3);
-  v[3] = csub(t1, t3);
+  v[1] = cadd_rot(t1, t3, inv);
+  v[3] = csub_rot(t1, t3, inv);
 }
 
 // multiply by exp(-+ i pi/4) = (1 -+ i)/sqrt(2)
@@ -74,12 +82,13 @@ template <typename T, typename C> __device__ __forceinline__ void dft8(C* v, boo
   dft4<T>(e, inv);
   dft4<T>(o, inv);
   o[1] = w8<T>(o[1], inv);
-  o[2] = rot90(o[2], inv);
-  o[3] = rot90(w8<T>(o[3], inv), inv);
+  o[3] = w8<T>(o[3], inv);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
+  for (int k = 0; k < 2; ++k) {
     v[k] = cadd(e[k], o[k]);
     v[k + 4] = csub(e[k], o[k]);
+    v[k + 2] = cadd_rot(e[k + 2], o[k + 2], inv);
+    v[k + 6] = csub_rot(e[k + 2], o[k + 2], inv);
   }
 }
 
