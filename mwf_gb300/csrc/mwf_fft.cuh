@@ -39,21 +39,23 @@ template <typename T, typename C> __device__ __forceinline__ void dft3(C* v, boo
   // y1,y2 = a - (b+c)/2 +- i s (b - c),  s = -sqrt(3)/2 forward, +sqrt(3)/2 inverse
   const T s = inv ? T(0.86602540378443864676) : T(-0.86602540378443864676);
   C t1 = cadd(v[1], v[2]);
-  C t2 = csub(v[1], v[2]);
-  C m;
   if constexpr (sizeof(T) == 4) {         // FP32: explicit rounding (see cmul<float2>)
-    m.x = __fmaf_rn(-0.5f, t1.x, v[0].x);
-    m.y = __fmaf_rn(-0.5f, t1.y, v[0].y);
+    const C m = __ffma2_rn(t1, make_float2(-0.5f, -0.5f), v[0]);
+    const C q = make_float2(v[2].y - v[1].y, v[1].x - v[2].x);      // i (b - c)
+    v[0] = cadd(v[0], t1);
+    v[1] = __ffma2_rn(q, make_float2(s, s), m);
+    v[2] = __ffma2_rn(q, make_float2(-s, -s), m);
   } else {
+    const C t2 = csub(v[1], v[2]);
+    C m, j;
     m.x = v[0].x - T(0.5) * t1.x;
     m.y = v[0].y - T(0.5) * t1.y;
+    j.x = -s * t2.y;
+    j.y = s * t2.x;
+    v[0] = cadd(v[0], t1);
+    v[1] = cadd(m, j);
+    v[2] = csub(m, j);
   }
-  C j;
-  j.x = -s * t2.y;
-  j.y = s * t2.x;
-  v[0] = cadd(v[0], t1);
-  v[1] = cadd(m, j);
-  v[2] = csub(m, j);
 }
 
 template <typename T, typename C> __device__ __forceinline__ void dft4(C* v, bool inv) {
@@ -81,6 +83,21 @@ template <typename T, typename C> __device__ __forceinline__ void dft8(C* v, boo
   C o[4] = {v[1], v[3], v[5], v[7]};
   dft4<T>(e, inv);
   dft4<T>(o, inv);
+  if constexpr (sizeof(T) == 4) {         // FP32: the factor sqrt(1/2) of odd k in the last addition
+    constexpr float h = 0.70710678118654752440f;
+    const C a = o[1], b = o[3];
+    const C p = inv ? make_float2(a.x - a.y, a.x + a.y) : make_float2(a.x + a.y, a.y - a.x);
+    const C q = inv ? make_float2(-b.x - b.y, b.x - b.y) : make_float2(b.y - b.x, -b.x - b.y);
+    v[0] = cadd(e[0], o[0]);
+    v[4] = csub(e[0], o[0]);
+    v[1] = __ffma2_rn(p, make_float2(h, h), e[1]);
+    v[5] = __ffma2_rn(p, make_float2(-h, -h), e[1]);
+    v[2] = cadd_rot(e[2], o[2], inv);
+    v[6] = csub_rot(e[2], o[2], inv);
+    v[3] = __ffma2_rn(q, make_float2(h, h), e[3]);
+    v[7] = __ffma2_rn(q, make_float2(-h, -h), e[3]);
+    return;
+  }
   o[1] = w8<T>(o[1], inv);
   o[3] = w8<T>(o[3], inv);
 #pragma unroll
