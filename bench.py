@@ -12,7 +12,8 @@ A step is one vel_TS over that state (dof = 11 * 1023 * 512 complex MPT coeffici
   e2e        the same metric through the C ABI with host buffers: every step copies the
              state in from pinned host memory, advances one step and copies it back
   roofline   the dominant pass (the z pass: z transforms + nonlinear term) against HBM,
-             plus its FP64 arithmetic rate against the measured FP64 FMA peak
+             plus its arithmetic rate against the measured FP64 FMA peak (above 1: the passes
+             compute in 64-bit fixed point, on the integer pipes)
   cpu_baseline  the C++ FP64 / OpenMP restatement of the step (oracle/cpu_step.cpp) on
              a bounded sample of the same workload (about 10 s on all host cores, plus about
              6 s on one core; rank 0, N = 1)
@@ -361,7 +362,7 @@ def measure_resident(ens, args, pg, world, dev):
                      "unit": "GB/s", "frac": achieved / hbm, "traffic": None,
                      "peak_source": f"{hbm_src} hbm_gbs"},
         "alu_roofline": {"kernel": "z_nonlinear", "achieved": z_tflops, "peak": peak_fma,
-                         "unit": "TFLOP/s", "frac": z_tflops / peak_fma, "pipe": "fp64" if fp64 else "fp32",
+                         "unit": "TFLOP/s", "frac": z_tflops / peak_fma, "pipe": "fp64 FMA (the passes run in 64-bit fixed point)" if fp64 else "fp32",
                          "peak_source": "measured FMA-chain probe on this GPU"},
     }
 
@@ -374,7 +375,9 @@ def mwf_solver():
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of the z pass per launch, from single-
 # kernel ncu captures of smaller cases (profiles/z_nonlinear_fp64_m6_768sq.md,
 # profiles/batched_dram_fp32_ensemble64.md) scaled by the points processed:
-#  - FP64 M6: the 768^2 grid read 108.07 MB and wrote 129.06 MB; the 1536^2 grid has 4x the points;
+#  - FP64 M6: the 768^2 grid read 108.07 MB and wrote 129.06 MB; the 1536^2 grid has 4x the points
+#    (captured from the pass in FP64 arithmetic; the fixed-point one moves the same T and NLT, and
+#    14 MB of row norms);
 #  - batched FP32 M4 z pass: DRAM read per run of MM = NN = 32, 48, 64, 96, 128 (the capture's
 #    reads divided by its runs of each size; 0.2-1.1 % above the algorithmic read of T), plus the
 #    algorithmic write KK X NN 8 B, which at the capture's size stays in L2.

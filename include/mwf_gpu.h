@@ -55,7 +55,8 @@ typedef struct mwf_run_desc {
   /* Tuning knobs, 0 = the planner's default (chosen by mwf_gb300.autotune by timing):
    * columns per x-forward / x-inverse work item, x lines per z-pass work item, and the
    * largest FFT radix of the x and z transforms (8, 12 or 16; capped per pass and
-   * precision).  No counterpart in the reference, whose FFTW plans are tuned at start-up
+   * precision).  Any knob of an FP64 run selects the passes in FP64 arithmetic in the place of
+   * those in 64-bit fixed point, a radix of an FP32 run the kernels with run-time plans.  No counterpart in the reference, whose FFTW plans are tuned at start-up
    * by FFTW itself (transform.fftw5.f90:33-59, flag FFTW_PATIENT). */
   int xf_cols;
   int xi_cols;
@@ -245,7 +246,8 @@ long long mwf_run_dof(const mwf_run_desc* d);
 long long mwf_footprint_bytes(const mwf_run_desc* runs, int n_runs);
 
 /* How the library would step one run: the kernels of its three passes and their tiling, as the
- * planner of mwf_create chooses them (host only: no device is needed).  batched_* = 1 selects
+ * planner chooses them (host only: no device is needed); mwf_create narrows the FP32 items of
+ * launches that would leave SMs without one.  batched_* = 1 selects
  * the FP32 kernels with compile-time plans (subset-split x passes, batched z pass), 0 the
  * kernels with run-time plans.  *_ctas_per_sm is the occupancy a batched kernel is compiled for
  * (0 for the others).  Returns MWF_OK, or MWF_ERR_SIZE / MWF_ERR_ARG (with mwf_last_error) for a

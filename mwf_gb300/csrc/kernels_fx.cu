@@ -19,9 +19,8 @@ static cudaError_t fx_launch(K k, int nt, const RunDesc* runs, const WorkItem* i
   return cudaGetLastError();
 }
 
-cudaError_t launch_x_forward_fx(int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st) {
-  return nt == 256 ? fx_launch(x_forward_fx_kernel<256>, nt, runs, items, n, smem, st)
-                   : fx_launch(x_forward_fx_kernel<512>, nt, runs, items, n, smem, st);
+cudaError_t launch_x_forward_fx(const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st) {
+  return fx_launch(x_forward_fx_kernel<256>, 256, runs, items, n, smem, st);
 }
 
 cudaError_t launch_z_fx(int K0, int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st) {

@@ -340,7 +340,7 @@ struct RunHost {
   // size of the z pass
   bool fx = false;
   int fx_nb = 0, fx_xi_nb = 0, fx_lines = 0, fx_nblk = 0, fx_tab = 0, fx_group = 0;
-  int fx_xf_nt = 0, fx_z_nt = 0, fx_xi_nt = 0;
+  int fx_z_nt = 0, fx_xi_nt = 0;      // the x forward always fits half an SM: 256
   size_t off_fx = 0;
   struct FxOff { size_t twX, twZ, twM, twQ, gn, mp, ms, rev, revQ, colE, blkE, rowE, minE, rowP, end; };
   FxOff fx_off() const {
@@ -533,7 +533,6 @@ bool plan_run(RunHost& r, const char*& why) {
     // widest column blocks (whole sectors of T) that still give every slot an item
     r.fx_nb = kFxMaxCols;
     while (r.fx_nb > 1 && (fx_xf_smem(d.MM, r.fx_nb) > half || (r.fx_nb > 2 && items(r.fx_nb, 2 * r.KK) < slots))) r.fx_nb /= 2;
-    r.fx_xf_nt = fx_xf_smem(d.MM, r.fx_nb) <= half ? 256 : 512;
     r.fx_nblk = (d.NN + r.fx_nb - 1) / r.fx_nb + 1;    // and column n = 0 by itself
     r.fx_xi_nb = kFxMaxCols;
     while (r.fx_xi_nb > 1 && (fx_xi_smem(d.MM, r.fx_xi_nb) > (r.fx_xi_nb == 2 ? whole : half) ||
@@ -625,7 +624,7 @@ struct Launch {
 
 cudaError_t launch_pass(const Launch& L, const RunDesc* runs, const WorkItem* items, int* err, cudaStream_t st) {
   if (L.fx) {
-    if (L.kind == 0) return launch_x_forward_fx(L.nt, runs, items, L.nitems, L.smem, st);
+    if (L.kind == 0) return launch_x_forward_fx(runs, items, L.nitems, L.smem, st);
     if (L.kind == 1) return launch_z_fx(L.K0, L.nt, runs, items, L.nitems, L.smem, st);
     return launch_x_inverse_fx(L.nt, runs, items, L.nitems, L.smem, st);
   }
@@ -1093,7 +1092,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
         for (int i = 0; i < n_runs; ++i) {
           const RunHost& r = h->runs[i];
           if (!r.fx) continue;
-          if (kind == 0 && r.fx_xf_nt == nt) {
+          if (kind == 0 && nt == 256) {
             for (int n0 = 0; n0 < r.d.NN; n0 += r.fx_nb)
               for (int f = 0; f < 2 * r.KK; ++f) items.push_back(WorkItem{i, n0, f, 0});
             L.smem = std::max(L.smem, fx_xf_smem(r.d.MM, r.fx_nb));

@@ -1,5 +1,8 @@
 // The three passes of one MWF timestep (sm_103a), templated on the arithmetic type T
-// (double for the plain FP64 path, float for the FP32 path) and on K0 (4 = M4, 6 = M6).
+// (double or float) and on K0 (4 = M4, 6 = M6).  They step the runs that tuning knobs direct to them,
+// M4 FP64 runs beyond NN = 768 and the runs of mwf_step_noalloc; other FP64 runs step in fixed point
+// (mwf_fxpass.cuh), FP32 runs in mwf_xbatch.cuh / mwf_zbatch.cuh or mwf_xwarp.cuh / mwf_zwarp.cuh.  Their
+// x forward also serves the FP32 diagnostics.
 //
 //   x_forward : MPT state -> u,v,w and d/dx u,v,w (var_mpt2spec + vel_addlam +
 //               var_spec_grad, variables.f90:390-434,600-612, velocity.f90:76-82), padded

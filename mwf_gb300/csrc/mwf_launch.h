@@ -107,7 +107,7 @@ constexpr size_t fx_z_smem(int K0, int Q, int L, int tables = 0) {
 }
 constexpr size_t fx_xf_smem(int MM, int nb) { return 16 * ((((size_t)3 * nb * MM + 7) & ~(size_t)7) + MM); }
 constexpr size_t fx_xi_smem(int MM, int nb) { return 16 * ((((size_t)9 * nb * MM + 7) & ~(size_t)7) + MM); }
-cudaError_t launch_x_forward_fx(int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st);
+cudaError_t launch_x_forward_fx(const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st);
 cudaError_t launch_z_fx(int K0, int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st);
 cudaError_t launch_x_inverse_fx(int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st);
 
