@@ -58,6 +58,14 @@ __device__ __forceinline__ FxNorm fx_norm_add(FxNorm a, FxNorm b) {
   return r;
 }
 
+__device__ __forceinline__ FxNorm fx_norm_mul(FxNorm a, FxNorm b) { return FxNorm{a.S * b.S, a.E + b.E}; }
+// |v| (truncated by less than 2^-23; subnormals count as zero)
+__device__ __forceinline__ FxNorm fx_norm(double v) {
+  const u64 b = fx_bits(v);
+  const int ex = (int)(b >> 52) & 0x7ff;
+  return FxNorm{ex == 0 ? 0.f : __uint_as_float(0x3f800000u | ((unsigned)(b >> 29) & 0x7fffffu)), ex - 1023};
+}
+
 // ---------------------------------------------------------------------------------------
 // x forward
 // ---------------------------------------------------------------------------------------
@@ -166,32 +174,35 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDes
     }
   }
   __syncthreads();
+  // (in floats with an exponent: an FP64 instruction of a warp takes 74 clocks, and these chains of
+  // them were 2 us of every block)
   if (threadIdx.x < nb) {
     const int l = threadIdx.x, n = n0 + l;
-    const double a1 = fabs(R.alpha), n1 = R.gamma * n, g1 = fabs(n1), kb = kbeta<double>(k), k1 = fabs(kb);
+    const FxNorm a1 = fx_norm(R.alpha), g1 = fx_norm_mul(fx_norm(R.gamma), FxNorm{(float)n, 0}), k1{(float)k * 1.570797f, 0};
     auto bound = [&](int i) {                         // i = 0: of the sum, 2: of the largest
-      const double s0 = scalbn((double)mom[0][i][l], momE[0][l]);
-      const double t0 = scalbn((double)mom[1][i][l], momE[1][l]), t1 = scalbn((double)mom[1][i + 1][l], momE[1][l]);
-      double L = comp == 0 ? g1 * s0 + k1 * a1 * t0 : comp == 2 ? a1 * s0 + k1 * g1 * t0 : a1 * a1 * t0 + g1 * g1 * t1;
+      const FxNorm s0{mom[0][i][l], momE[0][l]}, t0{mom[1][i][l], momE[1][l]}, t1{mom[1][i + 1][l], momE[1][l]};
+      FxNorm L = comp == 0   ? fx_norm_add(fx_norm_mul(g1, s0), fx_norm_mul(fx_norm_mul(k1, a1), t0))
+                 : comp == 2 ? fx_norm_add(fx_norm_mul(a1, s0), fx_norm_mul(fx_norm_mul(k1, g1), t0))
+                             : fx_norm_add(fx_norm_mul(fx_norm_mul(a1, a1), t0), fx_norm_mul(fx_norm_mul(g1, g1), t1));
       if (n == 0 && !deriv && comp != 1) {            // the mean flows u_k = psi_k, w_k = phi_k, and the base flow
         const double2 v = c[(size_t)(comp == 0 || k == 0 ? k : k + K0 - 1) * M];
-        L += fabs(v.x) + fabs(v.y) + (k == 1 ? 1.0 : 0.0);
+        L = fx_norm_add(L, fx_norm_add(fx_norm(v.x), fx_norm(v.y)));
+        if (k == 1) L = fx_norm_add(L, FxNorm{1.f, 0});
       }
-      if (deriv) L *= a1;
-      return L * 1.0001;
+      if (deriv) L = fx_norm_mul(L, a1);
+      L.S *= 1.0003f;
+      return L;
     };
-    const double L = bound(0);
-    const int ex = (int)(fx_bits(L) >> 52) & 0x7ff;
-    const int e = momN[0][l] || momN[1][l] || ex == 0x7ff ? kFxNan : (L == 0.0 ? kFxZero : 61 - (ex - 1022));
+    const FxNorm L = bound(0), most = bound(2);
+    const int e = momN[0][l] || momN[1][l] ? kFxNan : (L.S == 0.f ? kFxZero : 61 - (L.E + fx_bits_above(L.S)));
     // a value of the subset lines is the sum of two coefficients
-    const double most = bound(2);
-    const int mx = (int)(fx_bits(most) >> 52) & 0x7ff;
-    const int fg = mx == 0 || mx == 0x7ff ? 0
-        : fx_fine(R.fx_planM, true, (float)fx_value((fx_bits(most) & 0xfffffffffffffull) | (1024ull << 52)), mx - 1023, e);
+    const int fg = fx_fine(R.fx_planM, true, most.S, most.E + 1, e);
     for (int s = 0; s < 3; ++s) fine[3 * l + s] = fg;
     colE[l] = e;
     R.fx_colE[(size_t)f * NN + n] = e;
-    const double sg = deriv ? -1.0 : 1.0;
+  } else if (threadIdx.x >= 32 && threadIdx.x < 32 + nb) {
+    const int l = threadIdx.x - 32;
+    const double n1 = R.gamma * (n0 + l), kb = kbeta<double>(k), sg = deriv ? -1.0 : 1.0;
     colN[0][l] = fx_factor(comp == 0 ? -sg * n1 : comp == 2 ? sg : 1.0);
     colN[1][l] = fx_factor(comp == 0 ? sg * kb : comp == 2 ? sg * (kb * n1) : n1 * n1);
   }
