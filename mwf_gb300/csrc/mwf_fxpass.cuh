@@ -924,7 +924,10 @@ __global__ void __launch_bounds__(NT, 512 / NT) x_inverse_fx_kernel(const RunDes
       }
     }
     // AB2 / implicit update (velocity.f90:24-40); onl <- nl
-    auto update = [&](double rr, double il, double cv, double nv, double ov) { return fma(rr, cv, hdt * fma(3.0, nv, -ov)) * il; };
+    // (rounded as the FP64-arithmetic pass rounds it: rr c first, which is nearly all of the sum)
+    auto update = [&](double rr, double il, double cv, double nv, double ov) {
+      return fma(hdt, fma(3.0, nv, -ov), __dmul_rn(rr, cv)) * il;
+    };
     {
       const double2 ov = first ? npsi : o0;
       double x = update(r0, v0, c0.x, npsi.x, ov.x);

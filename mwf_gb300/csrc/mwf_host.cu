@@ -937,7 +937,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
 #endif
   // FP32 items by what their launch holds.  One run, us a step with the widest items and with these: M4,
   // 32 x 32 18.5 and 13.3, 64 x 64 23.8 and 16.5, 36 x 36 40.5 and 22.8, 72 x 72 54.2 and 28.9; M6, 64 x 64
-  // 25.2 and 21.1, 72 x 72 54.4 and 39.1; eight M4 36 x 36 43.5 and 37.  Full launches keep the widest.
+  // 25.2 and 20.4, 72 x 72 54.4 and 34.7; eight M4 36 x 36 43.5 and 32.9.  Full launches keep the widest.
   {
     std::map<std::vector<int>, std::vector<ItemWidth>> xf, z, xi, xwf, xwi, zw;
     for (RunHost& r : h->runs) {
