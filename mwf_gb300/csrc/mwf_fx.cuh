@@ -111,11 +111,15 @@ __host__ __device__ __forceinline__ i64 fx_shift(i64 x, int sh) {
   const int up = sh > 0 ? sh : 0;
   return (fx_sar(fx_shl(x, up + 1), up - sh) + 1) >> 1;
 }
-// x 2^-r, r >= 1, and x / 2, rounded to nearest, ties to even: ties rounded up are a bias of 2^-(r+1),
+// x 2^-r, r >= 1, |x| <= 2^62, and x / 2, rounded to nearest, ties to even: ties rounded up are a bias of 2^-(r+1),
 // the same for all values of a stage, which the later stages add up in the lowest wavenumbers (M4
 // 512 x 512, white spectrum: the nonlinear term was 1.24 times as far off as with FP64 arithmetic, now 0.96).
+// Shifts beyond 63, which leave nothing, are those of 63 (of 64 and more the half of the last bit
+// would be 0 or overflow, and everything, zeros too, could become -1): they come from directions or
+// rows of the coupling that are zero, or far below the others.
 __host__ __device__ __forceinline__ i64 fx_down(i64 x, int r) {
-  return fx_sar(x + (fx_shl(1, r - 1) - 1) + (i64)((int)fx_sar(x, r) & 1), r);
+  const int k = r < 63 ? r : 63;
+  return fx_sar(x + (fx_shl(1, k - 1) - 1) + (i64)((int)fx_sar(x, k) & 1), k);
 }
 __host__ __device__ __forceinline__ i64 fx_half(i64 x) { return (x >> 1) + (i64)((int)x & (int)(x >> 1) & 1); }
 // x 2^sh, rounded down when sh < 0.
