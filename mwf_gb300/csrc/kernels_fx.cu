@@ -4,16 +4,23 @@
 
 namespace mwf {
 
+// Allow kernel k the most dynamic shared memory that any call of it takes.  The limit belongs to the kernel, not
+// to a launch: the same value from every call keeps a launch recorded in a graph valid, and other
+// threads' calls with longer lines between their own setting and launch.
 template <typename K>
-static cudaError_t fx_launch(K k, int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st) {
-  if (n <= 0) return cudaSuccess;
-  // the largest size that any run takes, so that a launch recorded in a graph stays valid
+static cudaError_t fx_allow_smem(K k, size_t smem) {
   cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, k);
+  const cudaError_t e = cudaFuncGetAttributes(&fa, k);
   if (e != cudaSuccess) return e;
   const int most = (int)(zb_smem_budget(1) - fa.sharedSizeBytes);
   if (smem > (size_t)most) return cudaErrorInvalidValue;
-  e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
+template <typename K>
+static cudaError_t fx_launch(K k, int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  const cudaError_t e = fx_allow_smem(k, smem);
   if (e != cudaSuccess) return e;
   k<<<n, nt, smem, st>>>(runs, items);
   return cudaGetLastError();
@@ -49,8 +56,7 @@ static int fx_line_tile(int N, int all, int most, int outer) {
 template <typename K, typename... A>
 static cudaError_t fx_line_launch(K k, long grid, int N, int lines, cudaStream_t st, A... args) {
   const size_t smem = fx_line_smem_bytes(N, lines);
-  if (smem > zb_smem_budget(1)) return cudaErrorInvalidValue;
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = fx_allow_smem(k, smem);
   if (e != cudaSuccess) return e;
   k<<<(unsigned)grid, kFxLineThreads, smem, st>>>(args...);
   return cudaGetLastError();
