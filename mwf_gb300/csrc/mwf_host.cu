@@ -770,8 +770,9 @@ int check_device_err(mwf_handle* h) {
 }
 
 // Whether the device may access the n doubles at p in place: they lie within one pinned host
-// allocation (or registration).
+// allocation (or registration), at an address that the kernels' 8-byte accesses take (copies take any).
 bool device_reads_host(const double* p, size_t n) {
+  if (reinterpret_cast<uintptr_t>(p) % sizeof(double)) return false;
   static const auto attr = [] {
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult q;
