@@ -900,9 +900,9 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 1024 / NT : 512 / NT) x_i
 // Neumaier-compensated per-thread sums and a pairwise tree across the block.
 // ---------------------------------------------------------------------------------------
 // The state is checked for NaN and infinities (every coefficient, also the ones no field
-// reads) on the way, and the block that finishes last adds the partials, pairwise in a fixed order, and
-// writes the outcome to the host word `out` (mapped memory): one launch and no copy, where a memset,
-// a separate check, a serial final sum and three copies took 40 us per call.
+// reads) on the way, and the block that finishes last adds the partials in a fixed order, with
+// compensated sums, and writes the outcome to the host word `out` (mapped memory): one launch and no copy, where
+// a memset, a separate check, a serial final sum and three copies took 40 us per call.
 template <typename T>
 __global__ void __launch_bounds__(kEnergyThreads) energy_kernel(const RunDesc* __restrict__ runs, int run, double* partial,
                                                                  int* flag, unsigned* ticket, const int* err, HostOut* out) {
@@ -938,17 +938,14 @@ __global__ void __launch_bounds__(kEnergyThreads) energy_kernel(const RunDesc* _
       sum = y;
     }
   }
-  __shared__ double red[kEnergyThreads];
+  __shared__ double red[kEnergyThreads], redc[kEnergyThreads];
   __shared__ bool last;
-  auto tree = [&](double v) {
-    red[threadIdx.x] = v;
+  red[threadIdx.x] = sum + comp;
+  __syncthreads();
+  for (int h = kEnergyThreads / 2; h > 0; h >>= 1) {
+    if ((int)threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
     __syncthreads();
-    for (int h = kEnergyThreads / 2; h > 0; h >>= 1) {
-      if ((int)threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
-      __syncthreads();
-    }
-  };
-  tree(sum + comp);
+  }
   bad = __syncthreads_or(bad);
   if (threadIdx.x == 0) {
     partial[blockIdx.x] = red[0];
@@ -959,11 +956,29 @@ __global__ void __launch_bounds__(kEnergyThreads) energy_kernel(const RunDesc* _
   }
   __syncthreads();
   if (!last) return;
-  double v = 0.0;
-  for (unsigned i = threadIdx.x; i < gridDim.x; i += kEnergyThreads) v += __ldcg(&partial[i]);
-  tree(v);
+  // s + c += t with the rounding error of the sum kept in c; the terms are not negative, so their bits
+  // order them
+  auto add = [](double& s, double& c, double t) {
+    const bool up = __double_as_longlong(t) > __double_as_longlong(s);
+    const double a = up ? t : s, b = up ? s : t;
+    s = a + b;
+    c += b - (s - a);
+  };
+  double v = 0.0, vc = 0.0;
+  for (unsigned i = threadIdx.x; i < gridDim.x; i += kEnergyThreads) add(v, vc, __ldcg(&partial[i]));
+  red[threadIdx.x] = v;
+  redc[threadIdx.x] = vc;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  static_assert(kEnergyThreads == 64, "two warps");
+  for (unsigned o = 32; o > 0; o >>= 1) {
+    if (o >= gridDim.x) continue;                     // those threads had no partial
+    const double t = o == 32 ? red[threadIdx.x + 32] : __shfl_down_sync(0xffffffffu, v, o);
+    vc += o == 32 ? redc[threadIdx.x + 32] : __shfl_down_sync(0xffffffffu, vc, o);
+    add(v, vc, t);
+  }
   if (threadIdx.x == 0) {
-    out->value = red[0];
+    out->value = v + vc;
     out->flag = atomicExch(flag, 0);
     out->err = *err;
   }
