@@ -6,9 +6,11 @@ Knobs (fields of RunParams / mwf_run_desc, 0 = planner default):
     x_radix, z_radix   largest radix of the x / z transforms (8, 12, 16 within the caps)
 The x knobs and the z knobs are tuned separately: every candidate is one handle holding 1, 8
 or 32 copies of the run (the batch context: the best tiles of a run alone and of a run in a
-large batch differ) whose passes are timed with CUDA events (mwf_profile_passes); the
-default configuration is always a candidate, so tuning never picks a slower one in that
-context.  Results are cached in a JSON file keyed by precision, model, grid and context
+large batch differ) whose passes are timed with CUDA events (mwf_profile_passes).  A knob can
+also move other passes to other kernels (any knob of an FP64 run takes all three off the
+fixed-point ones), so the pass times of different candidates do not add up: the
+combination of the best is timed as a whole against the default configuration, which stays unless
+that is slower.  So tuning never picks a slower one in that context.  Results are cached in a JSON file keyed by precision, model, grid and context
 (MWF_TUNE_CACHE, default ~/.cache/mwf_gb300/tuning.json).  This plays the part of the FFTW_PATIENT planning the
 reference does at start-up (transform.fftw5.f90:33-59).
 """
@@ -21,6 +23,7 @@ from .solver import Ensemble, footprint_bytes
 
 CACHE = os.environ.get("MWF_TUNE_CACHE", os.path.join(os.path.expanduser("~"), ".cache", "mwf_gb300",
                                                       "tuning.json"))
+KNOBS = ("xf_cols", "xi_cols", "z_lines", "x_radix", "z_radix")
 _mem = {}
 
 
@@ -29,7 +32,7 @@ def batch_bucket(copies):
     return 1 if copies <= 1 else (8 if copies <= 8 else 32)
 
 
-KERNEL_VERSION = 5      # bumped when the kernels' tiling changes, so old cache entries are ignored
+KERNEL_VERSION = 6      # bumped when the kernels' tiling changes, so old cache entries are ignored
 
 
 def key(p, copies=1):
@@ -76,7 +79,7 @@ def tune(p, device=0, reps=3, copies=1):
     """Time the candidates for run p (in a handle of `copies` such runs, the tuning context)
     and return the best knob settings (a dict)."""
     copies = batch_bucket(copies)
-    base = p.with_(xf_cols=0, xi_cols=0, z_lines=0, x_radix=0, z_radix=0)
+    base = p.with_(**{n: 0 for n in KNOBS})
     x_radices = [8, 12, 16] if p.precision == "fp32" else [8, 12]
     z_radices = [8, 12] if p.precision == "fp32" else [8]
     widths = [1, 2, 4, 8, 16]
@@ -108,7 +111,14 @@ def tune(p, device=0, reps=3, copies=1):
                 best_zt, best_z = t[1], {"z_radix": zr, "z_lines": lines}
     out = dict(best_x)
     out.update(best_z)
-    out["ms"] = {"x": best_xt, "z": best_zt, "copies": copies}
+    default = {n: 0 for n in KNOBS}
+    step = {"default": sum(_time(base, device, reps, copies)), "tuned": None}
+    if out and out != default:
+        q = base.with_(**out)
+        step["tuned"] = sum(_time(q, device, reps, copies)) if _valid(q) else None
+    if step["tuned"] is None or step["tuned"] >= step["default"]:
+        out = default
+    out["ms"] = {"x": best_xt, "z": best_zt, "copies": copies, **step}
     return out
 
 
@@ -120,5 +130,5 @@ def tuned(p, device=0, reps=3, retune=False, copies=1):
     if retune or k not in db:
         db[k] = tune(p, device=device, reps=reps, copies=copies)
         _store()
-    knobs = {n: db[k][n] for n in ("xf_cols", "xi_cols", "z_lines", "x_radix", "z_radix")}
+    knobs = {n: db[k][n] for n in KNOBS}
     return p.with_(**knobs)
