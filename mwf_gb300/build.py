@@ -15,6 +15,10 @@ LIB = os.path.join(LIBDIR, "libmwfgpu.so")
 SOURCES = ["mwf_host.cu", "kernels_f64.cu", "kernels_f32.cu", "kernels_zb.cu", "kernels_xb.cu", "kernels_persist.cu", "kernels_fx.cu", "kernels_zw.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off"]
+# The batched FP32 passes are compiled once for every count of columns or lines that an item can hold, and
+# again in the persistent step; an item's count depends on what else its launch holds.  Their fused
+# multiply-adds are spelled out, and without the compiler's own a run has the same bits in all of them.
+SOURCE_FLAGS = {f: ["-fmad=false"] for f in ("kernels_zb.cu", "kernels_xb.cu", "kernels_persist.cu")}
 
 
 def nvcc():
@@ -24,7 +28,7 @@ def nvcc():
 
 def _compile(src):
     obj = os.path.join(BUILD, os.path.splitext(src)[0] + ".o")
-    cmd = [nvcc(), *ARCH, *FLAGS, "-c", os.path.join(CSRC, src), "-o", obj]
+    cmd = [nvcc(), *ARCH, *FLAGS, *SOURCE_FLAGS.get(src, []), "-c", os.path.join(CSRC, src), "-o", obj]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"nvcc failed for {src}:\n{r.stdout}\n{r.stderr}")
