@@ -9,9 +9,11 @@
 // coefficients alike the L1 norm is about 1.6 N of them, so 2^-61 of it is 2^-50 of a coefficient at
 // N = 1024, more than the 2^-53 of FP64 arithmetic.  So until the first two stages are
 // done, whose results are sums of only a few values, a line has finer scales from its largest value
-// (fx_fine).  Error of the nonlinear term against 80-bit arithmetic, M4 96 x 96 ... 512 x 512 and M6
-// modes, as a fraction of that of the FP64-arithmetic kernels: Gaussian states 0.30 ... 0.47, spectra
-// 1 / (1 + k^2 / 20) 0.56 ... 0.75, white ones 0.55 ... 0.96 (without the finer scales up to 1.7 at 256 x 256).
+// (fx_fine).  Error of the nonlinear term against extended precision, lengths of 3 ... 1024 modes,
+// as a fraction of that of the FP64-arithmetic kernels: Gaussian states 0.16 ... 0.22 on square grids and up to 0.95 on
+// thin ones, spectra 1 / (1 + k^2 / 20) 0.36 ... 0.92, white ones 0.27 ... 0.86, wall-normal modes that fall by 10 from
+// one to the next 0.4 ... 1.07 (of the whole term; the last of such modes alone up to 50: the coupling's operands share a
+// scale).
 //
 // Transforms are in place, decimation in frequency backward (natural in, digit-reversed out) and
 // decimation in time forward (digit-reversed in, natural out): a butterfly reads and writes the
@@ -113,7 +115,8 @@ __host__ __device__ __forceinline__ i64 fx_shift(i64 x, int sh) {
 }
 // x 2^-r, r >= 1, |x| <= 2^62, and x / 2, rounded to nearest, ties to even: ties rounded up are a bias of 2^-(r+1),
 // the same for all values of a stage, which the later stages add up in the lowest wavenumbers (M4
-// 512 x 512, white spectrum: the nonlinear term was 1.24 times as far off as with FP64 arithmetic, now 0.96).
+// 512 x 512, white spectrum: the nonlinear term was 1.24 times as far off as with FP64 arithmetic, with ties
+// to even 0.96 and, the coupling's sums rounded more finely, 0.38).
 // Shifts beyond 63, which leave nothing, are those of 63 (of 64 and more the half of the last bit
 // would be 0 or overflow, and everything, zeros too, could become -1): they come from directions or
 // rows of the coupling that are zero, or far below the others.
@@ -122,11 +125,6 @@ __host__ __device__ __forceinline__ i64 fx_down(i64 x, int r) {
   return fx_sar(x + (fx_shl(1, k - 1) - 1) + (i64)((int)fx_sar(x, k) & 1), k);
 }
 __host__ __device__ __forceinline__ i64 fx_half(i64 x) { return (x >> 1) + (i64)((int)x & (int)(x >> 1) & 1); }
-// x 2^sh, rounded down when sh < 0.
-__host__ __device__ __forceinline__ i64 fx_scale(i64 x, int sh) {
-  const int up = sh > 0 ? sh : 0;
-  return fx_sar(fx_shl(x, up), up - sh);
-}
 __host__ __device__ __forceinline__ longlong2 fx_shift2(longlong2 a, int sh) {
   longlong2 r;
   r.x = fx_shift(a.x, sh);
@@ -399,25 +397,40 @@ __device__ __forceinline__ void fx_fft(longlong2* buf, int base, int G, const Fx
   }
 }
 
-// ---- products of the coupling: operands of at most 57 bits as h 2^28 + l, |l| <= 2^27 ----
+// ---- products of the coupling: operands of at most 59 bits as h 2^30 + l, |l| <= 2^29 ----
 struct FxLimbs { int h, l; };
-struct FxAcc { i64 hi, cr; };      // hi 2^56 + cr 2^28
+struct FxAcc { i64 hi, cr; };      // hi 2^60 + cr 2^30
 __device__ __forceinline__ FxLimbs fx_limbs(i64 x) {
   FxLimbs o;
-  o.h = (int)((x + (1ll << 27)) >> 28);
-  o.l = (int)((unsigned)(u64)x << 4) >> 4;
+  o.h = (int)((x + (1ll << 29)) >> 30);
+  o.l = (int)((unsigned)(u64)x << 2) >> 2;
+  return o;
+}
+// fx_limbs(fx_shift(x, sh)), the two roundings of the shifted value in one addition each
+__device__ __forceinline__ FxLimbs fx_shift_limbs(i64 x, int sh) {
+  const int up = sh > 0 ? sh : 0;
+  const i64 t = fx_sar(fx_shl(x, up + 1), up - sh);
+  FxLimbs o;
+  o.h = (int)((t + ((1ll << 30) + 1)) >> 31);
+  o.l = (int)(((unsigned)(u64)t + 1u) << 1) >> 2;
   return o;
 }
 __device__ __forceinline__ FxLimbs fx_twice(FxLimbs a) { return FxLimbs{2 * a.h, 2 * a.l}; }
-__device__ __forceinline__ FxLimbs fx_times(FxLimbs a, int k) { return FxLimbs{k * a.h, k * a.l}; }
-// The sums over a coupling row stay below 2^62; the products of two low limbs (2^-60 of the
-// largest product) are dropped.
+// k = 1 ... 5 times an operand of 58 bits (5 l would overflow)
+__device__ __forceinline__ FxLimbs fx_times(FxLimbs a, int k) {
+  return k <= 4 ? FxLimbs{k * a.h, k * a.l} : fx_limbs(k * (((i64)a.h << 30) + a.l));
+}
+// For operands of 58 and 59 bits (58 and 58 in the y direction) and the largest weights of a coupling row, 12
+// (x, z) and 24 (y, the factors of fx_times included), hi stays below 2^61 and cr below 2^63; the products of two low
+// limbs (at most 2^-59 of the largest product) are dropped.
 __device__ __forceinline__ void fx_mac(FxAcc& a, FxLimbs v, FxLimbs d) {
   a.hi = fx_madw(v.h, d.h, a.hi);
   a.cr = fx_madw(v.h, d.l, fx_madw(v.l, d.h, a.cr));
 }
 __device__ __forceinline__ void fx_msb(FxAcc& a, FxLimbs v, FxLimbs d) { fx_mac(a, FxLimbs{-v.h, -v.l}, d); }
-// The sum in units of 2^56.
-__device__ __forceinline__ i64 fx_sum(FxAcc a) { return a.hi + ((a.cr + (1ll << 27)) >> 28); }
+// The sum times 2^(left - 60), rounded; 0 <= left <= 29, |.| < 2^63.
+__device__ __forceinline__ i64 fx_sum(FxAcc a, int left) {
+  return fx_shl(a.hi, left) + fx_sar(a.cr + fx_shl(1, 29 - left), 30 - left);
+}
 
 }  // namespace mwf

@@ -420,7 +420,10 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) z_fx_kernel(const RunDe
   int* mx = eL + NTR * L;                                        // [2 NTR L] the lines' finer first scale, then largest
                                                                  // high words (re, im), then shifts, then the finer scale
   int* ge = mx + 2 * NTR * L;                                    // [kFxGroups L] group exponents
-  int* eo = ge + kFxGroups * L;                                  // [3 L] exponents of the products
+  float* gb = reinterpret_cast<float*>(ge + kFxGroups * L);      // [3][kFxGroups L] of a group's fields, relative to its full
+                                                                 // scale: the largest value, the sum of the
+                                                                 // largest, the same sum with factors k
+  int* eo = reinterpret_cast<int*>(gb + 3 * kFxGroups * L);      // [3 L] exponents of the products
   int* sh = eo + 3 * L;                                          // [NPAIR L] forward line shifts
   int* bad = sh + NPAIR * L;                                     // [L] NaN lines
   // Where they fit (RunDesc::fx_tab): the subset's twiddles e^{-2 pi i ns/Z}, then gamma n, which the fill
@@ -579,18 +582,29 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) z_fx_kernel(const RunDe
   }
   __syncthreads();
 
-  // ---- one exponent per group: the largest value of a velocity group fills 56 bits, of a
-  //      derivative group 57; mx becomes the shift of each part of a line to its group ----
+  // ---- one exponent per group: the largest value of a velocity group fills 58 bits, of a
+  //      derivative group 59; mx becomes the shift of each part of a line to its group ----
   for (int i = threadIdx.x; i < kFxGroups * L; i += NT) {
     const int g = i / L, l = i - g * L, comp = g % 3;
-    const int f0 = fx_first<K0>(comp), f1 = f0 + fx_count<K0>(comp);
+    const int f0 = fx_first<K0>(comp), n = fx_count<K0>(comp);
     const bool vel = g < kFxDx;
     auto place = [&](int f) { return 2 * ((vel ? f / 2 : NPAIR + f) * L + l) + (vel ? (f & 1) : (g >= kFxDz)); };
     int top = -(1 << 29);
-    for (int f = f0; f < f1; ++f) top = max(top, fx_bitlen(mx[place(f)]) - eL[place(f) >> 1]);
-    const int e = (vel ? 56 : 57) - top;
+    for (int k = 0; k < n; ++k) top = max(top, fx_bitlen(mx[place(f0 + k)]) - eL[place(f0 + k) >> 1]);
+    const int e = (vel ? 58 : 59) - top;
     ge[i] = e;
-    for (int f = f0; f < f1; ++f) mx[place(f)] = e - eL[place(f) >> 1];
+    float most = 0.f, sum = 0.f, ksum = 0.f;
+    for (int k = 0; k < n; ++k) {
+      const int at = place(f0 + k), r = e - eL[at >> 1];
+      const float v = ((float)mx[at] + 1.f) * fx_pow2(r + 32 - (vel ? 58 : 59));
+      mx[at] = r;
+      most = fmaxf(most, v);
+      sum += v;
+      ksum += v * (float)(k + (comp == 1));
+    }
+    gb[i] = most;
+    gb[kFxGroups * L + i] = sum;
+    gb[2 * kFxGroups * L + i] = ksum;
   }
   __syncthreads();
 
@@ -601,6 +615,12 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) z_fx_kernel(const RunDe
   const FastDiv fQ = make_fastdiv(Q), fLQ = make_fastdiv(L * Q);
   const size_t ts = (size_t)TS * 16;
   const bool apart = 3 * L * Q <= NT;
+  // exponent of fx_sum without shifts (y: the sum is in units of b, and b/2 follows)
+  auto direction = [&](int comp, int dir, int l) {
+    return dir == 0   ? ge[kFxU * L + l] + ge[(kFxDx + comp) * L + l] - 60
+           : dir == 1 ? ge[kFxW * L + l] + ge[(kFxDz + comp) * L + l] - 60
+                      : ge[kFxV * L + l] + ge[comp * L + l] - 61;
+  };
   // velocities: scaled to their group and split, in place
   for (int e = threadIdx.x; e < L * Q; e += NT) {
     const int l = L == 1 ? 0 : fQ.div(e);
@@ -608,11 +628,29 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) z_fx_kernel(const RunDe
 #pragma unroll
     for (int f = 0; f < KK; ++f) {
       i64* const q = reinterpret_cast<i64*>(at + (f / 2) * ts) + (f & 1);
-      const FxLimbs v = fx_limbs(fx_scale(*q, mx[2 * ((f / 2) * L + l) + (f & 1)]));
+      const FxLimbs v = fx_shift_limbs(*q, mx[2 * ((f / 2) * L + l) + (f & 1)]);
       *reinterpret_cast<int2*>(q) = make_int2(v.h, v.l);
     }
   }
-  if (apart) __syncthreads();
+  // ---- one exponent per component of the products: a bound on the three directions' sums fills 62 bits.  In a
+  //      row of the coupling (i + j = k or |i - j| = k) each value of one factor meets at most two of the other, or one
+  //      twice: twice the sum of the one's largest values times the other's largest bounds it.  (From the group
+  //      scales and the largest weights alone the sums' rounding was five times that of their operands, and
+  //      for M6 32 x 512 modes that fall by 10 from one wall-normal mode to the next the term 1.3 times as far off
+  //      as with FP64 arithmetic.) ----
+  for (int i = NT - 1 - threadIdx.x; i < 3 * L; i += NT) {
+    const int comp = i / L, l = i - comp * L, N = kFxGroups * L;
+    auto bound = [&](int s_, int d, int p) {          // groups of the factors; which sum of the second (1, or 2: factors k)
+      const int a = s_ * L + l, b = d * L + l;
+      const float v = p == 1 ? fminf(gb[a] * gb[N + b], gb[N + a] * gb[b]) : 1.570797f * gb[a] * gb[2 * N + b];
+      return FxNorm{2.02f * v, (p == 1 ? 117 : 116) - ge[a] - ge[b]};
+    };
+    const FxNorm n = fx_norm_add(fx_norm_add(bound(kFxU, kFxDx + comp, 1), bound(kFxW, kFxDz + comp, 1)), bound(kFxV, comp, 2));
+    int go = n.S > 0.f ? 62 - (n.E + fx_bits_above(n.S)) : 2 * kFxZero;
+    for (int dir = 0; dir < 3; ++dir) go = min(go, direction(comp, dir, l) + 29);
+    eo[i] = go;
+  }
+  __syncthreads();
   for (int e0 = 0; e0 < (apart ? 1 : L * Q); e0 += NT) {
     const int i = e0 + threadIdx.x;
     const int part = apart ? fLQ.div(i) : 0, e = i - part * (L * Q);
@@ -625,14 +663,8 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) z_fx_kernel(const RunDe
       return FxLimbs{v.x, v.y};
     };
     constexpr FxConst b2 = fx_const(kFxQuarterPi);
-    const int gu = ge[kFxU * L + l], gv = ge[kFxV * L + l], gw = ge[kFxW * L + l];
 #pragma unroll 1
     for (int comp = first; comp < last; ++comp) {
-      const int gx = gu + ge[(kFxDx + comp) * L + l] - 56;
-      const int gz = gw + ge[(kFxDz + comp) * L + l] - 56;
-      const int gy = gv + (comp == 0 ? gu : comp == 1 ? gv : gw) - 57;
-      const int go = min(gx, min(gy, gz)) - 2;
-      if (on && e == l * Q) eo[comp * L + l] = go;
       const int f0 = comp == 0 ? 0 : comp == 1 ? K0 - 1 : 2 * K0 - 1;    // field of mode 0 (v has none)
       i64 sum[K0];
       FxAcc A[K0];
@@ -642,6 +674,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) z_fx_kernel(const RunDe
       for (int dir = on ? 0 : 3; dir < 3; ++dir) {    // x, z, y
 #pragma unroll
         for (int k = 0; k < K0; ++k) A[k] = FxAcc{0, 0};
+        const int up = eo[comp * L + l] - direction(comp, dir, l);
         if (dir < 2) {
           FxLimbs S[K0];
           const int s0 = dir ? 2 * K0 - 1 : 0;
@@ -649,13 +682,10 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) z_fx_kernel(const RunDe
           for (int k = 0; k < K0; ++k) S[k] = vel(s0 + k);
           auto ld = [&](int j) {
             const i64 q = *(reinterpret_cast<const i64*>(at + (NPAIR + f0 + j) * ts) + dir);
-            return fx_limbs(fx_scale(q, mx[2 * ((NPAIR + f0 + j) * L + l) + dir]));
+            return fx_shift_limbs(q, mx[2 * ((NPAIR + f0 + j) * L + l) + dir]);
           };
           if constexpr (K0 == 4) { if (comp == 1) nl_fx_v_4(S, ld, A); else nl_fx_p_4(S, ld, A); }
           else { if (comp == 1) nl_fx_v_6(S, ld, A); else nl_fx_p_6(S, ld, A); }
-          const int r = (dir ? gz : gx) - go;
-#pragma unroll
-          for (int k = 0; k < K0; ++k) sum[k] += fx_down(fx_sum(A[k]), r);
         } else {
           // in units of b = pi/2: 2 nl = sum v (j f_j) b
           FxLimbs V[K0], F[K0];
@@ -669,9 +699,22 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) z_fx_kernel(const RunDe
           } else {
             if constexpr (K0 == 4) nl_fx_yv_4(V, A); else nl_fx_yv_6(V, A);
           }
-#pragma unroll
-          for (int k = 0; k < K0; ++k) sum[k] += fx_down(fx_mulc(fx_sum(A[k]), b2), gy - go);
         }
+        // to the component's exponent: up by less than 30 bits, or down (a direction far below the others)
+        i64 x[K0];
+#pragma unroll
+        for (int k = 0; k < K0; ++k) x[k] = fx_sum(A[k], max(up, 0));
+        if (up < 0) {
+          const int r = min(-up, 62);
+#pragma unroll
+          for (int k = 0; k < K0; ++k) x[k] = fx_down(x[k] << 1, r + 1);
+        }
+        if (dir == 2) {
+#pragma unroll
+          for (int k = 0; k < K0; ++k) x[k] = fx_mulc(x[k], b2);
+        }
+#pragma unroll
+        for (int k = 0; k < K0; ++k) sum[k] += x[k];
       }
       // field f goes to line NPAIR + f/2, where only derivatives of this or an earlier component were
       if (apart) __syncthreads();

@@ -102,7 +102,7 @@ cudaError_t launch_persistent_step(const RunDesc* runs, const void* items, int n
 constexpr size_t fx_z_stride(int Q, int L) { return ((size_t)L * Q + 63) & ~(size_t)63; }
 constexpr size_t fx_z_smem(int K0, int Q, int L, int tables = 0) {
   const size_t kk = 3 * K0 - 1, np = (kk + 1) / 2, nt = np + kk;
-  return 16 * (nt * fx_z_stride(Q, L) + Q) + ((4 * (size_t)L * (3 * nt + 9 + 3 + np + 1) + 15) & ~(size_t)15) +
+  return 16 * (nt * fx_z_stride(Q, L) + Q) + ((4 * (size_t)L * (3 * nt + 4 * 9 + 3 + np + 1) + 15) & ~(size_t)15) +
          16 * (size_t)tables * Q;
 }
 constexpr size_t fx_xf_smem(int MM, int nb) { return 16 * ((((size_t)3 * nb * MM + 7) & ~(size_t)7) + MM); }
