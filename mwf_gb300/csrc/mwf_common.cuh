@@ -45,6 +45,10 @@ template <> __device__ __forceinline__ float2 cmul<float2>(float2 a, float2 b) {
 template <> __device__ __forceinline__ float2 cmulc<float2>(float2 a, float2 b) {
   return make_float2(__fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)), __fmaf_rn(a.y, b.x, -__fmul_rn(a.x, b.y)));
 }
+// c + a b
+__device__ __forceinline__ float2 cmac(float2 c, float2 a, float2 b) {
+  return make_float2(__fmaf_rn(a.x, b.x, __fmaf_rn(-a.y, b.y, c.x)), __fmaf_rn(a.x, b.y, __fmaf_rn(a.y, b.x, c.y)));
+}
 template <typename C> __device__ __forceinline__ C cconj(C a) { a.y = -a.y; return a; }
 
 // Division by a runtime divisor 1 <= d <= 2^16 of dividends 0 <= b < 2^16:

@@ -93,16 +93,6 @@ __device__ __forceinline__ void zb_stage(const float2* __restrict__ in, float2* 
   __syncthreads();
 }
 
-// Complex products of the fill and of P4 with every rounding spelled out (fused multiply-adds),
-// so that each kernel that inlines the item -- the per-pass launch and the persistent step --
-// rounds them alike, whatever contraction the compiler would choose in its context.
-__device__ __forceinline__ float2 zb_mul(float2 a, float2 b) {          // a b
-  return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
-}
-__device__ __forceinline__ float2 zb_mac(float2 c, float2 a, float2 b) {  // c + a b
-  return make_float2(__fmaf_rn(a.x, b.x, __fmaf_rn(-a.y, b.y, c.x)), __fmaf_rn(a.x, b.y, __fmaf_rn(a.y, b.x, c.y)));
-}
-
 // Shared memory of one batched z item: two buffers of 3 NTR L lines of Q complex floats, the
 // second starting on a 16-byte boundary (asynchronous 16-byte copy destinations).
 __host__ __device__ constexpr size_t zb_buf_elems(int K0, int Q, int L) {
@@ -245,8 +235,8 @@ __device__ __forceinline__ void z_batched_body(const RunDesc& R, int x0, unsigne
         } else {
           const C tz = s == 1 ? tz1 : tz2;              // conj(w)
           const C tq = s == 1 ? tq1 : tq2;              // eps w
-          Yn = zb_mac(zb_mul(cconj(tz), U), tq, V);
-          Yq = zb_mac(zb_mul(U2, cconj(tq)), V2, tz);
+          Yn = cmac(cmul(cconj(tz), U), tq, V);
+          Yq = cmac(cmul(U2, cconj(tq)), V2, tz);
         }
         C* dst = A + line(t, s, l) * LS;
         dst[pn] = cconj(Yn);
@@ -338,10 +328,10 @@ __device__ __forceinline__ void z_batched_body(const RunDesc& R, int x0, unsigne
         } else {
           const C tz = s == 1 ? tz1 : tz2;
           const C tq = s == 1 ? tq1 : tq2;
-          An = zb_mac(An, As, tz);
-          Bn = zb_mac(Bn, Bs, tz);
-          Aq = zb_mac(Aq, cconj(As), tq);
-          Bq = zb_mac(Bq, cconj(Bs), tq);
+          An = cmac(An, As, tz);
+          Bn = cmac(Bn, Bs, tz);
+          Aq = cmac(Aq, cconj(As), tq);
+          Bq = cmac(Bq, cconj(Bs), tq);
         }
       }
       store(t, l, n, An, Bn);
@@ -362,8 +352,8 @@ __device__ __forceinline__ void z_batched_body(const RunDesc& R, int x0, unsigne
       if (s == 0) {
         An = As; Bn = Bs;
       } else {
-        An = zb_mac(An, As, tz0);
-        Bn = zb_mac(Bn, Bs, tz0);
+        An = cmac(An, As, tz0);
+        Bn = cmac(Bn, Bs, tz0);
       }
     }
     store(t, l, 0, An, Bn);

@@ -214,8 +214,8 @@ __global__ void __launch_bounds__(NT, MINB) z_warp_kernel(const RunDesc* __restr
             Hq = cadd(U2, V2);
           } else {
             const float2 tz = __ldg(&om[n * s]), tq = __ldg(&om[nq * s]);     // conj(w), eps w
-            Hn = cadd(cmulc(U, tz), cmul(V, tq));
-            Hq = cadd(cmulc(U2, tq), cmul(V2, tz));
+            Hn = cmac(cmulc(U, tz), V, tq);
+            Hq = cmac(cmulc(U2, tq), V2, tz);
           }
           if (sl || even) buf[an + k * LS] = Hn;
           if (sl) buf[aq + k * LS] = Hq;
@@ -260,42 +260,54 @@ __global__ void __launch_bounds__(NT, MINB) z_warp_kernel(const RunDesc* __restr
       float2* __restrict__ oa = NLT + (size_t)(2 * t) * fstride + (size_t)l0 * Q;
       float2* __restrict__ ob = oa + fstride;
       auto put = [&](int o, float2 a, float2 b) {
-        if (NS == 1 && s0 > 0) {                      // this thread's sums of the earlier subsets
-          a = cadd(oa[o], a);
-          if (two) b = cadd(ob[o], b);
-        }
         oa[o] = a;
         if (two) ob[o] = b;
       };
+      const float2 none = make_float2(0.f, 0.f);
       for (int idx = lane; idx < nl * slots; idx += LN) {
         const int l = fSl.div(idx), sl = idx - l * slots;
         const int base = first + l * NS * LS, o = l * Q;
         const int n = sl ? sl : (even ? Q / 2 : 0), nq = sl ? Q - sl : n;
         const int an = base + zw_at(pl, n), aq = base + zw_at(pl, nq);
-        float2 An, Bn, Aq, Bq, A0 = make_float2(0.f, 0.f);
+        const int on = o + n, oq = o + (sl ? nq : 0);
+        const bool hasn = sl || even;
+        // sums over the subsets, with the subset's factor fused; one after the other: on top of this thread's sums of
+        // the earlier ones
+        float2 An = none, Bn = none, Aq = none, Bq = none;
+        if (NS == 1 && s0 > 0) {
+          if (hasn) { An = oa[on]; if (two) Bn = ob[on]; }
+          Aq = oa[oq];
+          if (two) Bq = ob[oq];
+        }
 #pragma unroll
         for (int k = 0; k < NS; ++k) {
           const int s = s0 + k;
           const float2 g = buf[an + k * LS], m = buf[aq + k * LS];
-          float2 A = make_float2(hscale * (g.x + m.x), hscale * (g.y - m.y));
-          float2 B = make_float2(hscale * (g.y + m.y), hscale * (m.x - g.x));
-          float2 A2 = cconj(A), B2 = cconj(B);
-          if (s != 0) {
-            const float2 tz = __ldg(&om[n * s]), tq = __ldg(&om[nq * s]);
-            A = cmul(A, tz);
-            B = cmul(B, tz);
-            A2 = cmul(A2, tq);
-            B2 = cmul(B2, tq);
+          const float2 A = make_float2(hscale * (g.x + m.x), hscale * (g.y - m.y));
+          const float2 B = make_float2(hscale * (g.y + m.y), hscale * (m.x - g.x));
+          if (s == 0) {
+            An = A;
+            Bn = B;
+          } else {
+            const float2 tz = __ldg(&om[n * s]);
+            An = cmac(An, A, tz);
+            Bn = cmac(Bn, B, tz);
           }
-          An = k ? cadd(An, A) : A;
-          Bn = k ? cadd(Bn, B) : B;
-          Aq = k ? cadd(Aq, A2) : A2;
-          Bq = k ? cadd(Bq, B2) : B2;
-          if (sl == 0) A0 = cadd(A0, buf[base + k * LS]);
+          if (sl == 0) {                              // n = 0
+            const float2 z = buf[base + k * LS];
+            Aq.x = __fmaf_rn(2.f * hscale, z.x, Aq.x);
+            Bq.x = __fmaf_rn(2.f * hscale, z.y, Bq.x);
+          } else if (s == 0) {
+            Aq = cconj(A);
+            Bq = cconj(B);
+          } else {
+            const float2 tq = __ldg(&om[nq * s]);
+            Aq = cmac(Aq, cconj(A), tq);
+            Bq = cmac(Bq, cconj(B), tq);
+          }
         }
-        if (sl || even) put(o + n, An, Bn);
-        if (sl) put(o + nq, Aq, Bq);
-        else put(o, make_float2(2.f * hscale * A0.x, 0.f), make_float2(2.f * hscale * A0.y, 0.f));
+        if (hasn) put(on, An, Bn);
+        put(oq, Aq, Bq);
       }
     }
     if (NS == 1) __syncthreads();                     // the next subset's fill takes the lines
