@@ -27,7 +27,7 @@ static cudaError_t fx_launch(K k, int nt, const RunDesc* runs, const WorkItem* i
 }
 
 cudaError_t launch_x_forward_fx(const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st) {
-  return fx_launch(x_forward_fx_kernel<256>, 256, runs, items, n, smem, st);
+  return fx_launch(x_forward_fx_kernel, kFxForwardThreads, runs, items, n, smem, st);
 }
 
 cudaError_t launch_z_fx(int K0, int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st) {

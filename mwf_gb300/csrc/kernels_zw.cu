@@ -16,14 +16,10 @@ static cudaError_t zw_launch(const RunDesc* runs, const WorkItem* items, int n, 
 
 cudaError_t launch_z_warp(int K0, int ns, int nt, const RunDesc* runs, const WorkItem* items, int n, size_t smem, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-#define MWF_ZW(K0_) \
-  if (K0 == K0_ && ns == 3 && nt == 256) return zw_launch<K0_, 3, 256, 2, 1>(runs, items, n, smem, st); \
-  if (K0 == K0_ && ns == 3 && nt == 576) return zw_launch<K0_, 3, 576, 1, 2>(runs, items, n, smem, st); \
-  if (K0 == K0_ && ns == 3 && nt == 512) return zw_launch<K0_, 3, 512, 1, 1>(runs, items, n, smem, st); \
-  if (K0 == K0_ && ns == 1 && nt == 256) return zw_launch<K0_, 1, 256, 2, 1>(runs, items, n, smem, st); \
-  if (K0 == K0_ && ns == 1 && nt == 576) return zw_launch<K0_, 1, 576, 1, 2>(runs, items, n, smem, st);
-  MWF_ZW(4)
-  MWF_ZW(6)
+#define MWF_ZW(K0_, NS_, NT_, MINB_, TW_) \
+  if (K0 == K0_ && ns == NS_ && nt == NT_) return zw_launch<K0_, NS_, NT_, MINB_, TW_>(runs, items, n, smem, st);
+  MWF_ZW(4, 3, 256, 2, 1) MWF_ZW(4, 3, 576, 1, 2) MWF_ZW(4, 1, 256, 2, 1) MWF_ZW(4, 1, 576, 1, 2)
+  MWF_ZW(6, 3, 256, 2, 1) MWF_ZW(6, 3, 512, 1, 1) MWF_ZW(6, 1, 256, 2, 1) MWF_ZW(6, 1, 576, 1, 2)
 #undef MWF_ZW
   return cudaErrorInvalidValue;
 }

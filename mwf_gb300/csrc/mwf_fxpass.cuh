@@ -125,8 +125,9 @@ __device__ __forceinline__ void fx_row_moments(const double2* __restrict__ row, 
   nan = all >= 0x7ff;
 }
 
-template <int NT>
-__global__ void __launch_bounds__(NT, 512 / NT) x_forward_fx_kernel(const RunDesc* __restrict__ runs, const WorkItem* __restrict__ items) {
+constexpr int kFxForwardThreads = 256;   // two CTAs per SM: the widest lines fit half an SM's shared memory
+__global__ void __launch_bounds__(kFxForwardThreads, 2) x_forward_fx_kernel(const RunDesc* __restrict__ runs, const WorkItem* __restrict__ items) {
+  constexpr int NT = kFxForwardThreads;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   longlong2* buf = reinterpret_cast<longlong2*>(smem_raw);       // line (l, s) at (3 l + s) MM
   __shared__ int colE[kFxMaxCols];
