@@ -373,15 +373,15 @@ def mwf_solver():
 
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of the z pass per launch, from single-
-# kernel ncu captures of smaller cases (profiles/z_nonlinear_fp64_m6_768sq.md,
+# kernel ncu captures of smaller cases (profiles/fixed_point_and_warp_passes.md,
 # profiles/batched_dram_fp32_ensemble64.md) scaled by the points processed:
-#  - FP64 M6: the 768^2 grid read 108.07 MB and wrote 129.06 MB; the 1536^2 grid has 4x the points
-#    (captured from the pass in FP64 arithmetic; the fixed-point one moves the same T and NLT, and
-#    14 MB of row norms);
+#  - FP64 M6, fixed point: DRAM read of the 768^2 grid, 110.63 MB (the algorithmic read of T is 106.95, the row
+#    norms 3.6), times 4 for the 1536^2 grid's points, plus the algorithmic write 3 KK X NN 16 B (of the
+#    768^2 grid's 160.4 MB a third stayed in L2);
 #  - batched FP32 M4 z pass: DRAM read per run of MM = NN = 32, 48, 64, 96, 128 (the capture's
 #    reads divided by its runs of each size; 0.2-1.1 % above the algorithmic read of T), plus the
 #    algorithmic write KK X NN 8 B, which at the capture's size stays in L2.
-ZPASS_TRAFFIC = {"m6-1024-fp64": 4 * (108.07e6 + 129.06e6)}
+ZPASS_TRAFFIC = {"m6-1024-fp64": 4 * 110.63e6 + 3 * 17 * 1536 * 512 * 16}
 ZB_READ_PER_RUN = {32: 7115520 / 13, 48: 19553536 / 16, 64: 19536640 / 9, 96: 78002432 / 16, 128: 86641408 / 10}
 
 

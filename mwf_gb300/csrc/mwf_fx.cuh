@@ -10,7 +10,7 @@
 // N = 1024, more than the 2^-53 of FP64 arithmetic.  So until the first two stages are
 // done, whose results are sums of only a few values, a line has finer scales from its largest value
 // (fx_fine).  Error of the nonlinear term against extended precision, lengths of 3 ... 1024 modes,
-// as a fraction of that of the FP64-arithmetic kernels: Gaussian states 0.16 ... 0.22 on square grids and up to 0.95 on
+// as a fraction of that of the FP64-arithmetic kernels: Gaussian states 0.16 ... 0.31 on square grids and up to 0.95 on
 // thin ones, spectra 1 / (1 + k^2 / 20) 0.36 ... 0.92, white ones 0.27 ... 0.86, wall-normal modes that fall by 10 from
 // one to the next 0.4 ... 1.07 (of the whole term; the last of such modes alone up to 50: the coupling's operands share a
 // scale).
@@ -116,7 +116,7 @@ __host__ __device__ __forceinline__ i64 fx_shift(i64 x, int sh) {
 // x 2^-r, r >= 1, |x| <= 2^62, and x / 2, rounded to nearest, ties to even: ties rounded up are a bias of 2^-(r+1),
 // the same for all values of a stage, which the later stages add up in the lowest wavenumbers (M4
 // 512 x 512, white spectrum: the nonlinear term was 1.24 times as far off as with FP64 arithmetic, with ties
-// to even 0.96 and, the coupling's sums rounded more finely, 0.38).
+// to even 0.96 and, the coupling's sums rounded more finely, 0.47).
 // Shifts beyond 63, which leave nothing, are those of 63 (of 64 and more the half of the last bit
 // would be 0 or overflow, and everything, zeros too, could become -1): they come from directions or
 // rows of the coupling that are zero, or far below the others.

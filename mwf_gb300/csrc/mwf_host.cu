@@ -927,7 +927,7 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
     o = run_bytes(r, o);
     h->stage_elems = std::max(h->stage_elems, r.csz);
   }
-  // the Euler-start flags of all runs side by side, so one memset per step clears them
+  // the Euler-start flags of all runs side by side, so one memset clears them (enqueue_step)
   const size_t off_nst_all = o; o = align_up(o + sizeof(int) * n_runs, 256);
   for (int i = 0; i < n_runs; ++i) h->runs[i].off_nst = off_nst_all + sizeof(int) * i;
   h->off_nst_all = off_nst_all;
@@ -940,9 +940,10 @@ int mwf_create(const mwf_run_desc* runs, int n_runs, int device, mwf_handle** ou
 #ifndef MWF_NO_PERSIST
   for (RunHost& r : h->runs) r.persist = r.d.precision == MWF_FP32 && r.xbf_nb && r.zb_lx && r.xbi_nb;
 #endif
-  // FP32 items by what their launch holds.  One run, us a step with the widest items and with these: M4,
-  // 32 x 32 18.5 and 13.3, 64 x 64 23.8 and 16.5, 36 x 36 40.5 and 22.8, 72 x 72 54.2 and 28.9; M6, 64 x 64
-  // 25.2 and 20.4, 72 x 72 54.4 and 34.7; eight M4 36 x 36 43.5 and 32.9.  Full launches keep the widest.
+  // FP32 items by what their launch holds (a run's results do not depend on the width, bitwise).  One run, us a
+  // step with the widest items, by the knobs, and with these: M4, MM = NN = 32 18.0 and 11.8, 64 22.5 and 16.3; M6,
+  // 64 24.6 and 20.1.  Warp-line runs when the rule came in, and now: M4 36 40.5, 22.8 and 21.8, 72 54.2,
+  // 28.9 and 27.7; M6 72 54.4, 39.1 and 33.8; eight M4 36 43.5, 32.9 and 32.1.  Full launches keep the widest.
   {
     std::map<std::vector<int>, std::vector<ItemWidth>> xf, z, xi, xwf, xwi, zw;
     for (RunHost& r : h->runs) {
